@@ -478,8 +478,22 @@ __global__ void __launch_bounds__(512) fft_tile_kernel(const C2 *in, C2 *out, Ti
 // ---------------------------------------------------------------------------
 // Table generation (FP64, sincospi), rounded to T.
 // ---------------------------------------------------------------------------
-// out[t] = e^{-2 pi i t * num / den} for t < count
-template <typename T> __global__ void roots_kernel(C2 *out, int64_t count, int64_t num, int64_t den) {
+// A root's cosine or sine times 2^62 as two signed halves, high and low (the
+// low half is negated in products: never the lowest int): the factors of
+// jt_fix64.cuh.
+__device__ __forceinline__ int2 fx_split(double c) {
+    long long v = __double2ll_rn(c * 4611686018427387904.0);
+    if ((int)v == INT32_MIN) v++;
+    return make_int2((int)(v >> 32) + (int)((uint32_t)v >> 31), (int)v);
+}
+__device__ __forceinline__ int4 fx_twiddle(double c, double s) {
+    const int2 a = fx_split(c), b = fx_split(s);
+    return make_int4(a.x, a.y, b.x, b.y);
+}
+
+// out[t] = e^{-2 pi i t * num / den} for t < count; fixed (double): the same
+// roots as fx_twiddle's after them
+template <typename T> __global__ void roots_kernel(C2 *out, int64_t count, int64_t num, int64_t den, bool fixed) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= count) return;
     // reduce t*num mod den exactly in integers, then angle = 2 * r / den (in half turns)
@@ -487,6 +501,7 @@ template <typename T> __global__ void roots_kernel(C2 *out, int64_t count, int64
     double s, c;
     sincospi(-2.0 * (double)r / (double)den, &s, &c);
     out[t] = mk<T>((T)c, (T)s);
+    if (sizeof(T) == 8 && fixed) reinterpret_cast<int4 *>(out + count)[t] = fx_twiddle(c, s);
 }
 
 // Bluestein chirp bk1[i] = e^{i pi (i^2 mod 2n) / n} (fft/DoubleFFT_1D.java:1864-1879)

@@ -4,7 +4,9 @@
 // Algorithm choice per complex length n (GPU-first, not the reference's
 // split-radix / FFTPACK / Bluestein choice, which only fixes the results):
 //   DIRECT    n <= 8192 (f32) / 4096 (f64) with prime factors <= 63: one
-//             shared-memory tile kernel per batch of lines.
+//             shared-memory tile kernel per batch of lines; powers of two in
+//             registers, floats in FP32 (jt_stockham.cuh), doubles in 64-bit
+//             fixed point (jt_fix64.cuh).
 //   TWOPASS   n = n1 * n2 with both DIRECT: column pass with the four-step
 //             twiddle fused into its store, then a row pass that writes the
 //             transposed (natural-order) result.  The batch is processed in
@@ -225,12 +227,10 @@ static int device_init() {
 // Register-resident power-of-two kernel launchers (jt_pow2_f32.cu, jt_pow2_f64.cu).
 bool stockham_launch(int L, int mode, int sign, const float2 *in, float2 *out, const StockParams &p, const CUtensorMap *tmap,
                      const float2 *W, const float2 *Whi, const float2 *Wlo, int *err, int sms, cudaStream_t s);
-bool stockham_launch(int L, int mode, int sign, const double2 *in, double2 *out, const StockParams &p, const CUtensorMap *tmap,
-                     const double2 *W, const double2 *Whi, const double2 *Wlo, int *err, int sms, cudaStream_t s);
+bool fix_launch(int L, int mode, int sign, const double2 *in, double2 *out, const StockParams &p, const double2 *W,
+                const double2 *Whi, const double2 *Wlo, const int4 *Whiq, const int4 *Wloq, cudaStream_t s);
 bool stockham_pipe_ok(int L, int mode, const float *);
-bool stockham_pipe_ok(int L, int mode, const double *);
 int stockham_lines_per_cta(int L, int mode, const float *);
-int stockham_lines_per_cta(int L, int mode, const double *);
 bool tc_split_ok(int L);
 // Register-form DCT/DST/DHT lines (jt_r2r_f32.cu, jt_r2r_f64.cu).
 bool r2r_reg_launch(int H, int op, const float *in, float *out, const R2rParams &p, const float2 *Wp, const float2 *Wr,
@@ -357,8 +357,8 @@ template <typename T> struct Fft1 {
         *bits = 0;
         while (((int64_t)1 << (2 * *bits)) < len) (*bits)++;
         const int64_t nlo = (int64_t)1 << *bits;
-        JT_TRY(make_roots(lo, nlo, 1, len));
-        return make_roots(hi, cdiv(len, nlo), nlo, len);
+        JT_TRY(make_roots(lo, nlo, 1, len, sizeof(T) == 8));
+        return make_roots(hi, cdiv(len, nlo), nlo, len, sizeof(T) == 8);
     }
 
     static bool generic_ok(int64_t n) { return n >= 2 && n <= Lim<T>::lmax() && !direct_radices(n).empty(); }
@@ -388,9 +388,10 @@ template <typename T> struct Fft1 {
     // whether a line pass with strided (column) layouts can run in one kernel
     bool cols_ok() const { return algo == ALG_DIRECT && (reg ? n <= 4096 : true); }
 
-    static int make_roots(C2 **out, int64_t count, int64_t num, int64_t den) {
-        JT_CU(cudaMalloc(out, sizeof(C2) * std::max<int64_t>(count, 1)));
-        roots_kernel<T><<<(unsigned)cdiv(count, 256), 256, 0, g_setup>>>(*out, count, num, den);
+    // fixed: followed by the same roots in fixed point (doubles only)
+    static int make_roots(C2 **out, int64_t count, int64_t num, int64_t den, bool fixed = false) {
+        JT_CU(cudaMalloc(out, sizeof(C2) * std::max<int64_t>(count, 1) * (fixed ? 2 : 1)));
+        roots_kernel<T><<<(unsigned)cdiv(count, 256), 256, 0, g_setup>>>(*out, count, num, den, fixed);
         g_launches++;
         JT_CU(cudaGetLastError());
         return JT_OK;
@@ -398,7 +399,7 @@ template <typename T> struct Fft1 {
 
     static int make_pass_table(C2 **out, int L) {
         const int count = stock_tw_count(L);
-        JT_CU(cudaMalloc(out, sizeof(C2) * std::max(count, 1)));
+        JT_CU(cudaMalloc(out, sizeof(C2) * std::max(count, 1) * (sizeof(T) == 8 ? 2 : 1)));
         if (count > 0) {
             passtw_kernel<T><<<(unsigned)cdiv(count, 256), 256, 0, g_setup>>>(*out, L);
             g_launches++;
@@ -704,9 +705,21 @@ template <typename T> struct Fft1 {
             sp.stream_out = hint_stream_out;
             sp.reverse = hint_reverse;
             if (ctx.dry) return JT_OK;
-            const int esz = (int)sizeof(C2);
-            // split-operand tensor-core kernel for Float32 row passes
-            if constexpr (sizeof(T) == 4) {
+            // doubles run in 64-bit fixed point (jt_fix64.cuh)
+            if constexpr (sizeof(T) == 8) {
+                int e2 = 0;
+                const bool pow2_scale = std::frexp(scale, &e2) == 0.5;
+                sp.scale_e2 = pow2_scale ? e2 - 1 : 0;
+                sp.scale_mul = !pow2_scale;
+                const int64_t nlo = (int64_t)1 << tw_lo_bits, nhi = tw_n ? cdiv(tw_n, nlo) : 0;
+                if (!fix_launch((int)n, mode, sign, in, out, sp, Wp, Whi_, Wlo_, (const int4 *)(Whi_ ? Whi_ + nhi : nullptr),
+                                (const int4 *)(Wlo_ ? Wlo_ + nlo : nullptr), ctx.s))
+                    return JT_EINVAL;
+                g_launches++;
+                return JT_OK;
+            } else {
+                const int esz = (int)sizeof(C2);
+                // split-operand tensor-core kernel for Float32 row passes
                 if (ctx.tc && mode == 0 && tc_split_ok((int)n)) {
                     if (!tc_split_launch((int)n, sign, (const float2 *)in, (float2 *)out, sp, (const float2 *)Wp, g_err_dev,
                                          g_sms, ctx.s))
@@ -714,27 +727,27 @@ template <typename T> struct Fft1 {
                     g_launches++;
                     return JT_OK;
                 }
+                // TMA pipeline when the 16-byte rules hold, else the plain kernel
+                const int Cl = stockham_lines_per_cta((int)n, mode, (const T *)nullptr);
+                CUtensorMap tm;
+                memset(&tm, 0, sizeof(tm));
+                bool pipe = g_opt_tma.load() && stockham_pipe_ok((int)n, mode, (const T *)nullptr) && ((uintptr_t)in % 16) == 0;
+                if (pipe && mode == 1) {
+                    pipe = lin.istride == 1 && lin.inner % Cl == 0 && nlines % lin.inner == 0 &&
+                           make_col_tmap(&tm, in, esz, lin.inner, n, nlines / lin.inner, lin.estride, lin.outer, Cl,
+                                         (int)std::min<int64_t>(n, 256));
+                    sp.tiles_per_col = lin.inner / Cl;
+                } else if (pipe) {
+                    bool contig = lin.inner == 1 && lin.outer == n;
+                    pipe = contig || ((lin.outer * esz) % 16 == 0 && (lin.inner == 1 || (lin.istride * esz) % 16 == 0));
+                    pipe = pipe && (n * esz) % 16 == 0;
+                }
+                if (!stockham_launch((int)n, mode, sign, in, out, sp, pipe ? &tm : nullptr, Wp, Whi_, Wlo_, g_err_dev, g_sms,
+                                     ctx.s))
+                    return JT_EINVAL;
+                g_launches++;
+                return JT_OK;
             }
-            // TMA pipeline when the 16-byte rules hold, else the plain kernel
-            const int Cl = stockham_lines_per_cta((int)n, mode, (const T *)nullptr);
-            CUtensorMap tm;
-            memset(&tm, 0, sizeof(tm));
-            bool pipe = g_opt_tma.load() && stockham_pipe_ok((int)n, mode, (const T *)nullptr) && ((uintptr_t)in % 16) == 0;
-            if (pipe && mode == 1) {
-                pipe = lin.istride == 1 && lin.inner % Cl == 0 && nlines % lin.inner == 0 &&
-                       make_col_tmap(&tm, in, esz, lin.inner, n, nlines / lin.inner, lin.estride, lin.outer, Cl,
-                                     (int)std::min<int64_t>(n, 256));
-                sp.tiles_per_col = lin.inner / Cl;
-            } else if (pipe) {
-                bool contig = lin.inner == 1 && lin.outer == n;
-                pipe = contig || ((lin.outer * esz) % 16 == 0 && (lin.inner == 1 || (lin.istride * esz) % 16 == 0));
-                pipe = pipe && (n * esz) % 16 == 0;
-            }
-            if (!stockham_launch((int)n, mode, sign, in, out, sp, pipe ? &tm : nullptr, Wp, Whi_, Wlo_, g_err_dev, g_sms,
-                                 ctx.s))
-                return JT_EINVAL;
-            g_launches++;
-            return JT_OK;
         }
         const int L = (int)n;
         const int Lp = padded_len(L);

@@ -1,48 +1,26 @@
-// jt_pow2_f64.cu -- instantiations of the register-resident power-of-two
-// Stockham kernels (jt_stockham.cuh) for double.
-#include "jt_stockham.cuh"
+// jt_pow2_f64.cu -- instantiations of the power-of-two line kernels for
+// double (jt_fix64.cuh).
+#include "jt_fix64.cuh"
 
 namespace jt {
 
-// Whether the pipelined (TMA) kernel exists for (L, mode).
-bool stockham_pipe_ok(int L, int mode, const double *) {
-#define JT_PCASE(LL) \
-    case LL:         \
-        return mode == 0 ? (Stockham<double, LL, 0, -1>::PIPE_OK || Stockham<double, LL, 0, -1>::BIG_OK) : (LL <= 4096 && Stockham<double, (LL <= 4096 ? LL : 16), 1, -1>::PIPE_OK);
-    switch (L) {
-        JT_PCASE(16) JT_PCASE(32) JT_PCASE(64) JT_PCASE(128) JT_PCASE(256) JT_PCASE(512) JT_PCASE(1024)
-        JT_PCASE(2048) JT_PCASE(4096) JT_PCASE(8192)
-
-        default: return false;
-    }
-#undef JT_PCASE
-}
-
-// Lines per CTA of (L, mode).
-int stockham_lines_per_cta(int L, int mode, const double *) { return StockCfg<double>::C(L, mode); }
-
 // Launches the kernel for line length L; returns false when (L, mode) has no
-// instantiation (row mode: 16..8192, column modes: 16..4096).  A non-null
-// `tmap` selects the pipelined TMA kernel (the caller has checked
-// stockham_pipe_ok and the 16-byte rules).
-bool stockham_launch(int L, int mode, int sign, const V2<double>::t *in, V2<double>::t *out, const StockParams &p,
-                     const CUtensorMap *tmap, const V2<double>::t *W, const V2<double>::t *Whi, const V2<double>::t *Wlo,
-                     int *err, int sms, cudaStream_t s) {
-#define JT_CASE(LL)                                                                       \
-    case LL:                                                                              \
-        StockLaunch<double, LL>::go(mode, sign, in, out, p, tmap, W, Whi, Wlo, err, sms, s); \
+// instantiation (row mode: 16..8192, column modes: 16..4096).  Whiq, Wloq: the
+// fixed-point forms of the two-level four-step tables Whi, Wlo; W's follow W.
+bool fix_launch(int L, int mode, int sign, const double2 *in, double2 *out, const StockParams &p, const double2 *W,
+                const double2 *Whi, const double2 *Wlo, const int4 *Whiq, const int4 *Wloq, cudaStream_t s) {
+    const int4 *Wq = reinterpret_cast<const int4 *>(W + stock_tw_count(L));
+#define JT_CASE(LL)                                                                          \
+    case LL:                                                                                 \
+        FixLaunch<LL>::go(mode, sign, in, out, p, W, Whi, Wlo, Wq, Whiq, Wloq, s);           \
         return true;
-    if (mode == 0) {
-        switch (L) {
-            JT_CASE(16) JT_CASE(32) JT_CASE(64) JT_CASE(128) JT_CASE(256) JT_CASE(512) JT_CASE(1024)
-            JT_CASE(2048) JT_CASE(4096) JT_CASE(8192)
-
-            default: return false;
-        }
-    }
     switch (L) {
         JT_CASE(16) JT_CASE(32) JT_CASE(64) JT_CASE(128) JT_CASE(256) JT_CASE(512) JT_CASE(1024)
         JT_CASE(2048) JT_CASE(4096)
+        case 8192:
+            if (mode != 0) return false;
+            FixLaunch<8192>::go(mode, sign, in, out, p, W, Whi, Wlo, Wq, Whiq, Wloq, s);
+            return true;
         default: return false;
     }
 #undef JT_CASE

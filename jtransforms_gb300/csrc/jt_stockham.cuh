@@ -38,6 +38,7 @@ struct StockParams {
     double scale;  // output multiplier (double plans)
     float scalef;  // the same for float plans: float kernels do no FP64 work
     int do_scale;
+    int scale_e2, scale_mul; // scale as 2^scale_e2 (doubles), else scale_mul = 1
     int64_t tw_n, tw_inner;  // four-step output twiddle w_{tw_n}^{pos * (b % tw_inner)}; tw_n = 0: none
     int tw_lo_bits;
     uint32_t tw_mask;        // exponent reduction: tw_n - 1 for a power of two up to 2^32, else all ones
@@ -107,6 +108,9 @@ __host__ __device__ inline int stock_tw_count(int L) {
     return tot;
 }
 
+//
+// Double tables are followed by the same entries in fixed point (int4,
+// fx_twiddle below).
 template <typename T> __global__ void passtw_kernel(typename V2<T>::t *out, int L) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int E = L >= 16 ? 16 : L;
@@ -137,6 +141,7 @@ template <typename T> __global__ void passtw_kernel(typename V2<T>::t *out, int 
                 double s, c;
                 sincospi(-2.0 * (double)num / (double)den, &s, &c);
                 out[idx] = mk<T>((T)c, (T)s);
+                if constexpr (sizeof(T) == 8) reinterpret_cast<int4 *>(out + stock_tw_count(L))[idx] = fx_twiddle(c, s);
                 return;
             }
             off += ns * R;
