@@ -228,17 +228,23 @@ static int device_init() {
 bool stockham_launch(int L, int mode, int sign, const float2 *in, float2 *out, const StockParams &p, const CUtensorMap *tmap,
                      const float2 *W, const float2 *Whi, const float2 *Wlo, int *err, int sms, cudaStream_t s);
 bool fix_launch(int L, int mode, int sign, const double2 *in, double2 *out, const StockParams &p, const double2 *W,
-                const double2 *Whi, const double2 *Wlo, const int4 *Whiq, const int4 *Wloq, cudaStream_t s);
+                const double2 *Whi, const double2 *Wlo, const int4 *Whiq, const int4 *Wloq, int sms, cudaStream_t s);
 bool stockham_pipe_ok(int L, int mode, const float *);
 int stockham_lines_per_cta(int L, int mode, const float *);
 bool tc_split_ok(int L);
-// Register-form DCT/DST/DHT lines (jt_r2r_f32.cu, jt_r2r_f64.cu).
+// Register-form DCT/DST/DHT lines (jt_r2r_f32.cu).
 bool r2r_reg_launch(int H, int op, const float *in, float *out, const R2rParams &p, const float2 *Wp, const float2 *Wr,
                     const float2 *Wd, cudaStream_t s);
-bool r2r_reg_launch(int H, int op, const double *in, double *out, const R2rParams &p, const double2 *Wp, const double2 *Wr,
-                    const double2 *Wd, cudaStream_t s);
 int r2r_reg_lines(int H, const float *);
-int r2r_reg_lines(int H, const double *);
+// The double lines' kernels (jt_fixr2r.cuh: half lengths up to 128, beyond).
+bool fix_r2r_launch(int H, int op, bool strided, const double *in, double *out, const R2rParams &p, const FixR2rScale &fs,
+                    const double2 *Wp, const double2 *Wr, const double2 *Wd, const int4 *Wpq, const int4 *Wrq, const int4 *Wdq,
+                    int sms, cudaStream_t s);
+bool fix_r2r_launch_long(int H, int op, bool strided, const double *in, double *out, const R2rParams &p, const FixR2rScale &fs,
+                         const double2 *Wp, const double2 *Wr, const double2 *Wd, const int4 *Wpq, const int4 *Wrq, const int4 *Wdq,
+                         int sms, cudaStream_t s);
+// most lines per CTA: strided ones move in runs of four (32 bytes) up to 2048
+static int r2r_reg_lines(int H, const double *) { return H <= 1024 ? 4096 / H : H <= 2048 ? 4 : 1; }
 bool tc_split_launch(int L, int sign, const float2 *in, float2 *out, const StockParams &p, const float2 *W, int *err, int sms,
                      cudaStream_t s);
 
@@ -713,7 +719,7 @@ template <typename T> struct Fft1 {
                 sp.scale_mul = !pow2_scale;
                 const int64_t nlo = (int64_t)1 << tw_lo_bits, nhi = tw_n ? cdiv(tw_n, nlo) : 0;
                 if (!fix_launch((int)n, mode, sign, in, out, sp, Wp, Whi_, Wlo_, (const int4 *)(Whi_ ? Whi_ + nhi : nullptr),
-                                (const int4 *)(Wlo_ ? Wlo_ + nlo : nullptr), ctx.s))
+                                (const int4 *)(Wlo_ ? Wlo_ + nlo : nullptr), g_sms, ctx.s))
                     return JT_EINVAL;
                 g_launches++;
                 return JT_OK;
@@ -1009,7 +1015,7 @@ template <typename T> struct Real1 {
         r->n = n;
         if (n >= 2 && n % 2 == 0) {
             JT_TRY(cached<Fft1<T>>(n / 2, r->half));
-            JT_TRY(Fft1<T>::make_roots(&r->Wr, n / 4 + 1, 1, n));
+            JT_TRY(Fft1<T>::make_roots(&r->Wr, n / 4 + 1, 1, n, sizeof(T) == 8 && is_pow2(n)));
         } else if (n > 1) {
             JT_TRY(cached<Fft1<T>>(n, r->full));
         }
@@ -1239,15 +1245,31 @@ static int r2r_fused(Ctx &ctx, int op, const Real1<T> *rf, const T *in, T *out, 
     // (at least 32-byte runs on strided lines, at least one warp per CTA)
     const int creg = r2r_reg_c<T>(h, rf);
     if (creg > 0 && (!strided || creg >= (int)(32 / sizeof(T)))) {
-        int cr = creg;
-        const int cmin = std::max<int>(strided ? (int)(32 / sizeof(T)) : 1, (int)std::max<int64_t>(1, 32 / (h / 16)));
-        while (cr > cmin && cdiv(nlines, cr) < 2 * (int64_t)g_sms) cr /= 2;
-        p.C = std::max(cr, 1);
-        if (ctx.dry) return JT_OK;
-        if (cdiv(nlines, creg) > 0x7fffffff) return JT_ETOOBIG;
-        if (!r2r_reg_launch((int)h, op, in, out, p, rf->half->Wp, rf->Wr, Wd, ctx.s)) return JT_EINVAL;
-        g_launches++;
-        return JT_OK;
+        if constexpr (sizeof(T) == 8) {
+            if (ctx.dry) return JT_OK;
+            if (cdiv(nlines, strided ? 4 : creg) > 0x7fffffff) return JT_ETOOBIG;
+            FixR2rScale fs;
+            fix_scale(mult, &fs.e2, &fs.k);
+            fix_scale(mult0, &fs.e20, &fs.k0);
+            fs.c0 = mult0 == mult ? 0 : mult0 == 2 * mult ? 2 : 1;
+            const int4 *Wpq = (const int4 *)(rf->half->Wp + stock_tw_count((int)h)), *Wrq = (const int4 *)(rf->Wr + n / 4 + 1);
+            const int4 *Wdq = Wd ? (const int4 *)(Wd + n) : nullptr;
+            if (!(h <= 128 ? fix_r2r_launch : fix_r2r_launch_long)((int)h, op, strided, in, out, p, fs, rf->half->Wp, rf->Wr, Wd, Wpq,
+                                                                   Wrq, Wdq, g_sms, ctx.s))
+                return JT_EINVAL;
+            g_launches++;
+            return JT_OK;
+        } else {
+            int cr = creg;
+            const int cmin = std::max<int>(strided ? (int)(32 / sizeof(T)) : 1, (int)std::max<int64_t>(1, 32 / (h / 16)));
+            while (cr > cmin && cdiv(nlines, cr) < 2 * (int64_t)g_sms) cr /= 2;
+            p.C = std::max(cr, 1);
+            if (ctx.dry) return JT_OK;
+            if (cdiv(nlines, creg) > 0x7fffffff) return JT_ETOOBIG;
+            if (!r2r_reg_launch((int)h, op, in, out, p, rf->half->Wp, rf->Wr, Wd, ctx.s)) return JT_EINVAL;
+            g_launches++;
+            return JT_OK;
+        }
     }
     if (ctx.dry) return JT_OK;
     const int64_t grid = cdiv(nlines, C);
@@ -1281,7 +1303,7 @@ template <typename T> struct Dct1 {
         d->n = n;
         if (n > 1) {
             JT_TRY(cached<Real1<T>>(n, d->rf));
-            JT_TRY(Fft1<T>::make_roots(&d->Wd, n, 1, 4 * n));  // e^{-i pi k/(2n)}
+            JT_TRY(Fft1<T>::make_roots(&d->Wd, n, 1, 4 * n, sizeof(T) == 8 && is_pow2(n)));  // e^{-i pi k/(2n)}
         }
         out = std::move(d);
         return JT_OK;

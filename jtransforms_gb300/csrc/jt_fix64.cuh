@@ -70,8 +70,9 @@ __device__ __forceinline__ long long fx_mulk(long long v, long long k) {
     const long long m = fx_madw(vl, kh, fx_madw(vh, kl, 1ll << 31));
     return fx_madw(vh, kh, m >> 32);
 }
-// round(f 2^64) for -1/2 < f < 1/2: cos(pi/4) - 1, tan(pi/16), sin(pi/8)
+// round(f 2^64) for -1/2 < f < 1/2: cos(pi/4) - 1, sqrt(2) - 1, tan(pi/16), sin(pi/8)
 static constexpr long long kFxHm1 = -5402926248376769404ll;
+static constexpr long long kFxR2m1 = 7640891576956012809ll;
 static constexpr long long kFxTan16 = 3669285534148243471ll;
 static constexpr long long kFxSin8 = 7059263338087549767ll;
 __device__ __forceinline__ long long fx_mulh(long long v) { return v + fx_mulk(v, kFxHm1); }  // v cos(pi/4)
@@ -180,11 +181,12 @@ __device__ __forceinline__ FxLine fx_line(uint32_t m) {
     l.ex = max(eb, 1) + l.pre - JT_FX_BIAS;
     return l;
 }
-__device__ __forceinline__ long long fx_from(double d, const FxLine &l) {
+// The line's numbers below 2^BITS (l.ex is for 58).
+template <int BITS = 58> __device__ __forceinline__ long long fx_from(double d, const FxLine &l) {
     const int hi = __double2hiint(d), lo = __double2loint(d);
     const int e = (hi >> 20) & 0x7ff;
     const uint32_t mh = ((uint32_t)hi & 0xfffffu) | 0x100000u;
-    const int r = min(l.ex + JT_FX_BIAS + 5 - e, 63);  // at least 5; zeros (and far smaller numbers) go to 0
+    const int r = min(l.ex + JT_FX_BIAS + 63 - BITS - e, 63);  // at least 63 - BITS; zeros (and far smaller numbers) go to 0
     unsigned long long u = (((unsigned long long)mh << 32) | (uint32_t)lo) << 10;
     u >>= r;
     const long long s = (long long)(hi >> 31);
@@ -200,11 +202,22 @@ __device__ __forceinline__ double fx_to(long long v, int ex) {
 // needed or not, and six of those per number were most of this kernel's time.
 __device__ __forceinline__ double fx_pre(int pre) { return pre > 0 ? 1.3407807929942597e154 : pre < 0 ? 7.458340731200207e-155 : 1.0; }
 
-// Shift that brings a line with these bits to 60 bits: right by s > 0 or left by -s.
-__device__ __forceinline__ int fx_norm_shift(uint32_t bits) { return bits ? 4 - __clz(bits) : 0; }
+// Shift that brings a line with these bits to BITS bits: right by s > 0 or left by -s.
+template <int BITS = 60> __device__ __forceinline__ int fx_norm_shift(uint32_t bits) { return bits ? 64 - BITS - __clz(bits) : 0; }
 // (v + rnd) >> s with rnd = half a unit of the result
 __device__ __forceinline__ Fx fx_shr(Fx v, int s, long long rnd) { return Fx{(v.x + rnd) >> s, (v.y + rnd) >> s}; }
 __device__ __forceinline__ long long fx_half(int s) { return s > 0 ? 1ll << (s - 1) : 0; }
+// N values by the shift s (fx_norm_shift's)
+template <int N> __device__ __forceinline__ void fx_norm(Fx *v, int s) {
+    if (s < 0) {
+#pragma unroll
+        for (int m = 0; m < N; m++) v[m] = Fx{v[m].x << -s, v[m].y << -s};
+        s = 0;
+    }
+    const long long r = fx_half(s);
+#pragma unroll
+    for (int m = 0; m < N; m++) v[m] = fx_shr(v[m], s, r);
+}
 
 // Fixed-point pass table of a length-L line: the entries of the double table
 // (stock_tw_count, factor k of a pass as NS entries) as int4.
@@ -213,50 +226,74 @@ __device__ __forceinline__ const int4 *fx_factor(const int4 *W, int off, int ns,
 }
 
 struct FxCfg {
-    // lines per CTA: 128 threads of 16 numbers for short rows; 128-byte
-    // segments (8 columns) for the column modes up to 512, fewer above
+    // most lines per CTA: 128 threads of 16 numbers for short lines; of the
+    // column modes' longer ones 8 columns (128-byte segments) up to 512, fewer above
     static constexpr int rows_C(int L) { return L >= 2048 ? 1 : 2048 / L; }
-    static constexpr int cols_C(int L) { return L <= 512 ? 8 : 4096 / L < 2 ? 2 : 4096 / L; }
+    static constexpr int cols_C(int L) { return L <= 256 ? 2048 / L : L <= 512 ? 8 : 4096 / L < 2 ? 2 : 4096 / L; }
     static constexpr int C(int L, int mode) { return mode == 0 ? rows_C(L) : cols_C(L); }
 };
 
-template <int L, int MODE, int SIGN> struct FxStock {
+// The passes of a CTA's lines: C lines (at most CM, a power of two) of TL
+// threads each; MODE 0 keeps a line's threads together, the column modes
+// spread the lines across a warp (c fastest).
+template <int L, int MODE, int SIGN, int CM> struct FxStock {
     typedef Stockham<double, L, MODE, SIGN> S;
-    static constexpr int E = 16, TL = L / 16, C = FxCfg::C(L, MODE), NT = C * TL, LP = S::LP;
+    static constexpr int E = 16, TL = L / 16, NT = CM * TL, LP = S::LP;
     static constexpr int NPASS = S::NPASS;
     static constexpr bool WARP_LINE = MODE == 0 && TL <= 32;  // a line's threads share a warp
-    static constexpr size_t SMEM = (size_t)C * LP * sizeof(Fx);
+    // A line's stride in shared memory.  The column modes' quarter-warps (16-byte
+    // accesses) cover C lines at 8 / C neighbouring positions: strides of
+    // 8 / C modulo 8 spread them over the banks (L + L/16 is a multiple of 8
+    // for the lines, of 128 and more, that run with C < 8).
+    static __host__ __device__ __forceinline__ int stride(int C) { return MODE == 0 || C >= 8 ? LP : LP - 1 + 8 / C; }
+    static constexpr size_t SMEM = (size_t)CM * (MODE == 0 || CM >= 8 ? LP : LP - 1 + 8 / CM) * sizeof(Fx);
     static constexpr int MINB = NT >= 512 ? 1 : 512 / NT > 8 ? 8 : 512 / NT;  // 128 registers a thread
+    static constexpr int RED = WARP_LINE ? 1 : (NPASS + 2) * CM;  // words of `red`
 
-    // OR of x over the threads of this thread's line that are in its warp
-    static __device__ __forceinline__ uint32_t warp_or(uint32_t x) {
-        constexpr int lo = MODE == 0 ? 1 : C, hi = MODE == 0 ? (TL < 32 ? TL : 32) : 32;
+    // fewest lines per CTA: whole warps
+    static constexpr int CMIN = TL >= 32 ? 1 : 32 / TL;
+
+    // OR (MAX: largest) of x over the threads of this thread's line that are in its warp
+    template <bool MAX> static __device__ __forceinline__ uint32_t warp_red(uint32_t x, int C) {
+        auto join = [](uint32_t a, uint32_t b) { return MAX ? max(a, b) : a | b; };
         if constexpr (MODE == 0 && TL >= 32) {
-            return __reduce_or_sync(0xffffffffu, x);
-        } else {
+            return MAX ? __reduce_max_sync(0xffffffffu, x) : __reduce_or_sync(0xffffffffu, x);
+        } else if constexpr (MODE == 0) {
 #pragma unroll
-            for (int o = lo; o < hi && o < 32; o <<= 1) x |= __shfl_xor_sync(0xffffffffu, x, o);
+            for (int o = 1; o < TL; o <<= 1) x = join(x, __shfl_xor_sync(0xffffffffu, x, o));
+        } else {
+            for (int o = C; o < 32; o <<= 1) x = join(x, __shfl_xor_sync(0xffffffffu, x, o));
+        }
+        return x;
+    }
+    // The same over the whole line: `slot` of red (CM words each, zeroed), and
+    // a barrier of the line's threads in any case
+    template <bool MAX> static __device__ __forceinline__ uint32_t line_red(uint32_t x, int slot, int c, int tid, int C, uint32_t *red) {
+        x = warp_red<MAX>(x, C);
+        if constexpr (WARP_LINE) {
+            __syncwarp();
             return x;
+        } else {
+            if (MODE == 0 ? tid % 32 == 0 : tid % 32 < C) {
+                if (MAX) atomicMax(&red[slot * CM + c], x);
+                else atomicOr(&red[slot * CM + c], x);
+            }
+            __syncthreads();
+            return red[slot * CM + c];
         }
     }
-    static __device__ __forceinline__ uint32_t warp_max(uint32_t x) {
-        constexpr int lo = MODE == 0 ? 1 : C, hi = MODE == 0 ? (TL < 32 ? TL : 32) : 32;
-        if constexpr (MODE == 0 && TL >= 32) {
-            return __reduce_max_sync(0xffffffffu, x);
-        } else {
-#pragma unroll
-            for (int o = lo; o < hi && o < 32; o <<= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, o));
-            return x;
-        }
+    static __device__ __forceinline__ void line_sync() {
+        if constexpr (WARP_LINE) __syncwarp();
+        else __syncthreads();
     }
-    // whether this thread reports its warp's part of line c
-    static __device__ __forceinline__ bool leader(int tid) { return MODE == 0 ? tid % 32 == 0 : tid % 32 < C; }
 
-    // Passes P.. on v; red: one word per line and pass (zeroed), c: the line
+    // Passes P.. on v (below 2^58 at P = 0); the last one's outputs idxD +
+    // k NS, k < R, go to store(idxD, u, q).
     template <int P, typename Store>
-    static __device__ __forceinline__ void run(Fx (&v)[E], int t, int c, int tid, Fx *xs, int base, const int4 *__restrict__ W,
+    static __device__ __forceinline__ void run(Fx (&v)[E], int t, int c, int tid, int C, Fx *xs, const int4 *__restrict__ W,
                                                uint32_t *red, FxLine &ln, Store &store) {
         typedef typename S::template Pass<P> PP;
+        const int base = c * stride(C);
         uint32_t bits = 0;
 #pragma unroll
         for (int q = 0; q < PP::NB; q++) {
@@ -272,7 +309,7 @@ template <int L, int MODE, int SIGN> struct FxStock {
             fx_dft<PP::R, SIGN>(u);
             const int idxD = (j - jm) * PP::R + jm;
             if constexpr (PP::LAST) {
-                store(idxD, u, q);  // outputs idxD + k NS, k < R
+                store(idxD, u, q);
             } else {
 #pragma unroll
                 for (int k = 0; k < PP::R; k++) {
@@ -283,20 +320,10 @@ template <int L, int MODE, int SIGN> struct FxStock {
         }
         if constexpr (!PP::LAST) {
             typedef typename S::template Pass<P + 1> NP;
-            bits = warp_or(bits);
-            if constexpr (WARP_LINE) {
-                __syncwarp();
-            } else {
-                if (leader(tid)) atomicOr(&red[(P + 1) * C + c], bits);
-                __syncthreads();
-                bits = red[(P + 1) * C + c];
-            }
+            bits = line_red<false>(bits, P + 1, c, tid, C, red);
 #pragma unroll
             for (int m = 0; m < E; m++) v[m] = xs[base + pad(t + m * TL)];
-            if constexpr (P + 2 < NPASS) {  // the next pass writes the buffer again
-                if constexpr (WARP_LINE) __syncwarp();
-                else __syncthreads();
-            }
+            if constexpr (P + 2 < NPASS) line_sync();  // the next pass writes the buffer again
             int s = fx_norm_shift(bits);
             ln.ex += s + 2;  // the twiddle products divide by 4
             if (s < 0) {
@@ -308,45 +335,45 @@ template <int L, int MODE, int SIGN> struct FxStock {
             const long long r0 = fx_half(s + 2), r1 = fx_half(s);
 #pragma unroll
             for (int m = 0; m < E; m++) v[m] = m < NP::NB ? fx_shr(v[m], s + 2, r0) : fx_shr(v[m], s, r1);
-            run<P + 1>(v, t, c, tid, xs, base, W, red, ln, store);
+            run<P + 1>(v, t, c, tid, C, xs, W, red, ln, store);
         }
     }
 };
 
-// One tile of C lines per CTA (several CTAs share an SM: their loads overlap
-// each other's arithmetic).
+// One tile of C = blockDim / TL lines per CTA (several CTAs share an SM:
+// their loads overlap each other's arithmetic).
 template <int L, int MODE, int SIGN, bool TW>
-__global__ void __launch_bounds__(FxStock<L, MODE, SIGN>::NT, FxStock<L, MODE, SIGN>::MINB)
+__global__ void __launch_bounds__(FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::NT, FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::MINB)
     fix_kernel(const double2 *__restrict__ in, double2 *__restrict__ out, StockParams p, const double2 *__restrict__ W,
                const double2 *__restrict__ Whi, const double2 *__restrict__ Wlo, const int4 *__restrict__ Wq,
                const int4 *__restrict__ Whiq, const int4 *__restrict__ Wloq) {
-    typedef FxStock<L, MODE, SIGN> F;
+    typedef FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)> F;
     typedef typename F::S S;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ uint32_t red[(F::NPASS + 1) * F::C];
+    __shared__ uint32_t red[F::RED];
     Fx *xs = reinterpret_cast<Fx *>(smem_raw);
-    const int tid = threadIdx.x;
-    const int c = MODE == 0 ? tid / F::TL : tid % F::C, t = MODE == 0 ? tid % F::TL : tid / F::C;
+    const int tid = threadIdx.x, NT = blockDim.x, C = NT / F::TL;
+    const int c = MODE == 0 ? tid / F::TL : tid & (C - 1), t = MODE == 0 ? tid % F::TL : tid / C;
     const int64_t ntiles = gridDim.x;
     const int64_t tile = p.reverse ? ntiles - 1 - blockIdx.x : blockIdx.x;
-    const int64_t b0 = tile * F::C, b = b0 + c;
+    const int64_t b0 = tile * C, b = b0 + c;
     const bool valid = b < p.nlines;
     if constexpr (!F::WARP_LINE)
-        for (int i = tid; i < (F::NPASS + 1) * F::C; i += F::NT) red[i] = 0;
-    const int base = c * F::LP;
+        for (int i = tid; i < F::RED; i += NT) red[i] = 0;
+    const int stride = F::stride(C), base = c * stride;
     double2 d[16];
     if constexpr (MODE == 2) {
         double2 *sd = reinterpret_cast<double2 *>(smem_raw);
         double2 x[16];
 #pragma unroll
         for (int u = 0; u < 16; u++) {
-            const int i = tid + u * F::NT, cc = i / L, e = i % L;
+            const int i = tid + u * NT, cc = i / L, e = i % L;
             x[u] = b0 + cc < p.nlines ? in[line_off(p.lin, b0 + cc) + e] : make_double2(0, 0);
         }
 #pragma unroll
         for (int u = 0; u < 16; u++) {
-            const int i = tid + u * F::NT, cc = i / L, e = i % L;
-            sd[cc * F::LP + pad(e)] = x[u];
+            const int i = tid + u * NT, cc = i / L, e = i % L;
+            sd[cc * stride + pad(e)] = x[u];
         }
         __syncthreads();
 #pragma unroll
@@ -363,9 +390,9 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN>::NT, FxStock<L, MODE, S
     for (int m = 0; m < 16; m++)
         mx = max(mx, max((uint32_t)__double2hiint(d[m].x) << 1, (uint32_t)__double2hiint(d[m].y) << 1));
     const bool special = mx >= 0xffe00000u;  // an infinity or a NaN
-    mx = F::warp_max(mx);
+    mx = F::template warp_red<true>(mx, C);
     if constexpr (!F::WARP_LINE)
-        if (F::leader(tid)) atomicMax(&red[c], mx);
+        if (MODE == 0 ? tid % 32 == 0 : tid % 32 < C) atomicMax(&red[c], mx);
     // (MODE 2: this barrier also ends the reads of the staged lines)
     const bool fp = __syncthreads_or(special);
     double2 *dst = out + (valid ? line_off(p.lout, b) : 0);
@@ -448,22 +475,32 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN>::NT, FxStock<L, MODE, S
             for (int k = 0; k < LP_::R; k++) st_hint(&dst[(int64_t)(pos + k * LP_::NS) * oes], r[k], spol);
         }
     };
-    F::template run<0>(v, t, c, tid, xs, base, Wq, red, ln, store);
+    F::template run<0>(v, t, c, tid, C, xs, Wq, red, ln, store);
+}
+
+// Lines per CTA: the most that fit, halved while the grid has fewer CTAs than
+// two per SM (whole warps, and 64-byte segments of the column modes, stay).
+inline int fix_lines(int64_t nlines, int most, int least, int sms) {
+    int C = most;
+    while (C > least && (nlines + C - 1) / C < 2 * (int64_t)sms) C /= 2;
+    return C;
 }
 
 template <int L> struct FixLaunch {
     template <int MODE, int SIGN, bool TW>
     static void one(const double2 *in, double2 *out, const StockParams &p, const double2 *W, const double2 *Whi, const double2 *Wlo,
-                    const int4 *Wq, const int4 *Whiq, const int4 *Wloq, cudaStream_t s) {
-        typedef FxStock<L, MODE, SIGN> F;
+                    const int4 *Wq, const int4 *Whiq, const int4 *Wloq, int sms, cudaStream_t s) {
+        constexpr int CM = FxCfg::C(L, MODE);
+        typedef FxStock<L, MODE, SIGN, CM> F;
         auto kern = fix_kernel<L, MODE, SIGN, TW>;
         static bool attr = false;
         if (!attr) {
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::SMEM);
             attr = true;
         }
-        const int64_t ntiles = (p.nlines + F::C - 1) / F::C;
-        kern<<<(unsigned)ntiles, F::NT, F::SMEM, s>>>(in, out, p, W, Whi, Wlo, Wq, Whiq, Wloq);
+        const int C = fix_lines(p.nlines, CM, std::min(CM, std::max(F::CMIN, MODE == 0 ? 1 : 4)), sms);
+        const int64_t ntiles = (p.nlines + C - 1) / C;
+        kern<<<(unsigned)ntiles, C * F::TL, (size_t)C * F::stride(C) * sizeof(Fx), s>>>(in, out, p, W, Whi, Wlo, Wq, Whiq, Wloq);
     }
     template <int MODE, int SIGN, typename... A> static void tw(const double2 *in, double2 *out, const StockParams &p, A... a) {
         if constexpr (MODE == 1) {

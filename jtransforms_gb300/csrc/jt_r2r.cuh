@@ -34,6 +34,8 @@
 #include "jt_device.cuh"
 #include "jt_stockham.cuh"
 
+#include <cmath>
+
 namespace jt {
 
 #define C2 typename V2<T>::t
@@ -57,6 +59,25 @@ struct R2rParams {
     int vec_in, vec_out;    // 1: contiguous lines whose scalar pairs (2j, 2j+1) are aligned
                             // complex values (the register form moves them as pairs)
 };
+
+// Multipliers of the fixed-point kernels' outputs (jt_fixr2r.cuh): 2^e2, times
+// k / 2^62 (0.5 <= k / 2^62 < 1) when k is not zero; e20, k0: that of number 0
+// (the DCT's C_0).  c0: what the inverse DCT's C_0 is multiplied with first
+// (0: 1, 1: sqrt(2), 2: 2).
+struct FixR2rScale {
+    int e2, e20, c0;
+    long long k, k0;
+};
+// m as such a pair.  The orthonormal factors of power-of-two lengths are
+// powers of two or those times sqrt(1/2), which is kept to 62 bits.
+inline void fix_scale(double m, int *e2, long long *k) {
+    const double mant = std::frexp(m, e2), root = 0.70710678118654752440;
+    *k = std::fabs(mant - root) < 4e-16 ? 3260954456333195553ll : (long long)std::ldexp(mant, 62);
+    if (mant == 0.5) {
+        *k = 0;
+        --*e2;
+    }
+}
 
 // e^{-2 pi i k/n}, 0 < k < h, from Wr (k <= n/4)
 template <typename T> __device__ __forceinline__ C2 r2r_wr(const C2 *__restrict__ Wr, int k, int h) {
@@ -330,13 +351,11 @@ template <typename T, int H, int OP> struct R2rReg {
 };
 
 template <typename T, int H, int OP>
-__global__ void __launch_bounds__(R2rReg<T, H, OP>::S::NT)
-    r2r_reg_kernel(const T *in, T *out, R2rParams p, const C2 *__restrict__ Wp, const C2 *__restrict__ Wr,
-                   const C2 *__restrict__ Wd) {
+__device__ __forceinline__ void r2r_reg_body(const T *in, T *out, const R2rParams &p, const C2 *__restrict__ Wp,
+                                             const C2 *__restrict__ Wr, const C2 *__restrict__ Wd, unsigned char *smem_raw) {
     typedef R2rReg<T, H, OP> G;
     typedef typename G::S S;
     constexpr int n = 2 * H, RX = G::RX;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     C2 *buf = reinterpret_cast<C2 *>(smem_raw);
     // lines per CTA: p.C (at most S::C), blockDim = p.C * TL
     const int tid = threadIdx.x, NT = blockDim.x;
@@ -497,8 +516,16 @@ __global__ void __launch_bounds__(R2rReg<T, H, OP>::S::NT)
     r2r_store<OP, T>(buf, RX, out, p, b0, lines, Wr, Wd, mult, mult0, tid, NT);
 }
 
-// Launches the register form for half length H (T's instantiations live in
-// jt_r2r_f32.cu / jt_r2r_f64.cu); false when H has none.
+template <typename T, int H, int OP>
+__global__ void __launch_bounds__(R2rReg<T, H, OP>::S::NT)
+    r2r_reg_kernel(const T *in, T *out, R2rParams p, const C2 *__restrict__ Wp, const C2 *__restrict__ Wr,
+                   const C2 *__restrict__ Wd) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    r2r_reg_body<T, H, OP>(in, out, p, Wp, Wr, Wd, smem_raw);
+}
+
+// Launches the register form for half length H (floats: jt_r2r_f32.cu; the
+// double lines run jt_fixr2r.cuh); false when H has none.
 template <typename T, int H> struct R2rRegLaunch {
     template <int OP>
     static void one(const T *in, T *out, const R2rParams &p, const C2 *Wp, const C2 *Wr, const C2 *Wd, cudaStream_t s) {

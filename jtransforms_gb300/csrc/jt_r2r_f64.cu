@@ -1,34 +1,19 @@
-// jt_r2r_f64.cu -- instantiations of the register-form DCT/DST/DHT line
-// kernels (jt_r2r.cuh) for double, half lengths 16..4096.
-#include "jt_r2r.cuh"
+// jt_r2r_f64.cu -- instantiations of the DCT/DST/DHT and packed real line
+// kernels for double (jt_fixr2r.cuh), half lengths 16..128.
+#include "jt_fixr2r.cuh"
 
 namespace jt {
 
-// Rows (lines) per CTA of the register form for half length H; 0 when H has none.
-int r2r_reg_lines(int H, const double *) {
+bool fix_r2r_launch(int H, int op, bool strided, const double *in, double *out, const R2rParams &p, const FixR2rScale &fs,
+                    const double2 *Wp, const double2 *Wr, const double2 *Wd, const int4 *Wpq, const int4 *Wrq, const int4 *Wdq,
+                    int sms, cudaStream_t s) {
+#define JT_RCASE(HH) \
+    case HH: return FixR2rLaunch<HH>::go(op, strided, in, out, p, fs, Wp, Wr, Wd, Wpq, Wrq, Wdq, sms, s);
     switch (H) {
-        case 16: return Stockham<double, 16, 0, -1>::C;
-        case 32: return Stockham<double, 32, 0, -1>::C;
-        case 64: return Stockham<double, 64, 0, -1>::C;
-        case 128: return Stockham<double, 128, 0, -1>::C;
-        case 256: return Stockham<double, 256, 0, -1>::C;
-        case 512: return Stockham<double, 512, 0, -1>::C;
-        case 1024: return Stockham<double, 1024, 0, -1>::C;
-        case 2048: return Stockham<double, 2048, 0, -1>::C;
-        case 4096: return Stockham<double, 4096, 0, -1>::C;
-        default: return 0;
-    }
-}
-
-bool r2r_reg_launch(int H, int op, const double *in, double *out, const R2rParams &p, const V2<double>::t *Wp,
-                    const V2<double>::t *Wr, const V2<double>::t *Wd, cudaStream_t s) {
-#define JT_RCASE(HH)                                                       \
-    case HH:                                                               \
-        R2rRegLaunch<double, HH>::go(op, in, out, p, Wp, Wr, Wd, s);          \
-        return true;
-    switch (H) {
-        JT_RCASE(16) JT_RCASE(32) JT_RCASE(64) JT_RCASE(128) JT_RCASE(256) JT_RCASE(512) JT_RCASE(1024) JT_RCASE(2048)
-        JT_RCASE(4096)
+        JT_RCASE(16)
+        JT_RCASE(32)
+        JT_RCASE(64)
+        JT_RCASE(128)
         default: return false;
     }
 #undef JT_RCASE

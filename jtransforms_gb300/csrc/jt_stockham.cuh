@@ -1,4 +1,6 @@
-// jt_stockham.cuh -- power-of-two complex FFT lines held in registers.
+// jt_stockham.cuh -- power-of-two complex FFT lines held in registers: the
+// float lines' kernels, and the FP64 passes that the double lines' kernels
+// (jt_fix64.cuh) keep for infinities and NaNs.
 //
 // One CTA transforms C lines of compile-time length L.  Each thread owns
 // E = 16 elements of one line (t, t+TL, ..., t+15*TL with TL = L/16): the

@@ -108,3 +108,87 @@ def test_two_and_three_passes(split, inverse):
             assert rel_l2(got[b], want[b]) <= tol(1 << lg, np.float64)
     finally:
         N.load().jt_set_split(N.FLOAT64, lg, -1, 0, 0)
+
+
+def _r2r_want(kind, fwd, x):
+    import scipy.fft as sfft
+    if kind == "dht":
+        z = np.fft.fft(x, axis=-1)
+        return (z.real - z.imag) / (1 if fwd else x.shape[-1])
+    return (sfft.dct if kind == "dct" else sfft.dst)(x, type=2 if fwd else 3, norm="ortho", axis=-1)
+
+
+@pytest.mark.parametrize("lg", range(5, 14))
+@pytest.mark.parametrize("kind", ["dct", "dst", "dht"])
+@pytest.mark.parametrize("fwd", [True, False])
+@pytest.mark.parametrize("off", [0, 1])
+def test_r2r_rows(lg, kind, fwd, off):
+    """Rows of the half lengths 16..4096, at even and odd offsets, 20 orders
+    of magnitude and a row of zeros among them, one row with an infinity."""
+    import torch
+    from jtransforms_gb300 import _native as N
+    n = 1 << lg
+    batch = max(4, 9000 // n)
+    x = np.random.default_rng(lg).standard_normal((batch, n)) * (10.0 ** np.linspace(-10, 10, batch))[:, None]
+    x[2] = 0
+    plan = N.Plan({"dct": N.DCT, "dst": N.DST, "dht": N.DHT}[kind], N.FLOAT64, [n])
+    for special in (False, True):
+        if special:
+            x[3, n // 3] = np.inf
+        buf = np.full(off + batch * n + 3, 5.0)
+        buf[off:off + batch * n] = x.ravel()
+        dev = torch.from_numpy(buf).cuda()
+        plan.execute(N.FORWARD if fwd else N.INVERSE, dev, off, kind != "dht" or not fwd, batch=batch, dist=n)
+        out = dev.cpu().numpy()
+        got = out[off:off + batch * n].reshape(batch, n)
+        assert np.all(out[:off] == 5.0) and np.all(out[off + batch * n:] == 5.0)
+        for b in range(batch):
+            if special and b == 3:
+                assert not np.isfinite(got[b]).any()
+            else:
+                assert rel_l2(got[b], _r2r_want(kind, fwd, x[b])) <= tol(n, np.float64)
+
+
+@pytest.mark.parametrize("n,cols", [(32, 150), (64, 33), (256, 40), (512, 17), (1024, 9), (2048, 6), (4096, 5), (8192, 3)])
+@pytest.mark.parametrize("kind", ["dct", "dst", "dht"])
+def test_r2r_columns(n, cols, kind):
+    import torch
+    import jtransforms_gb300 as J
+    x = np.random.default_rng(n).standard_normal((n, cols))
+    f = getattr(J, "Double%s_2D" % kind.upper())(n, cols)
+    dev = torch.from_numpy(x.copy().ravel()).cuda()
+    if kind == "dht":
+        f.forward(dev)
+        z = np.fft.fft2(x)
+        want = z.real - z.imag
+    else:
+        f.forward(dev, True)
+        want = _r2r_want(kind, True, _r2r_want(kind, True, x).T).T
+    assert rel_l2(dev.cpu().numpy().reshape(n, cols), want) <= tol(x.size, np.float64)
+    f.inverse(dev, True)
+    assert rel_l2(dev.cpu().numpy().reshape(n, cols), x) <= 2 * tol(x.size, np.float64)
+
+
+@pytest.mark.parametrize("lg", range(5, 14))
+@pytest.mark.parametrize("off", [0, 2])
+def test_packed_real_rows(lg, off):
+    import torch
+    import jtransforms_gb300 as J
+    from jtransforms_gb300 import _native as N
+    n = 1 << lg
+    batch = max(3, 9000 // n)
+    x = np.random.default_rng(lg).standard_normal((batch, n)) * (10.0 ** np.linspace(-10, 10, batch))[:, None]
+    f = J.DoubleFFT_1D(n)
+    dev = torch.from_numpy(np.concatenate([np.zeros(off), x.ravel()])).cuda()
+    f.plan.execute(N.REAL_FORWARD, dev, off, False, batch=batch, dist=n)
+    got = dev.cpu().numpy()[off:].reshape(batch, n)
+    F = np.fft.rfft(x, axis=1)
+    want = np.empty_like(x)
+    want[:, 0], want[:, 1] = F[:, 0].real, F[:, n // 2].real
+    want[:, 2::2], want[:, 3::2] = F[:, 1:n // 2].real, F[:, 1:n // 2].imag
+    for b in range(batch):
+        assert rel_l2(got[b], want[b]) <= tol(n, np.float64)
+    f.plan.execute(N.REAL_INVERSE, dev, off, True, batch=batch, dist=n)
+    back = dev.cpu().numpy()[off:].reshape(batch, n)
+    for b in range(batch):
+        assert rel_l2(back[b], x[b]) <= 2 * tol(n, np.float64)
