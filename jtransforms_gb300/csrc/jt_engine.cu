@@ -18,6 +18,7 @@
 #include "jt_device.cuh"
 #include "jt_stockham.cuh"
 #include "jt_batch.cuh"
+#include "jt_mixed.cuh"
 #include "jt_r2r.cuh"
 #include "jt_chirp.cuh"
 #include "jt_plan_table.h"
@@ -180,6 +181,15 @@ static std::atomic<int64_t> g_opt_arena_limit{0};
 static std::atomic<int> g_opt_batch_wait{1 << 24};
 static std::atomic<int> g_opt_batch_inject{0};
 
+// Mixed-radix lines (jt_mixed_fwd.cu, jt_mixed_inv.cu).
+void mix_setup_fwd(int smem_optin);
+void mix_setup_inv(int smem_optin);
+void mix_table(float2 *out, const MixParams &p, int count, cudaStream_t s);
+void mix_launch_fwd(int mode, const float2 *in, float2 *out, const MixParams &p, const float2 *tw, const float2 *Whi,
+                    const float2 *Wlo, unsigned grid, int threads, size_t smem, cudaStream_t s);
+void mix_launch_inv(int mode, const float2 *in, float2 *out, const MixParams &p, const float2 *tw, const float2 *Whi,
+                    const float2 *Wlo, unsigned grid, int threads, size_t smem, cudaStream_t s);
+
 static int device_init() {
     std::call_once(g_dev_once, [] {
         int n = 0;
@@ -205,6 +215,8 @@ static int device_init() {
         cudaFuncSetAttribute(fft_tile_kernel<1, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(fft_tile_kernel<-1, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(fft_tile_kernel<1, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
+        mix_setup_fwd(g_smem_optin);
+        mix_setup_inv(g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT3, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DHT, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
@@ -331,6 +343,62 @@ static int radix_order(int64_t n, bool f32) {
     return f32 ? kRadixOrderF32[lg] : kRadixOrderF64[lg];
 }
 
+// Radices of the mixed-radix kernel's passes (jt_mixed.cuh): the fewest of
+// 2..16, of those the smallest sum; empty for a prime factor above 13.  Odd
+// ones come first (largest first): the first pass writes shared memory in
+// strides of its radix, which odd strides do without bank conflicts; then
+// twice an odd number (two ways), the rest from the smallest.
+static void mix_search(int n, std::vector<int> &cur, int largest, std::vector<int> &best, int &best_sum, int sum) {
+    if (n == 1) {
+        if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && sum < best_sum)) {
+            best = cur;
+            best_sum = sum;
+        }
+        return;
+    }
+    if (!best.empty() && cur.size() >= best.size()) return;
+    for (int r = std::min(largest, 16); r >= 2; r--)
+        if (n % r == 0) {
+            cur.push_back(r);
+            mix_search(n / r, cur, r, best, best_sum, sum + r);
+            cur.pop_back();
+        }
+}
+static std::vector<int> mix_radices(int64_t n) {
+    int64_t m = n;
+    for (int p : {2, 3, 5, 7, 11, 13})
+        while (m % p == 0) m /= p;
+    if (m != 1 || n < 2 || n > 8192) return {};
+    std::vector<int> cur, best;
+    int sum = 0;
+    mix_search((int)n, cur, 16, best, sum, 0);
+    std::sort(best.begin(), best.end(), [](int a, int b) {
+        auto rank = [](int r) { return (r & 1) ? 0 : (r & 2) ? 1 : 2; };
+        if (rank(a) != rank(b)) return rank(a) < rank(b);
+        return (a & 1) ? a > b : a < b;
+    });
+    return best;
+}
+// A plan's parts of MixParams; returns the table's entries.
+static int mix_plan(int n, const std::vector<int> &R, MixParams *p) {
+    memset(p, 0, sizeof(*p));
+    p->L = n;
+    p->npass = (int)R.size();
+    int ns = 1, off = 0;
+    auto magic = [](int d) { return (uint32_t)(((uint64_t)1 << 32) / (uint64_t)d + 1); };
+    for (int i = 0; i < p->npass; i++) {
+        p->R[i] = R[i];
+        p->Ns[i] = ns;
+        p->mNs[i] = ns > 1 ? magic(ns) : 0;
+        p->mNb[i] = n / R[i] > 1 ? magic(n / R[i]) : 0;
+        p->toff[i] = off;
+        if (i > 0) off += (ns * (R[i] - 1) + 1) & ~1;  // even: the pairs are read 16 bytes at a time
+        ns *= R[i];
+    }
+    p->Lp = n | 1;  // odd: columns' neighbouring lines in neighbouring banks
+    return off;
+}
+
 template <typename T> struct Fft1 {
     typedef typename V2<T>::t C2;
     int64_t n = 0;
@@ -395,8 +463,9 @@ template <typename T> struct Fft1 {
     bool cols_ok() const { return algo == ALG_DIRECT && (reg ? n <= 4096 : true); }
 
     // fixed: followed by the same roots in fixed point (doubles only)
-    static int make_roots(C2 **out, int64_t count, int64_t num, int64_t den, bool fixed = false) {
-        JT_CU(cudaMalloc(out, sizeof(C2) * std::max<int64_t>(count, 1) * (fixed ? 2 : 1)));
+    // and by room for `more` entries
+    static int make_roots(C2 **out, int64_t count, int64_t num, int64_t den, bool fixed = false, int64_t more = 0) {
+        JT_CU(cudaMalloc(out, sizeof(C2) * (std::max<int64_t>(count, 1) * (fixed ? 2 : 1) + more)));
         roots_kernel<T><<<(unsigned)cdiv(count, 256), 256, 0, g_setup>>>(*out, count, num, den, fixed);
         g_launches++;
         JT_CU(cudaGetLastError());
@@ -435,11 +504,71 @@ template <typename T> struct Fft1 {
         return t[0] >= 0 ? t : nullptr;
     }
 
+    // mixed-radix kernel (jt_mixed.cuh): its part of the launch parameters and
+    // its pass table, which follows W; npass = 0: lengths it does not take
+    MixParams mix{};
+    C2 *Wm = nullptr;
+
     int init_direct() {
         algo = ALG_DIRECT;
         JT_TRY(set_reg(reg_ok(n)));
-        if (!reg) radix = direct_radices(n, radix_order(n, sizeof(T) == 4));
-        return make_roots(&W, n, 1, n);
+        if (reg) return make_roots(&W, n, 1, n);
+        radix = direct_radices(n, radix_order(n, sizeof(T) == 4));
+        if constexpr (sizeof(T) == 4) {
+            const std::vector<int> R = mix_radices(n);
+            const int count = R.empty() ? 0 : mix_plan((int)n, R, &mix);
+            JT_TRY(make_roots(&W, n, 1, n, false, count + 1));
+            if (count) {
+                Wm = W + ((n + 1) & ~(int64_t)1);  // 16-byte aligned
+                mix_table(Wm, mix, count, g_setup);
+                g_launches++;
+                JT_CU(cudaGetLastError());
+            }
+            return JT_OK;
+        } else {
+            return make_roots(&W, n, 1, n);
+        }
+    }
+
+    // Line pass of the mixed-radix kernel.  C lines per CTA: about 4096 numbers
+    // of lines below 96 (rows of 24: 4.7 TB/s, 3.8 with 1024), about 1024, one
+    // line at least, of longer ones (rows of 1080: 4.26 TB/s, 3.57 with 4096:
+    // the barriers hold up fewer threads); at least 16 columns (128-byte runs)
+    // of strided lines where two CTAs still share an SM; and fewer (down to 4
+    // columns) while the grid has fewer CTAs than two per SM.
+    int exec_mix(Ctx &ctx, const C2 *in, C2 *out, int64_t nlines, const Layout &lin, const Layout &lout, int sign, double scale,
+                 int64_t tw_n, int64_t tw_inner, const C2 *Whi_, const C2 *Wlo_, int tw_lo_bits) const {
+        MixParams p = mix;
+        const int mode = lin.estride != 1 ? 1 : lout.estride != 1 ? 2 : 0;
+        const bool strided = mode != 0;
+        const size_t per_line = (size_t)p.Lp * sizeof(C2) * (p.npass > 2 ? 2 : 1);
+        const int probe = g_opt_tile_elems.load();
+        int C = (int)std::max<int64_t>(1, (probe > 0 ? probe : n < 96 ? 4096 : 1024) / n);
+        if (strided) C = std::max(C, 16);
+        while (strided && C > 8 && per_line * C > 110 * 1024) C /= 2;
+        C = std::min(C, (int)std::max<size_t>(1, (size_t)g_smem_optin / per_line));
+        while (C > (strided ? 4 : 1) && cdiv(nlines, C) < 2 * (int64_t)g_sms) C /= 2;
+        if ((int64_t)C > nlines) C = (int)nlines;
+        p.C = C;
+        p.mC = C > 1 ? (uint32_t)(((uint64_t)1 << 32) / (uint64_t)C + 1) : 0;
+        p.nlines = nlines;
+        p.lin = lin;
+        p.lout = lout;
+        p.scale = (float)scale;
+        p.do_scale = scale != 1.0;
+        p.tw_n = tw_n;
+        p.tw_inner = tw_inner;
+        p.tw_lo_bits = tw_lo_bits;
+        if (ctx.dry) return JT_OK;
+        const int64_t grid = cdiv(nlines, C);
+        if (grid > 0x7fffffff) return JT_ETOOBIG;
+        // threads: the pass with most butterflies in whole rounds
+        const int most = C * (int)(n / *std::min_element(p.R, p.R + p.npass));
+        const int rounds = (int)cdiv(most, n >= 2048 ? JT_MIX_THREADS : 256);
+        const int threads = (int)cdiv(cdiv(most, rounds), 32) * 32;
+        (sign < 0 ? mix_launch_fwd : mix_launch_inv)(mode, in, out, p, Wm, Whi_, Wlo_, (unsigned)grid, threads, per_line * C, ctx.s);
+        g_launches++;
+        return JT_OK;
     }
 
     // n = n1 (column pass, four-step twiddle fused) x n2 (transposing row pass)
@@ -454,6 +583,7 @@ template <typename T> struct Fft1 {
         for (Fft1 *sub : {pa.get(), pb.get()})
             if (sub->reg && sub->n > 4096) {
                 sub->reg = false;
+                sub->mix.npass = 0;
                 sub->radix = direct_radices(sub->n, radix_order(sub->n, sizeof(T) == 4));
             }
         return make_twiddle_pair(n, &Whi, &Wlo, &lo_bits);
@@ -754,6 +884,12 @@ template <typename T> struct Fft1 {
                 g_launches++;
                 return JT_OK;
             }
+        }
+        // floats with prime factors up to 13: the mixed-radix kernel, but for
+        // rows of one pass, which the tile kernel moves in whole runs
+        if constexpr (sizeof(T) == 4) {
+            if (mix.npass > 1 || (mix.npass == 1 && lin.estride != 1 && lout.estride != 1))
+                return exec_mix(ctx, in, out, nlines, lin, lout, sign, scale, tw_n, tw_inner, Whi_, Wlo_, tw_lo_bits);
         }
         const int L = (int)n;
         const int Lp = padded_len(L);

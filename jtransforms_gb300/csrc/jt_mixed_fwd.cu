@@ -1,0 +1,24 @@
+// jt_mixed_fwd.cu -- the mixed-radix line kernel (jt_mixed.cuh) for float,
+// forward.
+#include "jt_mixed.cuh"
+
+namespace jt {
+
+void mix_launch_fwd(int mode, const float2 *in, float2 *out, const MixParams &p, const float2 *tw, const float2 *Whi,
+                     const float2 *Wlo, unsigned grid, int threads, size_t smem, cudaStream_t s) {
+    if (mode == 0) mix_kernel<-1, 0><<<grid, threads, smem, s>>>(in, out, p, tw, Whi, Wlo);
+    else if (mode == 1) mix_kernel<-1, 1><<<grid, threads, smem, s>>>(in, out, p, tw, Whi, Wlo);
+    else mix_kernel<-1, 2><<<grid, threads, smem, s>>>(in, out, p, tw, Whi, Wlo);
+}
+
+void mix_setup_fwd(int smem_optin) {
+    cudaFuncSetAttribute(mix_kernel<-1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
+    cudaFuncSetAttribute(mix_kernel<-1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
+    cudaFuncSetAttribute(mix_kernel<-1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin);
+}
+
+void mix_table(float2 *out, const MixParams &p, int count, cudaStream_t s) {
+    mix_table_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(out, p, count);
+}
+
+}  // namespace jt
