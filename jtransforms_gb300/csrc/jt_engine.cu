@@ -473,10 +473,10 @@ template <typename T> struct Fft1 {
     }
 
     static int make_pass_table(C2 **out, int L) {
-        const int count = stock_tw_count(L);
+        const int E = sizeof(T) == 8 ? fx_elems(L) : std::min(L, 16), count = stock_tw_count(L, E);
         JT_CU(cudaMalloc(out, sizeof(C2) * std::max(count, 1) * (sizeof(T) == 8 ? 2 : 1)));
         if (count > 0) {
-            passtw_kernel<T><<<(unsigned)cdiv(count, 256), 256, 0, g_setup>>>(*out, L);
+            passtw_kernel<T><<<(unsigned)cdiv(count, 256), 256, 0, g_setup>>>(*out, L, E);
             g_launches++;
             JT_CU(cudaGetLastError());
         }
@@ -1388,7 +1388,7 @@ static int r2r_fused(Ctx &ctx, int op, const Real1<T> *rf, const T *in, T *out, 
             fix_scale(mult, &fs.e2, &fs.k);
             fix_scale(mult0, &fs.e20, &fs.k0);
             fs.c0 = mult0 == mult ? 0 : mult0 == 2 * mult ? 2 : 1;
-            const int4 *Wpq = (const int4 *)(rf->half->Wp + stock_tw_count((int)h)), *Wrq = (const int4 *)(rf->Wr + n / 4 + 1);
+            const int4 *Wpq = (const int4 *)(rf->half->Wp + stock_tw_count((int)h, fx_elems((int)h))), *Wrq = (const int4 *)(rf->Wr + n / 4 + 1);
             const int4 *Wdq = Wd ? (const int4 *)(Wd + n) : nullptr;
             if (!(h <= 128 ? fix_r2r_launch : fix_r2r_launch_long)((int)h, op, strided, in, out, p, fs, rf->half->Wp, rf->Wr, Wd, Wpq,
                                                                    Wrq, Wdq, g_sms, ctx.s))

@@ -226,10 +226,10 @@ __device__ __forceinline__ const int4 *fx_factor(const int4 *W, int off, int ns,
 }
 
 struct FxCfg {
-    // most lines per CTA: 128 threads of 16 numbers for short lines; of the
-    // column modes' longer ones 8 columns (128-byte segments) up to 512, fewer above
-    static constexpr int rows_C(int L) { return L >= 2048 ? 1 : 2048 / L; }
-    static constexpr int cols_C(int L) { return L <= 256 ? 2048 / L : L <= 512 ? 8 : 4096 / L < 2 ? 2 : 4096 / L; }
+    // most lines per CTA: 128 threads for short lines; of the column modes'
+    // longer ones 8 columns (128-byte segments) up to 512, fewer above
+    static constexpr int rows_C(int L) { return L >= 128 * fx_elems(L) ? 1 : 128 * fx_elems(L) / L; }
+    static constexpr int cols_C(int L) { return L <= 16 * fx_elems(L) ? 128 * fx_elems(L) / L : L <= 512 ? 8 : 4096 / L < 2 ? 2 : 4096 / L; }
     static constexpr int C(int L, int mode) { return mode == 0 ? rows_C(L) : cols_C(L); }
 };
 
@@ -237,17 +237,20 @@ struct FxCfg {
 // threads each; MODE 0 keeps a line's threads together, the column modes
 // spread the lines across a warp (c fastest).
 template <int L, int MODE, int SIGN, int CM> struct FxStock {
-    typedef Stockham<double, L, MODE, SIGN> S;
-    static constexpr int E = 16, TL = L / 16, NT = CM * TL, LP = S::LP;
+    static constexpr int E = fx_elems(L), TL = L / E, NT = CM * TL, LP = L + L / E + 1;
+    typedef Stockham<double, L, MODE, SIGN, E> S;
+    // a spare slot per E numbers: the first pass writes in strides of E
+    static __device__ __forceinline__ int pad(int i) { return i + i / E; }
     static constexpr int NPASS = S::NPASS;
     static constexpr bool WARP_LINE = MODE == 0 && TL <= 32;  // a line's threads share a warp
     // A line's stride in shared memory.  The column modes' quarter-warps (16-byte
     // accesses) cover C lines at 8 / C neighbouring positions: strides of
-    // 8 / C modulo 8 spread them over the banks (L + L/16 is a multiple of 8
+    // 8 / C modulo 8 spread them over the banks (L + L/E is a multiple of 8
     // for the lines, of 128 and more, that run with C < 8).
     static __host__ __device__ __forceinline__ int stride(int C) { return MODE == 0 || C >= 8 ? LP : LP - 1 + 8 / C; }
     static constexpr size_t SMEM = (size_t)CM * (MODE == 0 || CM >= 8 ? LP : LP - 1 + 8 / CM) * sizeof(Fx);
-    static constexpr int MINB = NT >= 512 ? 1 : 512 / NT > 8 ? 8 : 512 / NT;  // 128 registers a thread
+    // 128 registers a thread, 64 with 8 numbers
+    static constexpr int REGT = E == 16 ? 512 : 1024, MINB = NT >= REGT ? 1 : REGT / NT > 16 ? 16 : REGT / NT;
     static constexpr int RED = WARP_LINE ? 1 : (NPASS + 2) * CM;  // words of `red`
 
     // fewest lines per CTA: whole warps
@@ -361,33 +364,33 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::NT,
     if constexpr (!F::WARP_LINE)
         for (int i = tid; i < F::RED; i += NT) red[i] = 0;
     const int stride = F::stride(C), base = c * stride;
-    double2 d[16];
+    double2 d[F::E];
     if constexpr (MODE == 2) {
         double2 *sd = reinterpret_cast<double2 *>(smem_raw);
-        double2 x[16];
+        double2 x[F::E];
 #pragma unroll
-        for (int u = 0; u < 16; u++) {
+        for (int u = 0; u < F::E; u++) {
             const int i = tid + u * NT, cc = i / L, e = i % L;
             x[u] = b0 + cc < p.nlines ? in[line_off(p.lin, b0 + cc) + e] : make_double2(0, 0);
         }
 #pragma unroll
-        for (int u = 0; u < 16; u++) {
+        for (int u = 0; u < F::E; u++) {
             const int i = tid + u * NT, cc = i / L, e = i % L;
-            sd[cc * stride + pad(e)] = x[u];
+            sd[cc * stride + F::pad(e)] = x[u];
         }
         __syncthreads();
 #pragma unroll
-        for (int m = 0; m < 16; m++) d[m] = sd[base + pad(t + m * F::TL)];
+        for (int m = 0; m < F::E; m++) d[m] = sd[base + F::pad(t + m * F::TL)];
     } else {
         const double2 *src = in + (valid ? line_off(p.lin, b) : 0);
         const int64_t es = MODE == 0 ? 1 : p.lin.estride;
 #pragma unroll
-        for (int m = 0; m < 16; m++) d[m] = valid ? src[(int64_t)(t + m * F::TL) * es] : make_double2(0, 0);
+        for (int m = 0; m < F::E; m++) d[m] = valid ? src[(int64_t)(t + m * F::TL) * es] : make_double2(0, 0);
         if constexpr (!F::WARP_LINE) __syncthreads();  // red is zeroed
     }
     uint32_t mx = 0;
 #pragma unroll
-    for (int m = 0; m < 16; m++)
+    for (int m = 0; m < F::E; m++)
         mx = max(mx, max((uint32_t)__double2hiint(d[m].x) << 1, (uint32_t)__double2hiint(d[m].y) << 1));
     const bool special = mx >= 0xffe00000u;  // an infinity or a NaN
     mx = F::template warp_red<true>(mx, C);
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::NT,
             if (p.do_scale) val = cscale<double>(val, p.scale);
             if (valid) st_hint(&dst[(int64_t)pos * oes], val, spol);
         };
-        PadIdx xi{base};
+        PadIdx xi{c * S::LP};
         S::run_all(d, t, reinterpret_cast<double2 *>(smem_raw), xi, W, store);
         return;
     }
@@ -419,11 +422,11 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::NT,
     if (__any_sync(0xffffffffu, ln.pre != 0)) {
         const double f = fx_pre(ln.pre);
 #pragma unroll
-        for (int m = 0; m < 16; m++) d[m] = cscale<double>(d[m], f);
+        for (int m = 0; m < F::E; m++) d[m] = cscale<double>(d[m], f);
     }
-    Fx v[16];
+    Fx v[F::E];
 #pragma unroll
-    for (int m = 0; m < 16; m++) v[m] = Fx{fx_from(d[m].x, ln), fx_from(d[m].y, ln)};
+    for (int m = 0; m < F::E; m++) v[m] = Fx{fx_from(d[m].x, ln), fx_from(d[m].y, ln)};
     // four-step twiddle w^{pos j2} of the last pass's outputs, pos = t + TL m
     // with m = q + k NB in slot q R + k: w^{t j2} g^m, g = w^{TL j2}, formed by
     // successive products (each a unit of 2^-60 off at most)

@@ -2,9 +2,9 @@
 // in one kernel each, in the 64-bit block fixed point of jt_fix64.cuh: the
 // line operations of jt_r2r.cuh for power-of-two half lengths H = 16..4096.
 //
-// A thread holds 16 of the line's H complex values, t + m H/16.  Everything
+// A thread holds E (16 or 8) of the line's H complex values, t + m H/E.  Everything
 // around the H-point FFT works on pairs (k, H - k) or (j, H - 1 - j): the
-// lower half of the line (m < 8) stays in the thread's registers and only the
+// lower half of the line (m < E/2) stays in the thread's registers and only the
 // upper half changes hands through shared memory.  Inputs come from global
 // memory into registers and outputs go from registers to global memory, in
 // runs across t (rows) or across lines (columns); nothing is staged.
@@ -24,8 +24,8 @@
 //
 // What bounded the FP64 form (jt_r2r.cuh) was the FP64 pipe; see jt_fix64.cuh.
 // Lines with an infinity or a NaN still run it.  Measured (GB300, both
-// directions): DoubleDCT_2D(1024^2) 79 us where the FP64 form took 254,
-// DoubleDHT_3D(128^3) 164 where it took 508; a quarter to a half of the error
+// directions): DoubleDCT_2D(1024^2) 74 us where the FP64 form took 254,
+// DoubleDHT_3D(128^3) 148 where it took 508; a quarter to a half of the error
 // against quad precision on 32^2..256^2 images and noise (where one
 // coefficient dominates an image's norm its last rounding decides either).
 // At these sizes a kernel is one wave of few warps and bound by their
@@ -42,8 +42,7 @@ template <int H, int MODE, int OP> struct FixR2r {
     static constexpr int SIGN = r2r_inverse(OP) ? 1 : -1;
     // most lines per CTA: 128 threads or one line; columns at least four
     // (32-byte runs)
-    static constexpr int TL = H / 16;
-    static constexpr int CM = MODE == 0 ? FxCfg::rows_C(H) : H <= 128 ? 2048 / H : H <= 256 ? 16 : H <= 512 ? 8 : 4;
+    static constexpr int CM = MODE == 0 ? FxCfg::rows_C(H) : H <= 128 ? 128 * fx_elems(H) / H : H <= 256 ? 16 : H <= 512 ? 8 : 4;
     typedef FxStock<H, MODE, SIGN, CM> F;
 };
 
@@ -51,7 +50,7 @@ template <int H, int MODE, int OP> struct FixR2r {
 template <int H, int OP>
 __device__ __noinline__ void fix_r2r_fp64(const double *in, double *out, const R2rParams &p, const double2 *Wp, const double2 *Wr,
                                           const double2 *Wd, unsigned char *smem) {
-    r2r_reg_body<double, H, OP>(in, out, p, Wp, Wr, Wd, smem);
+    r2r_reg_body<double, H, OP, fx_elems(H)>(in, out, p, Wp, Wr, Wd, smem);
 }
 
 template <int H, int MODE, int OP>
@@ -61,7 +60,8 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
                    const int4 *__restrict__ Wrq, const int4 *__restrict__ Wdq) {
     typedef typename FixR2r<H, MODE, OP>::F F;
     typedef typename F::S S;
-    constexpr int n = 2 * H, TL = F::TL;
+    constexpr int n = 2 * H, TL = F::TL, E = F::E, EH = E / 2;
+    auto pad = [](int i) { return F::pad(i); };
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t red[F::RED];
     Fx *xs = reinterpret_cast<Fx *>(smem_raw);
@@ -89,46 +89,46 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
     auto partner = [&](int m) -> int { return m == 0 && t == 0 ? H / 2 : H - (t + m * TL); };
 
     // ---- load -----------------------------------------------------------
-    double2 d[16];
+    double2 d[E];
     if constexpr (OP == R2R_DCT2) {
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
+        for (int m = 0; m < EH; m++) {
             const int k = t + m * TL;
             const double2 u = pair_in(4 * k), w = pair_in(4 * k + 2);
             d[m] = make_double2(u.x, w.x);
-            d[8 + m] = make_double2(w.y, u.y);  // z_{H-1-k}, for another thread
+            d[EH + m] = make_double2(w.y, u.y);  // z_{H-1-k}, for another thread
         }
         if (p.dst) {
 #pragma unroll
-            for (int m = 8; m < 16; m++) d[m] = make_double2(-d[m].x, -d[m].y);
+            for (int m = EH; m < E; m++) d[m] = make_double2(-d[m].x, -d[m].y);
         }
 #pragma unroll
-        for (int m = 0; m < 8; m++) xd[base + pad(H - 1 - t - m * TL)] = d[8 + m];
+        for (int m = 0; m < EH; m++) xd[base + pad(H - 1 - t - m * TL)] = d[EH + m];
     } else if constexpr (OP == R2R_DCT3) {
-        // d[m] = (C_k, C_{n-k}), d[8 + m] = (C_{H-k}, C_{H+k}); k = 0: (C_0, 0)
-        // and d[8] = (C_H, 0) go with H / 2's pair (C_{H/2}, C_{3H/2}), below
+        // d[m] = (C_k, C_{n-k}), d[EH + m] = (C_{H-k}, C_{H+k}); k = 0: (C_0, 0)
+        // and d[EH] = (C_H, 0) go with H / 2's pair (C_{H/2}, C_{3H/2}), below
         auto coef = [&](int k) { return one_in(p.dst ? n - 1 - k : k); };
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
+        for (int m = 0; m < EH; m++) {
             const int k = t + m * TL;
             const bool z = m == 0 && t == 0;
             d[m] = make_double2(coef(k), coef(z ? 3 * H / 2 : n - k));
-            d[8 + m] = make_double2(coef(z ? H / 2 : H - k), coef(H + k));
+            d[EH + m] = make_double2(coef(z ? H / 2 : H - k), coef(H + k));
         }
     } else if constexpr (OP == R2R_RINV) {
-        // d[m] = X_k, d[8 + m] = X_{H-k}; k = 0: (X_0, X_H), X_{H/2}
+        // d[m] = X_k, d[EH + m] = X_{H-k}; k = 0: (X_0, X_H), X_{H/2}
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
+        for (int m = 0; m < EH; m++) {
             d[m] = pair_in(2 * (t + m * TL));
-            d[8 + m] = pair_in(2 * partner(m));
+            d[EH + m] = pair_in(2 * partner(m));
         }
     } else {
 #pragma unroll
-        for (int m = 0; m < 16; m++) d[m] = pair_in(2 * (t + m * TL));
+        for (int m = 0; m < E; m++) d[m] = pair_in(2 * (t + m * TL));
     }
     uint32_t mx = 0;
 #pragma unroll
-    for (int m = 0; m < 16; m++)
+    for (int m = 0; m < E; m++)
         mx = max(mx, max((uint32_t)__double2hiint(d[m].x) << 1, (uint32_t)__double2hiint(d[m].y) << 1));
     const bool special = mx >= 0xffe00000u;  // an infinity or a NaN
     mx = F::template warp_red<true>(mx, C);
@@ -143,24 +143,24 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
     if constexpr (!F::WARP_LINE) mx = red[c];
     if constexpr (OP == R2R_DCT2) {
 #pragma unroll
-        for (int m = 8; m < 16; m++) d[m] = xd[base + pad(t + m * TL)];
+        for (int m = EH; m < E; m++) d[m] = xd[base + pad(t + m * TL)];
     }
     FxLine ln = fx_line(mx);
     const bool scaled = __any_sync(0xffffffffu, ln.pre != 0);
     if (scaled) {
         const double f = fx_pre(ln.pre);
 #pragma unroll
-        for (int m = 0; m < 16; m++) d[m] = cscale<double>(d[m], f);
+        for (int m = 0; m < E; m++) d[m] = cscale<double>(d[m], f);
     }
-    Fx v[16];
+    Fx v[E];
     if constexpr (r2r_inverse(OP)) {
         // ---- Z of the inverse FFT ---------------------------------------
         uint32_t bits = 0;
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
+        for (int m = 0; m < EH; m++) {
             const int k = t + m * TL;
             const bool z = m == 0 && t == 0;
-            Fx X{fx_from<61>(d[m].x, ln), fx_from<61>(d[m].y, ln)}, Y{fx_from<61>(d[8 + m].x, ln), fx_from<61>(d[8 + m].y, ln)};
+            Fx X{fx_from<61>(d[m].x, ln), fx_from<61>(d[m].y, ln)}, Y{fx_from<61>(d[EH + m].x, ln), fx_from<61>(d[EH + m].y, ln)};
             Fx X0{0, 0};  // k = 0: (X_0, X_H)
             if (OP == R2R_DCT3) {
                 // V = e^{+i pi k/2n} (C_k - i C_{n-k}) / 4
@@ -199,28 +199,28 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
         }
         bits = F::template line_red<false>(bits, F::NPASS + 1, c, tid, C, red);
 #pragma unroll
-        for (int m = 8; m < 16; m++) v[m] = xs[base + pad(t + m * TL)];
+        for (int m = EH; m < E; m++) v[m] = xs[base + pad(t + m * TL)];
         F::line_sync();
         const int s = fx_norm_shift<58>(bits);
-        fx_norm<16>(v, s);
+        fx_norm<E>(v, s);
         // from 61 bits, over 4 twice, and the half of Z
         ln.ex += -3 + 4 - 1 + s;
     } else {
 #pragma unroll
-        for (int m = 0; m < 16; m++) v[m] = Fx{fx_from(d[m].x, ln), fx_from(d[m].y, ln)};
+        for (int m = 0; m < E; m++) v[m] = Fx{fx_from(d[m].x, ln), fx_from(d[m].y, ln)};
         if constexpr (OP == R2R_DCT2) F::line_sync();  // the staged inputs are read
     }
     // ---- the H-point FFT: v[m] ends as Z_{t + m TL} ----------------------
     {
         typedef typename S::template Pass<F::NPASS - 1> LP_;
-        Fx z[16];
+        Fx z[E];
         auto store = [&](int, Fx *u, int q) {
 #pragma unroll
             for (int k = 0; k < LP_::R; k++) z[q + k * LP_::NB] = u[k];
         };
         F::template run<0>(v, t, c, tid, C, xs, Wpq, red, ln, store);
 #pragma unroll
-        for (int m = 0; m < 16; m++) v[m] = z[m];
+        for (int m = 0; m < E; m++) v[m] = z[m];
     }
     const int nk = fs.k != 0;
     auto real_out = [&](long long x) -> long long { return nk ? fx_mulk(x, fs.k) : x; };  // over 4 if nk
@@ -229,16 +229,16 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
     // ---- output ---------------------------------------------------------
     if constexpr (OP == R2R_RINV) {
         const int ex = ln.ex + fs.e2 + (nk ? 2 : 0);
-        double2 r[16];
+        double2 r[E];
 #pragma unroll
-        for (int m = 0; m < 16; m++) r[m] = make_double2(fx_to(real_out(v[m].x), ex), fx_to(real_out(v[m].y), ex));
+        for (int m = 0; m < E; m++) r[m] = make_double2(fx_to(real_out(v[m].x), ex), fx_to(real_out(v[m].y), ex));
         if (mul) {
 #pragma unroll
-            for (int m = 0; m < 16; m++) r[m] = cscale<double>(r[m], f);
+            for (int m = 0; m < E; m++) r[m] = cscale<double>(r[m], f);
         }
         if (valid) {
 #pragma unroll
-            for (int m = 0; m < 16; m++) {
+            for (int m = 0; m < E; m++) {
                 const int i = 2 * (t + m * TL);
                 if (vec_out) {
                     *reinterpret_cast<double2 *>(dst + i) = r[m];
@@ -254,10 +254,10 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
     if constexpr (OP == R2R_DCT3) {
         const int ex = ln.ex + fs.e2 + (nk ? 2 : 0);
 #pragma unroll
-        for (int m = 8; m < 16; m++) xs[base + pad(t + m * TL)] = v[m];
+        for (int m = EH; m < E; m++) xs[base + pad(t + m * TL)] = v[m];
         F::line_sync();
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
+        for (int m = 0; m < EH; m++) {
             const int k = t + m * TL;
             const Fx u = xs[base + pad(H - 1 - k)];
             double r0 = fx_to(real_out(v[m].x), ex), r1 = fx_to(real_out(u.y), ex), r2 = fx_to(real_out(v[m].y), ex),
@@ -289,15 +289,15 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
     }
     uint32_t bits = 0;
 #pragma unroll
-    for (int m = 0; m < 16; m++) bits |= fx_bits(v[m].x) | fx_bits(v[m].y);
+    for (int m = 0; m < E; m++) bits |= fx_bits(v[m].x) | fx_bits(v[m].y);
 #pragma unroll
-    for (int m = 8; m < 16; m++) xs[base + pad(t + m * TL)] = v[m];
+    for (int m = EH; m < E; m++) xs[base + pad(t + m * TL)] = v[m];
     bits = F::template line_red<false>(bits, F::NPASS, c, tid, C, red);
     const int s = fx_norm_shift(bits);
     // V / 4 with the half of a and d
     const int ex0 = ln.ex + s + 2 - 1 + (OP == R2R_DCT2 ? 2 : 0), ex = ex0 + fs.e2 + (nk ? 2 : 0);
 #pragma unroll
-    for (int m = 0; m < 8; m++) {
+    for (int m = 0; m < EH; m++) {
         const int k = t + m * TL;
         const bool z = m == 0 && t == 0;
         Fx zz[2] = {v[m], xs[base + pad(partner(m))]};

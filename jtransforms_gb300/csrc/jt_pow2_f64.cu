@@ -9,7 +9,7 @@ namespace jt {
 // fixed-point forms of the two-level four-step tables Whi, Wlo; W's follow W.
 bool fix_launch(int L, int mode, int sign, const double2 *in, double2 *out, const StockParams &p, const double2 *W,
                 const double2 *Whi, const double2 *Wlo, const int4 *Whiq, const int4 *Wloq, int sms, cudaStream_t s) {
-    const int4 *Wq = reinterpret_cast<const int4 *>(W + stock_tw_count(L));
+    const int4 *Wq = reinterpret_cast<const int4 *>(W + stock_tw_count(L, fx_elems(L)));
 #define JT_CASE(LL)                                                                          \
     case LL:                                                                                 \
         FixLaunch<LL>::go(mode, sign, in, out, p, W, Whi, Wlo, Wq, Whiq, Wloq, sms, s);           \

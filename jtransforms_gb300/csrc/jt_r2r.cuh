@@ -343,17 +343,17 @@ __global__ void __launch_bounds__(512) r2r_tile_kernel(const T *in, T *out, R2rP
 // A CTA holds Stockham<T, h, 0>::C lines in one shared-memory buffer that
 // serves as the load staging, the pass exchange and the output staging.
 // ---------------------------------------------------------------------------
-template <typename T, int H, int OP> struct R2rReg {
+template <typename T, int H, int OP, int E = 16> struct R2rReg {
     static constexpr int SIGN = r2r_inverse(OP) ? 1 : -1;
-    typedef Stockham<T, H, 0, SIGN> S;
+    typedef Stockham<T, H, 0, SIGN, E> S;
     static constexpr int RX = S::LP;  // row stride of a line in the buffer (complex)
     static constexpr size_t SMEM = (size_t)S::C * RX * sizeof(typename V2<T>::t);
 };
 
-template <typename T, int H, int OP>
+template <typename T, int H, int OP, int E = 16>
 __device__ __forceinline__ void r2r_reg_body(const T *in, T *out, const R2rParams &p, const C2 *__restrict__ Wp,
                                              const C2 *__restrict__ Wr, const C2 *__restrict__ Wd, unsigned char *smem_raw) {
-    typedef R2rReg<T, H, OP> G;
+    typedef R2rReg<T, H, OP, E> G;
     typedef typename G::S S;
     constexpr int n = 2 * H, RX = G::RX;
     C2 *buf = reinterpret_cast<C2 *>(smem_raw);

@@ -94,8 +94,18 @@ template <typename T> struct StockCfg {
 // 16-byte pairs each; double tables: factor k as NS entries.  Passes are
 // radix 16 (E = 16 elements per thread) with a last pass of the remaining
 // radix.
-__host__ __device__ inline int stock_tw_count(int L) {
-    const int E = L >= 16 ? 16 : L;
+// Numbers per thread of a length-L line of doubles (jt_fix64.cuh).  Eight
+// (radix-8 passes, 64 registers, twice the threads) where that takes no more
+// passes than sixteen: at 64 = 8 x 8 one pass over 2^16 points took 4.7 us
+// instead of 6.3, over 2^24 points 108 instead of 118; at 512 = 8 x 8 x 8 6.1
+// instead of 9.3, and 157 instead of 177.  One pass more costs long batches
+// more than the threads give short ones: 256 7.1 -> 6.1 and 130 -> 145, columns
+// of 1024 112 -> 141, 4096 11.7 -> 12.7 and 214 -> 243.
+__host__ __device__ constexpr int fx_elems(int L) { return L == 64 || L == 512 ? 8 : 16; }
+
+// E: elements per thread, 0 for the usual 16.
+__host__ __device__ inline int stock_tw_count(int L, int E = 0) {
+    if (E == 0) E = L >= 16 ? 16 : L;
     int logl = 0, loge = 0;
     while ((1 << logl) < L) logl++;
     while ((1 << loge) < E) loge++;
@@ -113,9 +123,8 @@ __host__ __device__ inline int stock_tw_count(int L) {
 //
 // Double tables are followed by the same entries in fixed point (int4,
 // fx_twiddle below).
-template <typename T> __global__ void passtw_kernel(typename V2<T>::t *out, int L) {
+template <typename T> __global__ void passtw_kernel(typename V2<T>::t *out, int L, int E) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    const int E = L >= 16 ? 16 : L;
     int logl = 0, loge = 0;
     while ((1 << logl) < L) logl++;
     while ((1 << loge) < E) loge++;
@@ -143,7 +152,7 @@ template <typename T> __global__ void passtw_kernel(typename V2<T>::t *out, int 
                 double s, c;
                 sincospi(-2.0 * (double)num / (double)den, &s, &c);
                 out[idx] = mk<T>((T)c, (T)s);
-                if constexpr (sizeof(T) == 8) reinterpret_cast<int4 *>(out + stock_tw_count(L))[idx] = fx_twiddle(c, s);
+                if constexpr (sizeof(T) == 8) reinterpret_cast<int4 *>(out + stock_tw_count(L, E))[idx] = fx_twiddle(c, s);
                 return;
             }
             off += ns * R;
@@ -169,9 +178,9 @@ template <int R, int SIGN, typename T> __device__ __forceinline__ void dft_pow2(
     else if (R == 16) dft16<SIGN, T>(u);
 }
 
-template <typename T, int L, int MODE, int SIGN> struct Stockham {
+template <typename T, int L, int MODE, int SIGN, int EL = (L >= 16 ? 16 : L)> struct Stockham {
     typedef typename V2<T>::t C2;
-    static constexpr int E = L >= 16 ? 16 : L;
+    static constexpr int E = EL;
     static constexpr int TL = L / E;
     static constexpr int C = StockCfg<T>::C(L, MODE);
     static constexpr int NT = C * TL;
