@@ -19,6 +19,7 @@
 #include "jt_stockham.cuh"
 #include "jt_batch.cuh"
 #include "jt_mixed.cuh"
+#include "jt_bluemix.cuh"
 #include "jt_r2r.cuh"
 #include "jt_chirp.cuh"
 #include "jt_plan_table.h"
@@ -49,7 +50,7 @@ static thread_local int64_t g_launches = 0;
     do {                                             \
         cudaError_t e_ = (call);                     \
         if (e_ != cudaSuccess) {                     \
-            g_last_cuda = (int)e_;                   \
+            g_last_cuda = (int)e_;                                                       \
             return e_ == cudaErrorMemoryAllocation ? JT_ENOMEM : JT_ECUDA; \
         }                                            \
     } while (0)
@@ -190,6 +191,14 @@ void mix_launch_fwd(int mode, const float2 *in, float2 *out, const MixParams &p,
 void mix_launch_inv(int mode, const float2 *in, float2 *out, const MixParams &p, const float2 *tw, const float2 *Whi,
                     const float2 *Wlo, unsigned grid, int threads, size_t smem, cudaStream_t s);
 
+// Float Bluestein lines (jt_bluemix.cu).
+void blue_setup(int smem_optin);
+void blue_mid(bool one, const float2 *in, float2 *out, const BlueMid &q, unsigned grid, int threads, size_t smem, cudaStream_t s);
+void blue_cols(bool first, const float2 *in, float2 *out, const MixParams &p, const MixBlue &bl, const float2 *tw, unsigned grid,
+               int threads, size_t smem, cudaStream_t s);
+void blue_twiddle(float2 *out, int n1, int n2, cudaStream_t s);
+void blue_spectrum(float2 *out, const double2 *in, int64_t n1, int64_t n2, cudaStream_t s);
+
 static int device_init() {
     std::call_once(g_dev_once, [] {
         int n = 0;
@@ -217,6 +226,7 @@ static int device_init() {
         cudaFuncSetAttribute(fft_tile_kernel<1, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         mix_setup_fwd(g_smem_optin);
         mix_setup_inv(g_smem_optin);
+        blue_setup(g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT3, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DHT, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
@@ -364,6 +374,11 @@ static void mix_search(int n, std::vector<int> &cur, int largest, std::vector<in
             cur.pop_back();
         }
 }
+static bool mix_order(int a, int b) {
+    auto rank = [](int r) { return (r & 1) ? 0 : (r & 2) ? 1 : 2; };
+    if (rank(a) != rank(b)) return rank(a) < rank(b);
+    return (a & 1) ? a > b : a < b;
+}
 static std::vector<int> mix_radices(int64_t n) {
     int64_t m = n;
     for (int p : {2, 3, 5, 7, 11, 13})
@@ -372,12 +387,83 @@ static std::vector<int> mix_radices(int64_t n) {
     std::vector<int> cur, best;
     int sum = 0;
     mix_search((int)n, cur, 16, best, sum, 0);
-    std::sort(best.begin(), best.end(), [](int a, int b) {
-        auto rank = [](int r) { return (r & 1) ? 0 : (r & 2) ? 1 : 2; };
-        if (rank(a) != rank(b)) return rank(a) < rank(b);
-        return (a & 1) ? a > b : a < b;
-    });
+    std::sort(best.begin(), best.end(), mix_order);
     return best;
+}
+// Fewest passes of the Bluestein kernels' radices (jt_bluemix.cuh) for every
+// length up to 8192 (0: none).
+static const std::vector<unsigned char> &blue_passes() {
+    static const std::vector<unsigned char> t = [] {
+        std::vector<unsigned char> np(8193, 0);
+        for (int n = 2; n <= 8192; n++) {
+#define JT_BLUE_STEP(R)                                                                                     \
+    if (n == R) np[n] = 1;                                                                                  \
+    else if (n % R == 0 && np[n / R] && (!np[n] || np[n / R] + 1 < np[n])) np[n] = (unsigned char)(np[n / R] + 1);
+            JT_BLUE_RADICES(JT_BLUE_STEP)
+#undef JT_BLUE_STEP
+        }
+        return np;
+    }();
+    return t;
+}
+// Radices of the Bluestein kernels for n.  Rows write shared memory in strides
+// of the first radix, and of the last one where they turn back: the best two
+// of mix_order go there.
+static std::vector<int> blue_radices(int n) {
+    const auto &np = blue_passes();
+    std::vector<int> R;
+    while (n > 1) {
+        int pick = 0;
+#define JT_BLUE_PICK(r) \
+    if (!pick && n % r == 0 && (n == r || (np[n / r] && np[n / r] == np[n] - 1))) pick = r;
+        JT_BLUE_RADICES(JT_BLUE_PICK)
+#undef JT_BLUE_PICK
+        R.push_back(pick);
+        n /= pick;
+    }
+    std::sort(R.begin(), R.end(), mix_order);
+    if (R.size() > 2) std::swap(R[1], R.back());
+    return R;
+}
+// Bank conflicts of those strides, as a share of a pass: r's common factor
+// with the 16 banks of a half-warp, over eight.
+static double blue_conflicts(int n) {
+    const std::vector<int> R = blue_radices(n);
+    auto ways = [](int r) { return (r & -r) - 1; };
+    return (ways(R.front()) + ways(R.back())) / 8.0;
+}
+// Convolution N = n1 n2 >= m of a Bluestein transform: n1 = 1 up to 8192 (one
+// kernel), else the n1 x n2 view.  The cheapest by length times memory and
+// passes: a pass counts as half a crossing of memory.
+static bool blue_split(int64_t m, int *n1, int *n2) {
+    const auto &np = blue_passes();
+    double best = 0;
+    if (m <= 8192) {
+        for (int n = (int)std::max<int64_t>(m, 20); n <= 8192; n++) {
+            if (np[n] < 2) continue;
+            const double c = (double)n * (2 + np[n] + blue_conflicts(n));
+            if (best == 0 || c < best) {
+                best = c;
+                *n1 = 1;
+                *n2 = n;
+            }
+            if (n * 4.0 >= best) break;
+        }
+        if (best > 0) return true;
+    }
+    for (int b = 64; b <= 4096; b++) {
+        if (np[b] < 2) continue;
+        int64_t a = std::max<int64_t>(cdiv(m, b), 16);
+        while (a <= 1024 && np[a] == 0) a++;
+        if (a > 1024) continue;
+        const double c = (double)a * b * (6 + np[a] + np[b] + blue_conflicts(b) + (a > 512 || b > 2048 ? 1 : 0));
+        if (best == 0 || c < best) {
+            best = c;
+            *n1 = (int)a;
+            *n2 = b;
+        }
+    }
+    return best > 0;
 }
 // A plan's parts of MixParams; returns the table's entries.
 static int mix_plan(int n, const std::vector<int> &R, MixParams *p) {
@@ -420,9 +506,17 @@ template <typename T> struct Fft1 {
     std::unique_ptr<Fft1> rec_alt;
     int64_t nB = 0;
     C2 *bk1 = nullptr, *bk2 = nullptr;
+    // floats outside batches (jt_bluemix.cuh): bn1 x bn2 convolution (bn1 = 1:
+    // one kernel, 0: none), the columns' and the rows' passes, their tables
+    // and the chirp's spectrum
+    int bn1 = 0, bn2 = 0;
+    MixParams bcol{}, bf{}, bg{};
+    C2 *btab = nullptr, *bspec = nullptr;
+    int boff_f = 0, boff_g = 0, btw = 0;
 
     ~Fft1() {
-        for (void *p : {(void *)W, (void *)Wp, (void *)Whi, (void *)Wlo, (void *)Whi2, (void *)Wlo2, (void *)bk1, (void *)bk2})
+        for (void *p : {(void *)W, (void *)Wp, (void *)Whi, (void *)Wlo, (void *)Whi2, (void *)Wlo2, (void *)bk1, (void *)bk2,
+                        (void *)btab, (void *)bspec})
             if (p) cudaFree(p);
     }
 
@@ -652,8 +746,12 @@ template <typename T> struct Fft1 {
                 f->algo = ALG_BLUESTEIN;
                 f->nB = next_pow2(2 * n - 1);
                 if (f->nB > kPow2PassMax) return JT_ETOOBIG;
-                JT_TRY(create(f->nB, f->pbl));
-                JT_TRY(f->make_chirp());
+                if constexpr (sizeof(T) == 4) JT_TRY(f->init_blue());
+                // batches record rec_alt where there is one
+                if (!f->bn1 || f->rec_length() == 0) {
+                    JT_TRY(create(f->nB, f->pbl));
+                    JT_TRY(f->make_chirp(f->nB, &f->bk2));
+                }
             }
         }
         if (top) JT_TRY(f->make_rec_alt());
@@ -661,7 +759,96 @@ template <typename T> struct Fft1 {
         return JT_OK;
     }
 
-    int make_chirp();
+    int make_chirp(int64_t N, C2 **spec, int64_t n1 = 1);
+
+    // Tables of the float Bluestein kernels.
+    // Convolutions up to 300,000 points, and up to 2^20 where the power of two
+    // (nB) is longer by two fifths, measured faster than the power-of-two
+    // passes between separate chirp kernels (8 M points of n = 10007: 259
+    // against 539 us, 65521: 333 / 339, 300007: 410 / 605; but 524287: 505 /
+    // 369, 1000003: 675 / 395, whose columns take three passes).
+    int init_blue() {
+        const bool found = blue_split(2 * n - 1, &bn1, &bn2);
+        const int64_t len = (int64_t)bn1 * bn2;
+        if (!found || len > ((int64_t)1 << 20) || (len > 300000 && nB * 5 < len * 7)) {
+            bn1 = 0;
+            return JT_OK;
+        }
+        const std::vector<int> f = blue_radices(bn2), g(f.rbegin(), f.rend());
+        const int cf = mix_plan(bn2, f, &bf), cg = mix_plan(bn2, g, &bg);
+        const int cc = bn1 > 1 ? mix_plan(bn1, blue_radices(bn1), &bcol) : 0;
+        boff_f = cc;
+        boff_g = cc + cf;
+        btw = cc + cf + cg;
+        const int64_t N = (int64_t)bn1 * bn2;
+        JT_CU(cudaMalloc(&btab, sizeof(C2) * (btw + (bn1 > 1 ? N : 0))));
+        if (cc) mix_table(btab, bcol, cc, g_setup);
+        if (bn1 > 1) blue_twiddle(btab + btw, bn1, bn2, g_setup);
+        mix_table(btab + boff_f, bf, cf, g_setup);
+        mix_table(btab + boff_g, bg, cg, g_setup);
+        g_launches += 2 + (cc ? 2 : 0);
+        JT_CU(cudaGetLastError());
+        return make_chirp(N, &bspec, bn1);
+    }
+    // `batch` transforms by those kernels; the convolutions of at most 128 MiB
+    // of transforms at a time.
+    int exec_blue(Ctx &ctx, const C2 *in, int64_t din, C2 *out, int64_t dout, int64_t batch, int sign, double scale) const {
+        const int64_t N = (int64_t)bn1 * bn2;
+        auto threads_of = [](const MixParams &p, int C) {
+            const int most = C * (p.L / *std::min_element(p.R, p.R + p.npass));
+            return (int)cdiv(cdiv(most, cdiv(most, p.L >= 2048 ? JT_MIX_THREADS : 256)), 32) * 32;
+        };
+        MixBlue bl{(int)n, bn2, sign > 0, din, dout, (float)scale, bk1, btab + btw};
+        BlueMid q;
+        q.f = bf;
+        q.g = bg;
+        q.twf = btab + boff_f;
+        q.twg = btab + boff_g;
+        q.Bp = bspec;
+        q.n1 = bn1;
+        q.bl = bl;
+        const size_t row = 2 * (size_t)bf.Lp * sizeof(C2);
+        auto mid_lines = [&](int64_t lines) {
+            int C = (int)std::max<int64_t>(1, (bn2 < 96 ? 4096 : 1024) / bn2);
+            while (C > 1 && cdiv(lines, C) < 2 * (int64_t)g_sms) C /= 2;
+            return C;
+        };
+        auto run_mid = [&](const C2 *a, C2 *b, int64_t lines) -> int {
+            const int C = mid_lines(lines);
+            q.f.C = q.g.C = C;
+            q.f.nlines = lines;
+            const int64_t grid = cdiv(lines, C);
+            if (grid > 0x7fffffff) return JT_ETOOBIG;
+            blue_mid(bn1 == 1, a, b, q, (unsigned)grid, threads_of(bf, C), row * C, ctx.s);
+            g_launches++;
+            return JT_OK;
+        };
+        if (bn1 == 1) return ctx.dry ? JT_OK : run_mid(in, out, batch);
+        // (in equal parts: short launches at the end fill the GPU badly)
+        const int64_t most = std::max<int64_t>(1, (int64_t)(128ll << 20) / (N * (int64_t)sizeof(C2)));
+        const int64_t chunk = cdiv(batch, cdiv(batch, most));
+        C2 *tmp = (C2 *)ctx.ws->get(sizeof(C2) * chunk * N, ctx.dry);
+        if (ctx.dry) return JT_OK;
+        MixParams p = bcol;
+        const size_t col = (size_t)p.Lp * sizeof(C2) * (p.npass > 2 ? 2 : 1);
+        p.lin = p.lout = Layout{bn2, N, 1, bn2};
+        for (int64_t b = 0; b < batch; b += chunk) {
+            const int64_t cb = std::min(chunk, batch - b), lines = cb * bn2;
+            int C = std::max(16, 1024 / bn1);
+            while (C > 8 && col * C > 110 * 1024) C /= 2;
+            while (C > 4 && cdiv(lines, C) < 2 * (int64_t)g_sms) C /= 2;
+            p.C = C;
+            p.mC = (uint32_t)(((uint64_t)1 << 32) / (uint64_t)C + 1);
+            p.nlines = lines;
+            const int64_t grid = cdiv(lines, C);
+            if (grid > 0x7fffffff) return JT_ETOOBIG;
+            blue_cols(true, in + b * din, tmp, p, bl, btab, (unsigned)grid, threads_of(p, C), col * C, ctx.s);
+            JT_TRY(run_mid(tmp, tmp, cb * bn1));
+            blue_cols(false, tmp, out + b * dout, p, bl, btab, (unsigned)grid, threads_of(p, C), col * C, ctx.s);
+            g_launches += 2;
+        }
+        return JT_OK;
+    }
 
     // A one-pass length whose line does not fit a batch task (the tile
     // kernel's limit or the batch's shared-memory cap) is recorded as the
@@ -672,17 +859,21 @@ template <typename T> struct Fft1 {
     // line on the mixed-radix tile passes, so the shorter convolution is
     // less work there (up to 2x); single calls keep the power of two, whose
     // register-kernel passes are faster.  Only for convolutions up to 2^20.
+    int64_t rec_length() const {
+        const int64_t nS = next_smooth(2 * n - 1);
+        return nB > ((int64_t)1 << 20) || (nS >= nB && !bn1) ? 0 : nS;
+    }
     int make_rec_alt() {
         if (algo == ALG_BLUESTEIN) {
-            const int64_t nS = next_smooth(2 * n - 1);
-            if (nB > ((int64_t)1 << 20) || nS >= nB) return JT_OK;
+            const int64_t nS = rec_length();
+            if (!nS) return JT_OK;
             rec_alt.reset(new (std::nothrow) Fft1());
             if (!rec_alt) return JT_ENOMEM;
             rec_alt->n = n;
             rec_alt->algo = ALG_BLUESTEIN;
             rec_alt->nB = nS;
             JT_TRY(create(nS, rec_alt->pbl));
-            return rec_alt->make_chirp();
+            return rec_alt->make_chirp(nS, &rec_alt->bk2);
         }
         if (algo != ALG_DIRECT || (generic_ok(n) && batch_line_ok<T>(n))) return JT_OK;
         int64_t best = 0;
@@ -993,6 +1184,9 @@ template <typename T> struct Fft1 {
             }
             case ALG_BLUESTEIN: {
                 if ((ctx.rec || ctx.rec_sizing) && rec_alt) return rec_alt->exec(ctx, in, din, out, dout, batch, sign, scale);
+                if constexpr (sizeof(T) == 4) {
+                    if (bn1 && !ctx.rec && !ctx.rec_sizing) return exec_blue(ctx, in, din, out, dout, batch, sign, scale);
+                }
                 if (blue_fused_ok(ctx)) return exec_blue_fused(ctx, in, din, out, dout, batch, sign, scale);
                 int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(batch, (int64_t)(128ll << 20) / (nB * (int64_t)sizeof(C2))));
                 C2 *tmp = (C2 *)ctx.ws->get(sizeof(C2) * chunk * nB, ctx.dry);
@@ -1027,26 +1221,27 @@ template <typename T> struct Fft1 {
     }
 };
 
-// bk1 (n) and bk2 = FFT_-(symmetric chirp / nB) (nB), built in FP64 on the
-// device and rounded to T (fft/DoubleFFT_1D.java:1864-1890).
-template <typename T> int Fft1<T>::make_chirp() {
-    JT_CU(cudaMalloc(&bk1, sizeof(C2) * n));
-    JT_CU(cudaMalloc(&bk2, sizeof(C2) * nB));
+// bk1 (n) and *spec = FFT_-(symmetric chirp / N) (N numbers; n1 > 1: in the
+// rows' order of the n1 x N/n1 view), built in FP64 on the device and rounded
+// to T (fft/DoubleFFT_1D.java:1864-1890).
+template <typename T> int Fft1<T>::make_chirp(int64_t N, C2 **spec, int64_t n1) {
+    if (!bk1) JT_CU(cudaMalloc(&bk1, sizeof(C2) * n));
+    JT_CU(cudaMalloc(spec, sizeof(C2) * N));
     double2 *b64 = nullptr;
-    JT_CU(cudaMallocAsync(&b64, sizeof(double2) * nB, g_setup));
-    chirp_kernel<T><<<(unsigned)cdiv(nB, 256), 256, 0, g_setup>>>(bk1, b64, n, nB);
+    JT_CU(cudaMallocAsync(&b64, sizeof(double2) * N, g_setup));
+    chirp_kernel<T><<<(unsigned)cdiv(N, 256), 256, 0, g_setup>>>(bk1, b64, n, N);
     g_launches++;
     int st = JT_OK;
     {
         std::unique_ptr<Fft1<double>> f64;
-        st = Fft1<double>::create(nB, f64);
+        st = Fft1<double>::create(N, f64);
         if (st == JT_OK) {
             Arena ar;
             Ctx c;
             c.s = g_setup;
             c.ws = &ar;
             c.dry = true;
-            st = f64->exec(c, b64, nB, b64, nB, 1, -1, 1.0);
+            st = f64->exec(c, b64, N, b64, N, 1, -1, 1.0);
             if (st == JT_OK) {
                 if (ar.peak) {
                     if (cudaMallocAsync((void **)&ar.base, ar.peak, g_setup) != cudaSuccess) st = JT_ENOMEM;
@@ -1054,7 +1249,7 @@ template <typename T> int Fft1<T>::make_chirp() {
                 }
                 ar.used = 0;
                 c.dry = false;
-                if (st == JT_OK) st = f64->exec(c, b64, nB, b64, nB, 1, -1, 1.0);
+                if (st == JT_OK) st = f64->exec(c, b64, N, b64, N, 1, -1, 1.0);
                 if (ar.base) cudaFreeAsync(ar.base, g_setup);
             }
             // the FP64 plan's own tables are freed when it goes out of scope:
@@ -1062,8 +1257,11 @@ template <typename T> int Fft1<T>::make_chirp() {
             cudaStreamSynchronize(g_setup);
         }
     }
-    if (st == JT_OK) {
-        d2t_kernel<T><<<(unsigned)cdiv(nB, 256), 256, 0, g_setup>>>(bk2, b64, nB);
+    if (st == JT_OK && n1 > 1) {
+        if constexpr (sizeof(T) == 4) blue_spectrum(*spec, b64, n1, N / n1, g_setup);
+        g_launches++;
+    } else if (st == JT_OK) {
+        d2t_kernel<T><<<(unsigned)cdiv(N, 256), 256, 0, g_setup>>>(*spec, b64, N);
         g_launches++;
     }
     cudaFreeAsync(b64, g_setup);

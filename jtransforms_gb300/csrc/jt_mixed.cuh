@@ -171,14 +171,35 @@ template <int R, int SIGN> __device__ __forceinline__ void mix_twiddle(float2 *v
     }
 }
 
-// What the passes of one launch share.
-template <int SIGN, int MODE> struct MixTile {
+// Bluestein transforms of n points around a convolution of N = n1 n2 points
+// (jt_bluemix.cuh): the chirp bk1 multiplies input and output (conjugated
+// forwards), both of which end at n; columns are c < n2.
+struct MixBlue {
+    int n, n2, inv;
+    int64_t din, dout;  // distance of transforms
+    float scale;
+    const float2 *bk1;
+    const float2 *tw;   // w_N^{k1 c} at [k1 n2 + c]
+};
+enum { MIX_PLAIN = 0, MIX_BLUE_IN = 1, MIX_BLUE_OUT = 2 };
+
+__device__ __forceinline__ float2 mix_chirp(float2 x, const MixBlue &bl, int i) {
+    const float2 w = __ldg(&bl.bk1[i]);
+    return bl.inv ? cmul<float>(x, w) : cmulc<float>(x, w);
+}
+
+// What the passes of one launch share.  POL: MIX_BLUE_IN loads chirped
+// columns of the caller's lines, MIX_BLUE_OUT multiplies its columns with the
+// conjugate four-step twiddle on the load and stores chirped lines (both take
+// that twiddle from a whole table).
+template <int SIGN, int MODE, int POL = MIX_PLAIN> struct MixTile {
     const float2 *in;
     float2 *out;
     const MixParams &p;
     const float2 *tw, *Whi, *Wlo;
     int64_t b0;
     int lines;
+    MixBlue bl;
 
     // The butterflies of pass ps: from global memory (FIRST) or src, to global
     // memory (LAST) or dst.  Strided lines are walked lines first.
@@ -199,11 +220,28 @@ template <int SIGN, int MODE> struct MixTile {
                 j = q - c * nb;
             }
             float2 v[R];
-            if (FIRST) {
+            if (FIRST && POL == MIX_BLUE_IN) {
+                int64_t col;
+                const int64_t tr = div_fast(b0 + c, bl.n2, &col);
+                const float2 *g = in + tr * bl.din;
+                int i = j * bl.n2 + (int)col;
+#pragma unroll
+                for (int k = 0; k < R; k++) {
+                    v[k] = i < bl.n ? mix_chirp(g[i], bl, i) : make_float2(0, 0);
+                    i += nb * bl.n2;
+                }
+            } else if (FIRST) {
                 const int64_t es = MODE == 1 ? p.lin.estride : 1, step = nb * es;
                 const float2 *g = in + line_off(p.lin, b0 + c) + j * es;
 #pragma unroll
                 for (int k = 0; k < R; k++) v[k] = g[k * step];
+                if (POL == MIX_BLUE_OUT) {
+                    int64_t col;
+                    div_fast(b0 + c, bl.n2, &col);
+                    const float2 *w = bl.tw + j * bl.n2 + col;
+#pragma unroll
+                    for (int k = 0; k < R; k++) v[k] = cmulc<float>(v[k], __ldg(w + k * nb * bl.n2));
+                }
             } else {
                 const float2 *s = src + c * Lp + j;
 #pragma unroll
@@ -219,10 +257,26 @@ template <int SIGN, int MODE> struct MixTile {
                 mix_twiddle<R, SIGN>(v, twp, Ns, jm);
             }
             dft_any<R, SIGN, float>(v);
-            if (LAST) {
+            if (LAST && POL == MIX_BLUE_OUT) {
+                int64_t col;
+                const int64_t tr = div_fast(b0 + c, bl.n2, &col);
+                float2 *g = out + tr * bl.dout;
+                int i = base * bl.n2 + (int)col;
+#pragma unroll
+                for (int k = 0; k < R; k++) {
+                    if (i < bl.n) g[i] = cscale<float>(mix_chirp(v[k], bl, i), bl.scale);
+                    i += Ns * bl.n2;
+                }
+            } else if (LAST) {
                 const int64_t es = MODE != 0 ? p.lout.estride : 1, step = Ns * es;
                 float2 *g = out + line_off(p.lout, b0 + c) + base * es;
-                if (p.tw_n) {
+                if (POL == MIX_BLUE_IN) {
+                    int64_t col;
+                    div_fast(b0 + c, bl.n2, &col);
+                    const float2 *w = bl.tw + base * bl.n2 + col;
+#pragma unroll
+                    for (int k = 0; k < R; k++) v[k] = cmul<float>(v[k], __ldg(w + k * Ns * bl.n2));
+                } else if (p.tw_n) {
                     // i < n1 and the line's column below n2: the products stay below tw_n = n1 n2 < 2^31
                     int64_t j2;
                     div_fast(b0 + c, p.tw_inner, &j2);
@@ -296,7 +350,7 @@ __global__ void __launch_bounds__(JT_MIX_THREADS, 2) mix_kernel(const float2 *in
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int64_t b0 = (int64_t)blockIdx.x * p.C;
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
-    MixTile<SIGN, MODE>{in, out, p, tw, Whi, Wlo, b0, (int)min((int64_t)p.C, p.nlines - b0)}.run(A, A + p.C * p.Lp);
+    MixTile<SIGN, MODE>{in, out, p, tw, Whi, Wlo, b0, (int)min((int64_t)p.C, p.nlines - b0), MixBlue{}}.run(A, A + p.C * p.Lp);
 }
 
 // Pass tables of the radices R[0..npass) (mix_twiddle's layout): pass P >= 1

@@ -67,3 +67,25 @@ def test_two_passes(n, batch):
     assert rel_l2(got, np.fft.fft(z.astype(complex), axis=1)) <= tol(n, np.float32)
     f.plan.execute(N.COMPLEX_INVERSE, dev, 0, True, batch=batch, dist=2 * n)
     assert rel_l2(dev.cpu().numpy().view(np.complex64).reshape(batch, n), z) <= 2 * tol(n, np.float32)
+
+
+@pytest.mark.parametrize("n", [67, 71, 101, 127, 263, 509, 1021, 2 * 1021, 2039, 3 * 1361, 4093, 4099, 8191, 10007, 2 * 5003, 20011, 65521,
+                               131071, 3 * 67 * 1009, 524287])
+@pytest.mark.parametrize("batch", [1, 3, 40])
+def test_bluestein(n, batch):
+    """Lengths with a prime factor above 61: one kernel up to 4096 points
+    (jt_bluemix.cuh), three beyond."""
+    import jtransforms_gb300 as J
+    from jtransforms_gb300 import _native as N
+    if n * batch > 3000000:
+        batch = 2
+    f = J.FloatFFT_1D(n)
+    dist = n + 3
+    z = _c64((batch, dist), n)
+    dev = _device(z)
+    f.plan.execute(N.COMPLEX_FORWARD, dev, 0, False, batch=batch, dist=2 * dist)
+    got = dev.cpu().numpy().view(np.complex64).reshape(batch, dist)
+    assert np.array_equal(got[:, n:], z[:, n:])  # what lies between the lines is left alone
+    assert rel_l2(got[:, :n], np.fft.fft(z[:, :n].astype(complex), axis=1)) <= tol(n, np.float32)
+    f.plan.execute(N.COMPLEX_INVERSE, dev, 0, True, batch=batch, dist=2 * dist)
+    assert rel_l2(dev.cpu().numpy().view(np.complex64).reshape(batch, dist)[:, :n], z[:, :n]) <= 2 * tol(n, np.float32)
