@@ -54,7 +54,7 @@ __device__ void blue_tile_body(const C2 *in, C2 *out, const BlueParams &p, const
         bufA[c * Lp + pad(i)] = v;
     }
     __syncthreads();
-    C2 *z = tile_passes<-1, T>(bufA, bufB, lines, nB, Lp, p.npass, p.radix, W);
+    C2 *z = tile_passes<-1, T>(bufA, bufB, lines, nB, Lp, p.npass, p.radix, W, bufB + p.C * Lp);
     for (int idx = tid; idx < tot; idx += nt) {
         const int c = idx / nB, k = idx - c * nB;
         C2 &v = z[c * Lp + pad(k)];
@@ -62,7 +62,7 @@ __device__ void blue_tile_body(const C2 *in, C2 *out, const BlueParams &p, const
         v = SIGN < 0 ? cmul<T>(v, w) : cmulc<T>(v, w);
     }
     __syncthreads();
-    const C2 *y = tile_passes<1, T>(z, z == bufA ? bufB : bufA, lines, nB, Lp, p.npass, p.radix, W);
+    const C2 *y = tile_passes<1, T>(z, z == bufA ? bufB : bufA, lines, nB, Lp, p.npass, p.radix, W, bufB + p.C * Lp);
     const int tn = lines * n;
     for (int idx = tid; idx < tn; idx += nt) {
         const int c = idx / n, i = idx - c * n;

@@ -20,6 +20,7 @@
 #include "jt_batch.cuh"
 #include "jt_mixed.cuh"
 #include "jt_bluemix.cuh"
+#include "jt_fixmix.cuh"
 #include "jt_r2r.cuh"
 #include "jt_chirp.cuh"
 #include "jt_plan_table.h"
@@ -191,6 +192,11 @@ void mix_launch_fwd(int mode, const float2 *in, float2 *out, const MixParams &p,
 void mix_launch_inv(int mode, const float2 *in, float2 *out, const MixParams &p, const float2 *tw, const float2 *Whi,
                     const float2 *Wlo, unsigned grid, int threads, size_t smem, cudaStream_t s);
 
+// Mixed-radix lines of doubles (jt_fixmix.cu).
+void fixmix_setup(int smem_optin);
+void fixmix_table(int4 *out, const MixParams &p, int count, cudaStream_t s);
+void fixmix_launch(const double2 *in, double2 *out, const FixMixParams &p, unsigned grid, int threads, size_t smem, cudaStream_t s);
+
 // Float Bluestein lines (jt_bluemix.cu).
 void blue_setup(int smem_optin);
 void blue_mid(bool one, const float2 *in, float2 *out, const BlueMid &q, unsigned grid, int threads, size_t smem, cudaStream_t s);
@@ -227,6 +233,7 @@ static int device_init() {
         mix_setup_fwd(g_smem_optin);
         mix_setup_inv(g_smem_optin);
         blue_setup(g_smem_optin);
+        fixmix_setup(g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT3, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DHT, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
@@ -299,9 +306,11 @@ static const int kMaxThreads = 512;
 // elements per task of a recorded (batch) tile step: the batch kernel's
 // threads then all own a radix-16 butterfly (shared memory permitting)
 static const int64_t kBatchTileElems = 16 * JT_BATCH_THREADS;
+// shared memory per line of a tile step
+template <typename T> static size_t tile_line(int L) { return 2 * (size_t)padded_len(L) * sizeof(typename V2<T>::t) + tile_words<T>(); }
 // whether one line of length L fits a batch task's shared-memory cap
 template <typename T> static bool batch_line_ok(int64_t L) {
-    return 2 * (size_t)padded_len((int)L) * sizeof(typename V2<T>::t) <= (size_t)JT_BATCH_SMEM_CAP;
+    return tile_line<T>((int)L) <= (size_t)JT_BATCH_SMEM_CAP;
 }
 
 template <typename T> struct Lim {
@@ -358,7 +367,8 @@ static int radix_order(int64_t n, bool f32) {
 // ones come first (largest first): the first pass writes shared memory in
 // strides of its radix, which odd strides do without bank conflicts; then
 // twice an odd number (two ways), the rest from the smallest.
-static void mix_search(int n, std::vector<int> &cur, int largest, std::vector<int> &best, int &best_sum, int sum) {
+static void mix_search(int n, std::vector<int> &cur, int largest, std::vector<int> &best, int &best_sum, int sum,
+                       unsigned allowed = ~0u) {
     if (n == 1) {
         if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && sum < best_sum)) {
             best = cur;
@@ -368,9 +378,9 @@ static void mix_search(int n, std::vector<int> &cur, int largest, std::vector<in
     }
     if (!best.empty() && cur.size() >= best.size()) return;
     for (int r = std::min(largest, 16); r >= 2; r--)
-        if (n % r == 0) {
+        if (n % r == 0 && (allowed >> r & 1)) {
             cur.push_back(r);
-            mix_search(n / r, cur, r, best, best_sum, sum + r);
+            mix_search(n / r, cur, r, best, best_sum, sum + r, allowed);
             cur.pop_back();
         }
 }
@@ -390,6 +400,30 @@ static std::vector<int> mix_radices(int64_t n) {
     std::sort(best.begin(), best.end(), mix_order);
     return best;
 }
+// Radices of the doubles' mixed-radix kernel (jt_fixmix.cuh): the fewest; the
+// first one leaves at most 512 butterflies, the block's threads, and is odd if
+// one of those is (no bank conflicts), the largest.
+static std::vector<int> fixmix_radices(int64_t n) {
+    unsigned allowed = 0;
+#define JT_FIXMIX_BIT(R) allowed |= 1u << R;
+    JT_FIXMIX_RADICES(JT_FIXMIX_BIT)
+#undef JT_FIXMIX_BIT
+    std::vector<int> cur, R;
+    int sum = 0;
+    if (n < 17 || n > 4096) return {};
+    mix_search((int)n, cur, 16, R, sum, 0, allowed);
+    if (R.size() < 2) return {};
+    std::sort(R.begin(), R.end(), mix_order);
+    int first = -1;
+    for (int i = 0; i < (int)R.size(); i++) {
+        if (n / R[i] > JT_FIXMIX_THREADS) continue;
+        if (first < 0 || ((R[i] & 1) == (R[first] & 1) && R[i] > R[first])) first = i;
+    }
+    if (first < 0) return {};
+    std::rotate(R.begin(), R.begin() + first, R.begin() + first + 1);
+    return R;
+}
+
 // Fewest passes of the Bluestein kernels' radices (jt_bluemix.cuh) for every
 // length up to 8192 (0: none).
 static const std::vector<unsigned char> &blue_passes() {
@@ -598,15 +632,17 @@ template <typename T> struct Fft1 {
         return t[0] >= 0 ? t : nullptr;
     }
 
-    // mixed-radix kernel (jt_mixed.cuh): its part of the launch parameters and
-    // its pass table, which follows W; npass = 0: lengths it does not take
+    // mixed-radix kernels (jt_mixed.cuh, jt_fixmix.cuh): their part of the launch parameters and
+    // the pass table, which follows W; npass = 0: lengths it does not take
+    // (psh: jt_fixmix.cuh's)
     MixParams mix{};
     C2 *Wm = nullptr;
+    int psh = 31;
 
     int init_direct() {
         algo = ALG_DIRECT;
         JT_TRY(set_reg(reg_ok(n)));
-        if (reg) return make_roots(&W, n, 1, n);
+        if (reg) return make_roots(&W, n, 1, n, sizeof(T) == 8);
         radix = direct_radices(n, radix_order(n, sizeof(T) == 4));
         if constexpr (sizeof(T) == 4) {
             const std::vector<int> R = mix_radices(n);
@@ -620,8 +656,89 @@ template <typename T> struct Fft1 {
             }
             return JT_OK;
         } else {
-            return make_roots(&W, n, 1, n);
+            const std::vector<int> R = fixmix_radices(n);
+            int count = 0;
+            if (!R.empty()) {
+                mix_plan((int)n, R, &mix);
+                for (int i = 1; i < mix.npass; i++) {  // factor by factor, no pairs
+                    mix.toff[i] = count;
+                    count += mix.Ns[i] * (R[i] - 1);
+                }
+                // even first radices write shared memory in strides that a spare number per eight spreads
+                psh = (R[0] & 1) ? 31 : 3;
+                mix.Lp = ((int)n + ((int)n >> psh)) | 1;
+            }
+            JT_TRY(make_roots(&W, n, 1, n, true, count));
+            if (count) {
+                Wm = W + 2 * n;
+                fixmix_table((int4 *)Wm, mix, count, g_setup);
+                g_launches++;
+                JT_CU(cudaGetLastError());
+            }
+            return JT_OK;
         }
+    }
+
+    // Line pass of the doubles' mixed-radix kernel.  C lines per CTA: a first
+    // pass of 256 butterflies for rows, 512 for strided lines (up to 8: 128-byte
+    // runs), fewer (down to 2 columns) while the grid has fewer CTAs than two
+    // per SM.
+    int exec_fixmix(Ctx &ctx, const C2 *in, C2 *out, int64_t nlines, const Layout &lin, const Layout &lout, int sign, double scale,
+                    int64_t tw_n, int64_t tw_inner, const C2 *Whi_, const C2 *Wlo_, int tw_lo_bits) const {
+        FixMixParams p;
+        memset(&p, 0, sizeof(p));
+        p.m = mix;
+        p.psh = psh;
+        p.cols_in = lin.estride != 1;
+        p.cols_out = lout.estride != 1;
+        p.inv = sign > 0;
+        const bool strided = p.cols_in || p.cols_out;
+        const int nb = (int)n / mix.R[0];
+        const size_t per_line = (size_t)mix.Lp * sizeof(C2) * (mix.npass > 2 ? 2 : 1) + tile_words<T>();
+        int C = std::max(1, (strided ? JT_FIXMIX_THREADS : 256) / nb);
+        if (strided) C = std::min(C, std::max(8, 128 / nb));
+        C = std::min(C, (int)std::max<size_t>(1, (size_t)g_smem_optin / per_line));
+        while (C > (strided ? 2 : 1) && C * nb > 32 && cdiv(nlines, C) < 2 * (int64_t)g_sms) C /= 2;
+        if ((int64_t)C > nlines) C = (int)nlines;
+        p.m.C = C;
+        p.m.mC = C > 1 ? (uint32_t)(((uint64_t)1 << 32) / (uint64_t)C + 1) : 0;
+        p.m.nlines = nlines;
+        p.m.lin = lin;
+        p.m.lout = lout;
+        p.m.tw_n = tw_n;
+        p.m.tw_inner = tw_inner;
+        p.m.tw_lo_bits = tw_lo_bits;
+        int e2 = 0;
+        const bool pow2_scale = std::frexp(scale, &e2) == 0.5;
+        p.scale_e2 = pow2_scale ? e2 - 1 : 0;
+        p.scale_mul = !pow2_scale;
+        p.scale = scale;
+        p.tw = (const int4 *)Wm;
+        const int64_t nlo = (int64_t)1 << tw_lo_bits, nhi = tw_n ? cdiv(tw_n, nlo) : 0;
+        p.Whiq = (const int4 *)(Whi_ ? Whi_ + nhi : nullptr);
+        p.Wloq = (const int4 *)(Wlo_ ? Wlo_ + nlo : nullptr);
+        p.fp.L = (int)n;
+        p.fp.npass = (int)radix.size();
+        for (int i = 0; i < p.fp.npass; i++) p.fp.radix[i] = radix[i];
+        p.fp.C = 1;
+        p.fp.nlines = nlines;
+        p.fp.lin = lin;
+        p.fp.lout = lout;
+        p.fp.scale = scale;
+        p.fp.do_scale = scale != 1.0;
+        p.fp.tw_n = tw_n;
+        p.fp.tw_inner = tw_inner;
+        p.fp.tw_lo_bits = tw_lo_bits;
+        p.W = W;
+        p.Whi = Whi_;
+        p.Wlo = Wlo_;
+        if (ctx.dry) return JT_OK;
+        const int64_t grid = cdiv(nlines, C);
+        if (grid > 0x7fffffff) return JT_ETOOBIG;
+        const size_t smem = std::max(per_line * C, 2 * (size_t)padded_len((int)n) * sizeof(C2));
+        fixmix_launch(in, out, p, (unsigned)grid, (int)cdiv(C * nb, 32) * 32, smem, ctx.s);
+        g_launches++;
+        return JT_OK;
     }
 
     // Line pass of the mixed-radix kernel.  C lines per CTA: about 4096 numbers
@@ -913,7 +1030,7 @@ template <typename T> struct Fft1 {
         if (rr.empty() || (int)rr.size() > JT_MAX_PASSES) return JT_EINVAL;
         p.npass = (int)rr.size();
         for (int i = 0; i < p.npass; i++) p.radix[i] = rr[i];
-        const size_t per_line = 2 * (size_t)padded_len((int)nB) * sizeof(C2);
+        const size_t per_line = tile_line<T>((int)nB);
         int C = (int)std::max<int64_t>(1, (ctx.rec ? kBatchTileElems : (sizeof(T) == 4 ? 4096 : 2048)) / nB);
         C = std::min(C, (int)std::max<size_t>(1, (size_t)g_smem_optin / per_line));
         if ((int64_t)C > batch) C = (int)batch;
@@ -968,12 +1085,11 @@ template <typename T> struct Fft1 {
         o.Wlo = Wlo_;
         if (generic_ok(n)) {
             const int L = (int)n;
-            const int Lp = padded_len(L);
             const bool strided = lin.estride != 1 || lout.estride != 1;
             int64_t target = kBatchTileElems;  // the batch CTA has 512 threads: 512 radix-16 butterflies
             int C = (int)std::max<int64_t>(1, target / L);
             if (strided) C = std::max(C, sizeof(T) == 4 ? 16 : 8);
-            size_t per_line = 2 * (size_t)Lp * sizeof(C2);
+            size_t per_line = tile_line<T>(L);
             int cmax = (int)std::max<size_t>(1, std::min<size_t>(g_smem_optin, JT_BATCH_SMEM_CAP) / per_line);
             C = std::min(C, cmax);
             if ((int64_t)C > nlines) C = (int)nlines;
@@ -1081,14 +1197,15 @@ template <typename T> struct Fft1 {
         if constexpr (sizeof(T) == 4) {
             if (mix.npass > 1 || (mix.npass == 1 && lin.estride != 1 && lout.estride != 1))
                 return exec_mix(ctx, in, out, nlines, lin, lout, sign, scale, tw_n, tw_inner, Whi_, Wlo_, tw_lo_bits);
+        } else {
+            if (mix.npass) return exec_fixmix(ctx, in, out, nlines, lin, lout, sign, scale, tw_n, tw_inner, Whi_, Wlo_, tw_lo_bits);
         }
         const int L = (int)n;
-        const int Lp = padded_len(L);
         const bool strided = lin.estride != 1 || lout.estride != 1;
         const int64_t target = tile_elems(L);
         int C = (int)std::max<int64_t>(1, target / L);
         if (strided) C = std::max(C, sizeof(T) == 4 ? 16 : 8);
-        size_t per_line = 2 * (size_t)Lp * sizeof(C2);
+        size_t per_line = tile_line<T>(L);
         int cmax = (int)std::max<size_t>(1, (size_t)g_smem_optin / per_line);
         C = std::min(C, cmax);
         if ((int64_t)C > nlines) C = (int)nlines;
@@ -1516,7 +1633,7 @@ template <typename T> static bool r2r_strided_ok(const Ctx &ctx, int64_t n, cons
     const int64_t h = n / 2;
     const int need = (int)(32 / sizeof(T));
     if (r2r_reg_c<T>(h, rf) >= need) return true;
-    const size_t per_line = 2 * (size_t)padded_len((int)h) * sizeof(typename V2<T>::t);
+    const size_t per_line = tile_line<T>((int)h);
     return (size_t)g_smem_optin / per_line >= (size_t)need;
 }
 
@@ -1533,11 +1650,10 @@ static int r2r_fused(Ctx &ctx, int op, const Real1<T> *rf, const T *in, T *out, 
     p.n = (int)n;
     p.npass = (int)rr.size();
     for (int i = 0; i < p.npass; i++) p.radix[i] = rr[i];
-    const int Lp = padded_len((int)h);
     const bool strided = lin.estride != 1 || lout.estride != 1;
     int C = (int)std::max<int64_t>(1, (ctx.rec ? kBatchTileElems : (sizeof(T) == 4 ? 4096 : 2048)) / h);
     if (strided) C = std::max(C, sizeof(T) == 4 ? 16 : 8);
-    const size_t per_line = 2 * (size_t)Lp * sizeof(C2);
+    const size_t per_line = tile_line<T>((int)h);
     C = std::min(C, (int)std::max<size_t>(1, (size_t)g_smem_optin / per_line));
     if ((int64_t)C > nlines) C = (int)nlines;
     p.C = C;

@@ -29,195 +29,10 @@
 // spread as they always did.
 #pragma once
 
+#include "jt_fixmath.cuh"
 #include "jt_stockham.cuh"
 
 namespace jt {
-
-// Fixed-point complex value (one exponent per line, kept beside it).
-struct Fx {
-    long long x, y;
-};
-
-__device__ __forceinline__ long long fx_madw(int a, int b, long long c) {
-    long long r;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
-    return r;
-}
-// v as vh 2^32 + vl with both halves signed
-__device__ __forceinline__ int fx_hi(long long v) { return (int)(v >> 32) + (int)((uint32_t)v >> 31); }
-__device__ __forceinline__ int fx_lo(long long v) { return (int)v; }
-
-// Fixed-point factors w are fx_twiddle's (x, y: cosine's halves; z, w: sine's).
-// v w / 4 (SIGN < 0) or v conj(w) / 4, rounded to nearest.  |v| below 2^62.5:
-// the partial sums stay below 2^63.  The low x low product is left out (a
-// quarter of a unit at most).
-template <int SIGN> __device__ __forceinline__ Fx fx_mul(Fx v, int4 w) {
-    const int xh = fx_hi(v.x), xl = fx_lo(v.x), yh = fx_hi(v.y), yl = fx_lo(v.y);
-    const int ph = SIGN < 0 ? w.z : -w.z, pl = SIGN < 0 ? w.w : -w.w;  // im += x p
-    const int nh = SIGN < 0 ? -w.z : w.z, nl = SIGN < 0 ? -w.w : w.w;  // re += y n
-    const long long half = 1ll << 31;
-    long long m = fx_madw(yl, nh, fx_madw(yh, nl, fx_madw(xl, w.x, fx_madw(xh, w.y, half))));
-    Fx r;
-    r.x = fx_madw(yh, nh, fx_madw(xh, w.x, m >> 32));
-    m = fx_madw(xl, ph, fx_madw(xh, pl, fx_madw(yl, w.x, fx_madw(yh, w.y, half))));
-    r.y = fx_madw(xh, ph, fx_madw(yh, w.x, m >> 32));
-    return r;
-}
-
-// v k / 2^64 rounded, for a constant |k| < 2^63: v times a factor in (-1/2, 1/2)
-__device__ __forceinline__ long long fx_mulk(long long v, long long k) {
-    const int vh = fx_hi(v), vl = fx_lo(v), kh = (int)((k + (1ll << 31)) >> 32), kl = (int)k;
-    const long long m = fx_madw(vl, kh, fx_madw(vh, kl, 1ll << 31));
-    return fx_madw(vh, kh, m >> 32);
-}
-// round(f 2^64) for -1/2 < f < 1/2: cos(pi/4) - 1, sqrt(2) - 1, tan(pi/16), sin(pi/8)
-static constexpr long long kFxHm1 = -5402926248376769404ll;
-static constexpr long long kFxR2m1 = 7640891576956012809ll;
-static constexpr long long kFxTan16 = 3669285534148243471ll;
-static constexpr long long kFxSin8 = 7059263338087549767ll;
-__device__ __forceinline__ long long fx_mulh(long long v) { return v + fx_mulk(v, kFxHm1); }  // v cos(pi/4)
-
-__device__ __forceinline__ Fx fx_add(Fx a, Fx b) { return Fx{a.x + b.x, a.y + b.y}; }
-__device__ __forceinline__ Fx fx_sub(Fx a, Fx b) { return Fx{a.x - b.x, a.y - b.y}; }
-template <int SIGN> __device__ __forceinline__ Fx fx_si(Fx a) { return SIGN > 0 ? Fx{-a.y, a.x} : Fx{a.y, -a.x}; }
-
-// a e^{SIGN i pi/8}: three shears of the plane (x -= t y, y += s x, x -= t y
-// with t = tan(pi/16), s = sin(pi/8)), nine multiply-adds where four real
-// products take twelve
-template <int SIGN> __device__ __forceinline__ Fx fx_rot8(Fx a) {
-    constexpr long long t = SIGN > 0 ? kFxTan16 : -kFxTan16, s = SIGN > 0 ? kFxSin8 : -kFxSin8;
-    a.x -= fx_mulk(a.y, t);
-    a.y += fx_mulk(a.x, s);
-    a.x -= fx_mulk(a.y, t);
-    return a;
-}
-
-template <int SIGN> __device__ __forceinline__ void fx_dft4(Fx &v0, Fx &v1, Fx &v2, Fx &v3) {
-    const Fx t0 = fx_add(v0, v2), t1 = fx_sub(v0, v2), t2 = fx_add(v1, v3), d = fx_sub(v1, v3);
-    v0 = fx_add(t0, t2);
-    v2 = fx_sub(t0, t2);
-    // t1 +- SIGN i d
-    v1 = SIGN > 0 ? Fx{t1.x - d.y, t1.y + d.x} : Fx{t1.x + d.y, t1.y - d.x};
-    v3 = SIGN > 0 ? Fx{t1.x + d.y, t1.y - d.x} : Fx{t1.x - d.y, t1.y + d.x};
-}
-
-template <int SIGN> __device__ __forceinline__ void fx_dft8(Fx *v) {
-    Fx e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
-    Fx o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
-    fx_dft4<SIGN>(e0, e1, e2, e3);
-    fx_dft4<SIGN>(o0, o1, o2, o3);
-    // e^{SIGN i pi/4} and e^{SIGN 3 i pi/4}
-    o1 = SIGN > 0 ? Fx{fx_mulh(o1.x - o1.y), fx_mulh(o1.x + o1.y)} : Fx{fx_mulh(o1.x + o1.y), fx_mulh(o1.y - o1.x)};
-    o2 = fx_si<SIGN>(o2);
-    o3 = SIGN > 0 ? Fx{fx_mulh(-o3.x - o3.y), fx_mulh(o3.x - o3.y)} : Fx{fx_mulh(o3.y - o3.x), fx_mulh(-o3.x - o3.y)};
-    v[0] = fx_add(e0, o0); v[4] = fx_sub(e0, o0);
-    v[1] = fx_add(e1, o1); v[5] = fx_sub(e1, o1);
-    v[2] = fx_add(e2, o2); v[6] = fx_sub(e2, o2);
-    v[3] = fx_add(e3, o3); v[7] = fx_sub(e3, o3);
-}
-
-// radix 16 as 4 x 4: element (k, j) at v[j + 4k] takes e^{SIGN i pi jk/8}
-template <int SIGN> __device__ __forceinline__ void fx_dft16(Fx *v) {
-#pragma unroll
-    for (int j = 0; j < 4; j++) fx_dft4<SIGN>(v[j], v[j + 4], v[j + 8], v[j + 12]);
-    auto w2 = [](Fx a) {  // e^{SIGN i pi/4}
-        return SIGN > 0 ? Fx{fx_mulh(a.x - a.y), fx_mulh(a.x + a.y)} : Fx{fx_mulh(a.x + a.y), fx_mulh(a.y - a.x)};
-    };
-    v[5] = fx_rot8<SIGN>(v[5]);
-    v[6] = w2(v[6]);
-    v[7] = fx_rot8<-SIGN>(fx_si<SIGN>(v[7]));    // w^3 = SIGN i w^-1
-    v[9] = w2(v[9]);
-    v[10] = fx_si<SIGN>(v[10]);
-    v[11] = w2(fx_si<SIGN>(v[11]));              // w^6
-    v[13] = fx_rot8<-SIGN>(fx_si<SIGN>(v[13]));  // w^3
-    v[14] = w2(fx_si<SIGN>(v[14]));              // w^6
-    v[15] = fx_rot8<SIGN>(v[15]);                // w^9 = -w
-    v[15] = Fx{-v[15].x, -v[15].y};
-#pragma unroll
-    for (int k = 0; k < 4; k++) fx_dft4<SIGN>(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-    Fx t[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) t[i] = v[i];
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) v[k + 4 * j] = t[4 * k + j];
-}
-
-template <int R, int SIGN> __device__ __forceinline__ void fx_dft(Fx *v) {
-    if (R == 2) {
-        const Fx a = v[0], b = v[1];
-        v[0] = fx_add(a, b);
-        v[1] = fx_sub(a, b);
-    } else if (R == 4) {
-        fx_dft4<SIGN>(v[0], v[1], v[2], v[3]);
-    } else if (R == 8) {
-        fx_dft8<SIGN>(v);
-    } else if (R == 16) {
-        fx_dft16<SIGN>(v);
-    }
-}
-
-// Bits in use: the OR of these over a line has the bit length of its largest
-// magnitude's high word.
-__device__ __forceinline__ uint32_t fx_bits(long long v) {
-    const int h = (int)(v >> 32);
-    return (uint32_t)(h ^ (h >> 31));
-}
-
-// A line's exponent and what its doubles are scaled by around the transform.
-struct FxLine {
-    int ex;    // a value is v 2^ex
-    int pre;   // 0, or +-512: the doubles were multiplied by 2^pre first
-};
-
-#define JT_FX_BIAS 1080  // a double of the line's largest exponent eb is v 2^(eb - 1080), v < 2^58
-
-// From the line's largest (high word << 1) over all its numbers.
-__device__ __forceinline__ FxLine fx_line(uint32_t m) {
-    const int eb = (int)(m >> 21);
-    FxLine l;
-    l.pre = eb < 123 ? 512 : eb > 1923 ? -512 : 0;  // (lines of zeros too: subnormals may have no high word)
-    l.ex = max(eb, 1) + l.pre - JT_FX_BIAS;
-    return l;
-}
-// The line's numbers below 2^BITS (l.ex is for 58).
-template <int BITS = 58> __device__ __forceinline__ long long fx_from(double d, const FxLine &l) {
-    const int hi = __double2hiint(d), lo = __double2loint(d);
-    const int e = (hi >> 20) & 0x7ff;
-    const uint32_t mh = ((uint32_t)hi & 0xfffffu) | 0x100000u;
-    const int r = min(l.ex + JT_FX_BIAS + 63 - BITS - e, 63);  // at least 63 - BITS; zeros (and far smaller numbers) go to 0
-    unsigned long long u = (((unsigned long long)mh << 32) | (uint32_t)lo) << 10;
-    u >>= r;
-    const long long s = (long long)(hi >> 31);
-    return ((long long)u ^ s) - s;
-}
-__device__ __forceinline__ double fx_to(long long v, int ex) {
-    const double d = __ll2double_rn(v);
-    const int hi = __double2hiint(d);
-    return v == 0 ? 0.0 : __hiloint2double(hi + (ex << 20), __double2loint(d));
-}
-// 2^pre and 2^-pre.  Products with them stand behind one branch per block of
-// values: a conditional product is issued to the FP64 pipe for every value,
-// needed or not, and six of those per number were most of this kernel's time.
-__device__ __forceinline__ double fx_pre(int pre) { return pre > 0 ? 1.3407807929942597e154 : pre < 0 ? 7.458340731200207e-155 : 1.0; }
-
-// Shift that brings a line with these bits to BITS bits: right by s > 0 or left by -s.
-template <int BITS = 60> __device__ __forceinline__ int fx_norm_shift(uint32_t bits) { return bits ? 64 - BITS - __clz(bits) : 0; }
-// (v + rnd) >> s with rnd = half a unit of the result
-__device__ __forceinline__ Fx fx_shr(Fx v, int s, long long rnd) { return Fx{(v.x + rnd) >> s, (v.y + rnd) >> s}; }
-__device__ __forceinline__ long long fx_half(int s) { return s > 0 ? 1ll << (s - 1) : 0; }
-// N values by the shift s (fx_norm_shift's)
-template <int N> __device__ __forceinline__ void fx_norm(Fx *v, int s) {
-    if (s < 0) {
-#pragma unroll
-        for (int m = 0; m < N; m++) v[m] = Fx{v[m].x << -s, v[m].y << -s};
-        s = 0;
-    }
-    const long long r = fx_half(s);
-#pragma unroll
-    for (int m = 0; m < N; m++) v[m] = fx_shr(v[m], s, r);
-}
 
 // Fixed-point pass table of a length-L line: the entries of the double table
 // (stock_tw_count, factor k of a pass as NS entries) as int4.

@@ -324,8 +324,8 @@ __device__ void r2r_tile_body(const T *in, T *out, const R2rParams &p, const C2 
         }
         __syncthreads();
     }
-    const C2 *z = r2r_inverse(OP) ? tile_passes<1, T>(bufA, bufB, lines, h, Lp, p.npass, p.radix, W)
-                                  : tile_passes<-1, T>(bufA, bufB, lines, h, Lp, p.npass, p.radix, W);
+    const C2 *z = r2r_inverse(OP) ? tile_passes<1, T>(bufA, bufB, lines, h, Lp, p.npass, p.radix, W, bufB + p.C * Lp)
+                                  : tile_passes<-1, T>(bufA, bufB, lines, h, Lp, p.npass, p.radix, W, bufB + p.C * Lp);
     r2r_store<OP, T>(z, Lp, out, p, b0, lines, Wr, Wd, mult, mult0, threadIdx.x, blockDim.x);
 }
 
