@@ -2133,16 +2133,19 @@ template <typename T> struct PlanImpl {
             double mult = (!fwd && scale) ? 1.0 / (double)dims[0] : 1.0;
             return h->lines(ctx, a, batch, Layout{1, dist, 0, 1}, mult);
         }
+        // the inverse's 1/N rides on the last axis
+        int left = nd;
         JT_TRY(real_axes(
             ctx, a, batch,
-            [&](Ctx &c, int64_t len, T *x, int64_t nb, const Layout &l) { return dht.at(len)->lines(c, x, nb, l, 1.0); },
+            [&](Ctx &c, int64_t len, T *x, int64_t nb, const Layout &l) {
+                return dht.at(len)->lines(c, x, nb, l, --left == 0 && !fwd && scale ? 1.0 / (double)N : 1.0);
+            },
             [&](int64_t len) { return dht.at(len)->strided_ok(ctx); }));
         for (int64_t b = 0; b < batch; b++) {
             T *p = a + b * dist;
             if (nd == 2) LAUNCH1D(ctx, (dims[0] / 2 + 1) * (dims[1] / 2 + 1), ytransform2_kernel<T>, p, dims[0], dims[1]);
             else LAUNCH1D(ctx, (dims[0] / 2 + 1) * (dims[1] / 2 + 1) * (dims[2] / 2 + 1), ytransform3_kernel<T>, p, dims[0], dims[1], dims[2]);
         }
-        if (!fwd && scale) LAUNCH1D(ctx, batch * N, scale_kernel<T>, a, dist, N, batch, 1.0 / (double)N);
         return JT_OK;
     }
 
