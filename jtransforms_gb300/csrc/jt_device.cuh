@@ -1228,6 +1228,19 @@ __global__ void ytransform3_kernel(T *a, int64_t slices, int64_t rows, int64_t c
     a[x4] = q - G;
 }
 
+// The right half of the spectrum of real data: F[-s][-r][C - k] = conj
+// F[s][r][k], 0 < k < C / 2 (C even), per array of S x R x C.
+template <typename T> __global__ void fill_symmetric_kernel(C2 *a, int64_t S, int64_t R, int64_t C, int64_t batch) {
+    const int64_t q = C / 2 - 1, idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (idx >= batch * S * R * q) return;
+    int64_t k, r, s;
+    const int64_t line = div_fast(idx, q, &k), sl = div_fast(line, R, &r), b = div_fast(sl, S, &s);
+    k++;
+    const C2 v = a[line * C + k];
+    const int64_t s2 = s ? S - s : 0, r2 = r ? R - r : 0;
+    a[((b * S + s2) * R + r2) * C + C - k] = cconj<T>(v);
+}
+
 // out[o][c][r] = in[o][r][c] for a batch of R x C matrices of E-byte
 // elements (E = 4, 8 or 16), 32x32 tiles through shared memory.
 template <typename E>

@@ -1950,6 +1950,8 @@ template <typename T> struct PlanImpl {
                 JT_TRY(get_fft(dims[1], &f));
                 return get_fft(dims[0], &f);
             }
+            if (nd > 1 && (op == JT_REAL_FORWARD_FULL || op == JT_REAL_INVERSE_FULL) && dims[nd - 1] % 2 == 0)
+                JT_TRY(get_real(dims[nd - 1], &r));
             for (int a = 0; a < nd; a++) JT_TRY(get_fft(dims[a], &f));
             return JT_OK;
         }
@@ -1998,6 +2000,48 @@ template <typename T> struct PlanImpl {
                 transpose<C2>(ctx, tmp, a, outer, inner, len);
             }
         }
+        return JT_OK;
+    }
+
+    // Full spectrum of real data, even rows: rows by half-length FFTs, the other
+    // axes over the left half of the columns, the right half by symmetry: half
+    // the arithmetic of the complex transform, and no copies of the reals.
+    int real_full_nd(Ctx &ctx, T *a, int64_t batch, int sign, bool scale) {
+        const int64_t n = dims[nd - 1], h = n / 2, R = dims[nd - 2], S = nd == 3 ? dims[0] : 1, rows = batch * S * R;
+        const Real1<T> *r = real.at(n).get();
+        const bool sc = sign > 0 && scale;
+        const double s = sc ? 1.0 / (double)n : 1.0;
+        C2 *c = (C2 *)a, *tmp = (C2 *)ctx.ws->get(sizeof(C2) * rows * h, ctx.dry);
+        JT_TRY(r->half->exec(ctx, c, h, tmp, h, rows, sign, 1.0));
+        if (sign < 0) LAUNCH1D(ctx, rows * (h / 2 + 1), (real_post_full_kernel<-1, T>), (const T *)tmp, n, a, 2 * n, n, rows, r->Wr, s);
+        else LAUNCH1D(ctx, rows * (h / 2 + 1), (real_post_full_kernel<1, T>), (const T *)tmp, n, a, 2 * n, n, rows, r->Wr, s);
+        // columns 0..h, to the next 16 (whole tiles of the column kernels); the
+        // ones beyond h are overwritten at the end
+        const int64_t w = std::min(n, (h + 16) & ~(int64_t)15);
+        Fft1<T> *fr = fft.at(R).get();
+        const double s1 = sc ? 1.0 / (double)R : 1.0;
+        JT_TRY(half_columns(ctx, fr, c, batch * S, R, w, n, R * n, n, sign, s1));
+        if (nd == 3) {
+            Fft1<T> *fs = fft.at(S).get();
+            for (int64_t b = 0; b < batch; b++)
+                JT_TRY(half_columns(ctx, fs, c + b * S * R * n, R, S, w, n, n, R * n, sign, sc ? 1.0 / (double)S : 1.0));
+        }
+        LAUNCH1D(ctx, rows * (h - 1), fill_symmetric_kernel<T>, c, S, R, n, batch);
+        return JT_OK;
+    }
+    // FFTs of length len over the first w columns of `blocks` blocks (stride
+    // `block`) of rows of n, elements `es` apart: in place where the length has
+    // a column kernel, else through a transposed copy of whole rows.
+    int half_columns(Ctx &ctx, Fft1<T> *f, C2 *a, int64_t blocks, int64_t len, int64_t w, int64_t n, int64_t block, int64_t es,
+                     int sign, double s) {
+        if (f->algo == ALG_TRIVIAL) return JT_OK;
+        const Layout l = {w, block, 1, es};
+        if (f->cols_ok()) return f->exec_direct(ctx, a, a, blocks * w, l, l, sign, s);
+        const int64_t outer = es == n ? blocks : 1, inner = es;  // [outer][len][inner], whole rows
+        C2 *tmp = (C2 *)ctx.ws->get(sizeof(C2) * outer * len * inner, ctx.dry);
+        transpose<C2>(ctx, a, tmp, outer, len, inner);
+        JT_TRY(f->exec(ctx, tmp, len, tmp, len, outer * inner, sign, s));
+        transpose<C2>(ctx, tmp, a, outer, inner, len);
         return JT_OK;
     }
 
@@ -2060,6 +2104,8 @@ template <typename T> struct PlanImpl {
                 case JT_COMPLEX_INVERSE: return complex_nd(ctx, (C2 *)a, batch, 1, scale);
                 case JT_REAL_FORWARD_FULL:
                 case JT_REAL_INVERSE_FULL: {
+                    if (dims[nd - 1] % 2 == 0)
+                        return real_full_nd(ctx, a, batch, op == JT_REAL_FORWARD_FULL ? -1 : 1, op == JT_REAL_INVERSE_FULL && scale);
                     T *tmp = (T *)ctx.ws->get(sizeof(T) * batch * N, ctx.dry);
                     LAUNCH1D(ctx, batch * N, copy_real_kernel<T>, a, dist, tmp, N, N, batch);
                     LAUNCH1D(ctx, batch * N, real_to_complex_kernel<T>, tmp, N, (C2 *)a, N, batch);
