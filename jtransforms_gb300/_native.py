@@ -125,6 +125,7 @@ class Plan:
         self.handle = h
         self.kind, self.prec, self.dims = kind, prec, tuple(int(x) for x in dims)
         self.dtype = np.float32 if prec == FLOAT32 else np.float64
+        self._extents = {}  # per op: the sizes never change
 
     def __del__(self):
         h = getattr(self, "handle", None)
@@ -136,9 +137,12 @@ class Plan:
             self.handle = None
 
     def extent(self, op: int) -> int:
-        v = ctypes.c_int64()
-        check(self._lib.jt_plan_extent(self.handle, op, ctypes.byref(v)))
-        return v.value
+        ext = self._extents.get(op)
+        if ext is None:
+            v = ctypes.c_int64()
+            check(self._lib.jt_plan_extent(self.handle, op, ctypes.byref(v)))
+            ext = self._extents[op] = v.value
+        return ext
 
     def set_mode(self, mode: int):
         check(self._lib.jt_plan_set_mode(self.handle, mode))

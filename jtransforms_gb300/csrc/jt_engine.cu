@@ -1457,6 +1457,7 @@ template <typename T> struct Real1 {
     int64_t n = 0;
     std::shared_ptr<Fft1<T>> half, full;
     C2 *Wr = nullptr;
+    bool half_generic = false;  // the tile passes run the half length
     ~Real1() {
         if (Wr) cudaFree(Wr);
     }
@@ -1466,6 +1467,7 @@ template <typename T> struct Real1 {
         r->n = n;
         if (n >= 2 && n % 2 == 0) {
             JT_TRY(cached<Fft1<T>>(n / 2, r->half));
+            r->half_generic = Fft1<T>::generic_ok(n / 2);
             JT_TRY(Fft1<T>::make_roots(&r->Wr, n / 4 + 1, 1, n, sizeof(T) == 8 && is_pow2(n)));
         } else if (n > 1) {
             JT_TRY(cached<Fft1<T>>(n, r->full));
@@ -1616,7 +1618,7 @@ template <typename T> struct Real1 {
 // ---------------------------------------------------------------------------
 template <typename T> static bool r2r_fused_ok(const Ctx &ctx, int64_t n, const Real1<T> *rf) {
     return n >= 4 && n % 2 == 0 && rf && rf->half && rf->half->algo == ALG_DIRECT && rf->half->W && rf->Wr &&
-           Fft1<T>::generic_ok(n / 2) && (!(ctx.rec || ctx.rec_sizing) || batch_line_ok<T>(n / 2));
+           rf->half_generic && (!(ctx.rec || ctx.rec_sizing) || batch_line_ok<T>(n / 2));
 }
 
 // Lines per CTA of the register form for half length h (0: none): power-of-
@@ -1643,13 +1645,17 @@ static int r2r_fused(Ctx &ctx, int op, const Real1<T> *rf, const T *in, T *out, 
     typedef typename V2<T>::t C2;
     if (nlines <= 0) return JT_OK;
     const int64_t n = rf->n, h = n / 2;
-    std::vector<int> rr = direct_radices(h, radix_order(h, sizeof(T) == 4));
-    if (rr.empty() || (int)rr.size() > JT_MAX_PASSES) return JT_EINVAL;
     R2rParams p;
     memset(&p, 0, sizeof(p));
     p.n = (int)n;
-    p.npass = (int)rr.size();
-    for (int i = 0; i < p.npass; i++) p.radix[i] = rr[i];
+    // passes of the tile form
+    auto set_radices = [&]() -> bool {
+        const std::vector<int> rr = direct_radices(h, radix_order(h, sizeof(T) == 4));
+        if (rr.empty() || (int)rr.size() > JT_MAX_PASSES) return false;
+        p.npass = (int)rr.size();
+        for (int i = 0; i < p.npass; i++) p.radix[i] = rr[i];
+        return true;
+    };
     const bool strided = lin.estride != 1 || lout.estride != 1;
     int C = (int)std::max<int64_t>(1, (ctx.rec ? kBatchTileElems : (sizeof(T) == 4 ? 4096 : 2048)) / h);
     if (strided) C = std::max(C, sizeof(T) == 4 ? 16 : 8);
@@ -1674,6 +1680,7 @@ static int r2r_fused(Ctx &ctx, int op, const Real1<T> *rf, const T *in, T *out, 
     p.vec_out = paired(out, lout) ? 1 : 0;
     if (ctx.rec) {
         // a batch step: the tile form, run by the batch kernel's CTAs
+        if (!set_radices()) return JT_EINVAL;
         BOp o;
         memset(&o, 0, sizeof(o));
         o.type = BOP_R2R;
@@ -1722,6 +1729,7 @@ static int r2r_fused(Ctx &ctx, int op, const Real1<T> *rf, const T *in, T *out, 
         }
     }
     if (ctx.dry) return JT_OK;
+    if (!set_radices()) return JT_EINVAL;
     const int64_t grid = cdiv(nlines, C);
     if (grid > 0x7fffffff) return JT_ETOOBIG;
     const int threads = (int)std::min<int64_t>(512, std::max<int64_t>(64, cdiv((int64_t)C * h / 8, 32) * 32));
@@ -2229,6 +2237,7 @@ namespace {
 #define JT_HOST_RING 3
 
 struct ThreadState {
+    int *err_word = nullptr;  // pinned: the device error flag, copied out with the result
     cudaStream_t stream = nullptr;
     cudaStream_t h2d = nullptr, d2h = nullptr;
     cudaEvent_t in_done[JT_HOST_RING] = {}, run_done[JT_HOST_RING] = {}, out_done[JT_HOST_RING] = {};
@@ -2246,6 +2255,11 @@ int ensure_stream() {
         JT_CU(cudaStreamCreateWithFlags(&t_state.stream, cudaStreamNonBlocking));
         JT_CU(cudaEventCreateWithFlags(&t_state.done, cudaEventDisableTiming));
     }
+    return JT_OK;
+}
+
+int ensure_err_word() {
+    if (!t_state.err_word) JT_CU(cudaMallocHost(&t_state.err_word, sizeof(int)));
     return JT_OK;
 }
 
@@ -2470,7 +2484,7 @@ int exec_host(jt_plan *p, int op, void *host, int64_t len, int64_t off, int64_t 
     if (off + (batch - 1) * dist + ext > len) return JT_ESHORTBUF;
     JT_TRY(device_init());
     JT_TRY(ensure_stream());
-    JT_TRY(ensure_copy_streams());
+    JT_TRY(ensure_err_word());
     cudaStream_t s = t_state.stream;
     // device copy laid out densely at distance ext (even, for complex views)
     int64_t dd = (ext + 1) & ~(int64_t)1;
@@ -2496,7 +2510,10 @@ int exec_host(jt_plan *p, int op, void *host, int64_t len, int64_t off, int64_t 
     for (int r = 0; r < ring; r++) t_state.arena.get(per * piece, true);
     std::lock_guard<std::mutex> g(im->mu);
     JT_TRY(im->run(c, op, (T *)nullptr, piece, dd, scale != 0));
-    const int64_t budget = device_budget();
+    // (scratch that the arena already holds needs no look at the free memory,
+    // which takes longer than a small transform)
+    const bool held = t_state.arena.peak <= t_state.arena.cap && g_opt_arena_limit.load() == 0;
+    const int64_t budget = held ? INT64_MAX : device_budget();
     if ((int64_t)t_state.arena.peak > budget) {
         // one transform's working set exceeds the device: complex 1D
         // multi-pass lengths stream through host pieces, the rest fail
@@ -2526,10 +2543,18 @@ int exec_host(jt_plan *p, int op, void *host, int64_t len, int64_t off, int64_t 
         JT_CU(cudaEventRecord(t_state.done, t_state.last));
         JT_CU(cudaStreamWaitEvent(s, t_state.done, 0));
     }
-    // the copy streams start after earlier work on this thread's arena
-    JT_CU(cudaEventRecord(t_state.done, s));
-    JT_CU(cudaStreamWaitEvent(t_state.h2d, t_state.done, 0));
-    JT_CU(cudaStreamWaitEvent(t_state.d2h, t_state.done, 0));
+    // one piece has nothing to overlap: its copies go to the transform's stream
+    const bool one = npieces == 1;
+    cudaStream_t in_s = s, out_s = s;
+    if (!one) {
+        JT_TRY(ensure_copy_streams());
+        in_s = t_state.h2d;
+        out_s = t_state.d2h;
+        // the copy streams start after earlier work on this thread's arena
+        JT_CU(cudaEventRecord(t_state.done, s));
+        JT_CU(cudaStreamWaitEvent(in_s, t_state.done, 0));
+        JT_CU(cudaStreamWaitEvent(out_s, t_state.done, 0));
+    }
     t_state.arena.used = 0;
     c.dry = false;
     T *buf[JT_HOST_RING];
@@ -2550,25 +2575,34 @@ int exec_host(jt_plan *p, int op, void *host, int64_t len, int64_t off, int64_t 
         const int r = (int)(i % ring);
         const int64_t b0 = i * piece, nb = std::min(piece, batch - b0);
         // buffer r is free once the copy out of piece i - ring finished
-        if (i >= ring) JT_CU(cudaStreamWaitEvent(t_state.h2d, t_state.out_done[r], 0));
-        JT_TRY(copy(buf[r], h + b0 * dist, nb, cudaMemcpyHostToDevice, t_state.h2d));
-        JT_CU(cudaEventRecord(t_state.in_done[r], t_state.h2d));
-        JT_CU(cudaStreamWaitEvent(s, t_state.in_done[r], 0));
+        if (i >= ring) JT_CU(cudaStreamWaitEvent(in_s, t_state.out_done[r], 0));
+        JT_TRY(copy(buf[r], h + b0 * dist, nb, cudaMemcpyHostToDevice, in_s));
+        if (!one) {
+            JT_CU(cudaEventRecord(t_state.in_done[r], in_s));
+            JT_CU(cudaStreamWaitEvent(s, t_state.in_done[r], 0));
+        }
         t_state.arena.used = mark;  // the pieces run in order on one stream: one scratch region
         JT_TRY(im->run(c, op, buf[r], nb, dd, scale != 0));
-        JT_CU(cudaEventRecord(t_state.run_done[r], s));
-        JT_CU(cudaStreamWaitEvent(t_state.d2h, t_state.run_done[r], 0));
-        JT_TRY(copy(h + b0 * dist, buf[r], nb, cudaMemcpyDeviceToHost, t_state.d2h));
-        JT_CU(cudaEventRecord(t_state.out_done[r], t_state.d2h));
+        if (!one) {
+            JT_CU(cudaEventRecord(t_state.run_done[r], s));
+            JT_CU(cudaStreamWaitEvent(out_s, t_state.run_done[r], 0));
+        }
+        JT_TRY(copy(h + b0 * dist, buf[r], nb, cudaMemcpyDeviceToHost, out_s));
+        if (!one) JT_CU(cudaEventRecord(t_state.out_done[r], out_s));
     }
     // later work on this thread's arena (on any stream) follows the copies out
-    JT_CU(cudaEventRecord(t_state.done, t_state.d2h));
-    JT_CU(cudaStreamWaitEvent(s, t_state.done, 0));
+    if (!one) {
+        JT_CU(cudaEventRecord(t_state.done, out_s));
+        JT_CU(cudaStreamWaitEvent(s, t_state.done, 0));
+    }
     t_state.last = s;
-    JT_CU(cudaStreamSynchronize(t_state.d2h));
+    // the error flag comes out with the result: one wait for both
+    JT_CU(cudaMemcpyAsync(t_state.err_word, g_err_dev, sizeof(int), cudaMemcpyDeviceToHost, s));
     JT_CU(cudaStreamSynchronize(s));
     JT_CU(cudaGetLastError());
-    return check_err_flag();
+    if (!*t_state.err_word) return JT_OK;
+    JT_CU(cudaMemset(g_err_dev, 0, sizeof(int)));
+    return JT_ETIMEOUT;
 }
 
 }  // namespace
