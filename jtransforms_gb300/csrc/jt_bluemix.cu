@@ -11,14 +11,14 @@ void blue_setup(int smem_optin) {
 }
 
 void blue_mid(bool one, const float2 *in, float2 *out, const BlueMid &q, unsigned grid, int threads, size_t smem, cudaStream_t s) {
-    if (one) blue_mid_kernel<true><<<grid, threads, smem, s>>>(in, out, q);
-    else blue_mid_kernel<false><<<grid, threads, smem, s>>>(in, out, q);
+    if (one) pdl_launch(blue_mid_kernel<true>, grid, threads, smem, s, in, out, q);
+    else pdl_launch(blue_mid_kernel<false>, grid, threads, smem, s, in, out, q);
 }
 
 void blue_cols(bool first, const float2 *in, float2 *out, const MixParams &p, const MixBlue &bl, const float2 *tw, unsigned grid,
                int threads, size_t smem, cudaStream_t s) {
-    if (first) blue_cols_kernel<-1, MIX_BLUE_IN><<<grid, threads, smem, s>>>(in, out, p, bl, tw);
-    else blue_cols_kernel<1, MIX_BLUE_OUT><<<grid, threads, smem, s>>>(in, out, p, bl, tw);
+    if (first) pdl_launch(blue_cols_kernel<-1, MIX_BLUE_IN>, grid, threads, smem, s, in, out, p, bl, tw);
+    else pdl_launch(blue_cols_kernel<1, MIX_BLUE_OUT>, grid, threads, smem, s, in, out, p, bl, tw);
 }
 
 void blue_twiddle(float2 *out, int n1, int n2, cudaStream_t s) {

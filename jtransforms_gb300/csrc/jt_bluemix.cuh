@@ -150,6 +150,7 @@ template <bool ONE> struct BlueTile {
 
 template <bool ONE> __global__ void __launch_bounds__(JT_MIX_THREADS, 2) blue_mid_kernel(const float2 *in, float2 *out, BlueMid q) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_begin();
     const int64_t b0 = (int64_t)blockIdx.x * q.f.C;
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
     BlueTile<ONE>{in, out, q, b0, (int)min((int64_t)q.f.C, q.f.nlines - b0)}.run(A, A + q.f.C * q.f.Lp);
@@ -160,6 +161,7 @@ template <int SIGN, int POL>
 __global__ void __launch_bounds__(JT_MIX_THREADS, 2) blue_cols_kernel(const float2 *in, float2 *out, MixParams p, MixBlue bl,
                                                                       const float2 *__restrict__ tw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_begin();
     const int64_t b0 = (int64_t)blockIdx.x * p.C;
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
     MixTile<SIGN, 1, POL>{in, out, p, tw, nullptr, nullptr, b0, (int)min((int64_t)p.C, p.nlines - b0), bl}.run(A, A + p.C * p.Lp);

@@ -77,6 +77,7 @@ template <int SIGN, typename T>
 __global__ void __launch_bounds__(512) blue_tile_kernel(const C2 *in, C2 *out, BlueParams p, const C2 *__restrict__ W,
                                                         const C2 *__restrict__ bk1, const C2 *__restrict__ bk2) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_begin();
     blue_tile_body<SIGN, T>(in, out, p, W, bk1, bk2, (int64_t)blockIdx.x, smem_raw);
 }
 

@@ -26,6 +26,7 @@
 #include <stdint.h>
 
 #include "jt_fixmath.cuh"
+#include "jt_launch.cuh"
 
 namespace jt {
 
@@ -662,6 +663,7 @@ __device__ void tile_fft_body(const C2 *in, C2 *out, const TileParams &p, const 
 template <int SIGN, typename T>
 __global__ void __launch_bounds__(512) fft_tile_kernel(const C2 *in, C2 *out, TileParams p, const C2 *__restrict__ W,
                                                         const C2 *__restrict__ Whi, const C2 *__restrict__ Wlo) {
+    pdl_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     tile_fft_body<SIGN, T>(in, out, p, W, Whi, Wlo, (int64_t)blockIdx.x, smem_raw);
 }
@@ -739,6 +741,7 @@ __device__ __forceinline__ void bluestein_pre_body(const C2 *a, int64_t dist, C2
 template <int SIGN, typename T>
 __global__ void bluestein_pre_kernel(const C2 *a, int64_t dist, C2 *tmp, const C2 *__restrict__ bk1, int64_t n, int64_t nB,
                                      int64_t batch) {
+    pdl_begin();
     bluestein_pre_body<SIGN, T>(a, dist, tmp, bk1, n, nB, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -751,6 +754,7 @@ __device__ __forceinline__ void bluestein_mul_body(C2 *tmp, const C2 *__restrict
 
 template <int SIGN, typename T>
 __global__ void bluestein_mul_kernel(C2 *tmp, const C2 *__restrict__ bk2, int64_t nB, int64_t total) {
+    pdl_begin();
     bluestein_mul_body<SIGN, T>(tmp, bk2, nB, total, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -768,6 +772,7 @@ __device__ __forceinline__ void bluestein_post_body(C2 *a, int64_t dist, const C
 template <int SIGN, typename T>
 __global__ void bluestein_post_kernel(C2 *a, int64_t dist, const C2 *tmp, const C2 *__restrict__ bk1, int64_t n, int64_t nB,
                                       int64_t batch, T scale) {
+    pdl_begin();
     bluestein_post_body<SIGN, T>(a, dist, tmp, bk1, n, nB, batch, scale, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -815,6 +820,7 @@ __device__ __forceinline__ void real_post_packed_body(T *a, int64_t dist, int64_
 
 template <typename T>
 __global__ void real_post_packed_kernel(T *a, int64_t dist, int64_t n, int64_t batch, const C2 *__restrict__ Wr) {
+    pdl_begin();
     real_post_packed_body<T>(a, dist, n, batch, Wr, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -855,6 +861,7 @@ __device__ __forceinline__ void real_post_full_body(const T *zin, int64_t zdist,
 template <int SIGN, typename T>
 __global__ void real_post_full_kernel(const T *zin, int64_t zdist, T *out, int64_t odist, int64_t n, int64_t batch,
                                       const C2 *__restrict__ Wr, T scale) {
+    pdl_begin();
     real_post_full_body<SIGN, T>(zin, zdist, out, odist, n, batch, Wr, scale, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -894,6 +901,7 @@ __device__ __forceinline__ void real_pre_inverse_body(T *a, int64_t dist, int64_
 
 template <typename T>
 __global__ void real_pre_inverse_kernel(T *a, int64_t dist, int64_t n, int64_t batch, const C2 *__restrict__ Wr, T mult) {
+    pdl_begin();
     real_pre_inverse_body<T>(a, dist, n, batch, Wr, mult, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -908,6 +916,7 @@ __device__ __forceinline__ void real_to_complex_body(const T *a, int64_t dist, C
 
 template <typename T>
 __global__ void real_to_complex_kernel(const T *a, int64_t dist, C2 *tmp, int64_t n, int64_t batch) {
+    pdl_begin();
     real_to_complex_body<T>(a, dist, tmp, n, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -929,6 +938,7 @@ __device__ __forceinline__ void pack_from_full_body(const C2 *F, T *a, int64_t d
 
 template <typename T>
 __global__ void pack_from_full_kernel(const C2 *F, T *a, int64_t dist, int64_t n, int64_t batch) {
+    pdl_begin();
     pack_from_full_body<T>(F, a, dist, n, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -950,6 +960,7 @@ __device__ __forceinline__ void unpack_to_full_body(const T *a, int64_t dist, C2
 
 template <typename T>
 __global__ void unpack_to_full_kernel(const T *a, int64_t dist, C2 *F, int64_t n, int64_t batch) {
+    pdl_begin();
     unpack_to_full_body<T>(a, dist, F, n, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -963,6 +974,7 @@ __device__ __forceinline__ void real_part_body(const C2 *F, T *a, int64_t dist, 
 
 template <typename T>
 __global__ void real_part_kernel(const C2 *F, T *a, int64_t dist, int64_t n, int64_t batch, T mult) {
+    pdl_begin();
     real_part_body<T>(F, a, dist, n, batch, mult, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -981,6 +993,7 @@ __device__ __forceinline__ void copy_complex_body(const C2 *src, int64_t sdist, 
 template <typename T>
 __global__ void copy_complex_kernel(const C2 *src, int64_t sdist, C2 *dst, int64_t ddist, int64_t len, int64_t batch,
                                     T scale, int conj) {
+    pdl_begin();
     copy_complex_body<T>(src, sdist, dst, ddist, len, batch, scale, conj, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1001,6 +1014,7 @@ __device__ __forceinline__ void dct2_pre_body(const T *a, int64_t dist, T *v, in
 
 template <typename T>
 __global__ void dct2_pre_kernel(const T *a, int64_t dist, T *v, int64_t vdist, int64_t n, int64_t batch, int dst) {
+    pdl_begin();
     dct2_pre_body<T>(a, dist, v, vdist, n, batch, dst, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1031,6 +1045,7 @@ __device__ __forceinline__ void dct2_post_body(const T *v, int64_t vdist, T *a, 
 template <typename T>
 __global__ void dct2_post_kernel(const T *v, int64_t vdist, T *a, int64_t dist, int64_t n, int64_t batch,
                                  const C2 *__restrict__ Wd, T mult, T mult0, int dst) {
+    pdl_begin();
     dct2_post_body<T>(v, vdist, a, dist, n, batch, Wd, mult, mult0, dst, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1063,6 +1078,7 @@ __device__ __forceinline__ void dct3_pre_body(const T *a, int64_t dist, T *v, in
 template <typename T>
 __global__ void dct3_pre_kernel(const T *a, int64_t dist, T *v, int64_t vdist, int64_t n, int64_t batch,
                                 const C2 *__restrict__ Wd, T mult, T mult0, int dst) {
+    pdl_begin();
     dct3_pre_body<T>(a, dist, v, vdist, n, batch, Wd, mult, mult0, dst, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1079,6 +1095,7 @@ __device__ __forceinline__ void dct3_post_body(const T *v, int64_t vdist, T *a, 
 
 template <typename T>
 __global__ void dct3_post_kernel(const T *v, int64_t vdist, T *a, int64_t dist, int64_t n, int64_t batch, int dst) {
+    pdl_begin();
     dct3_post_body<T>(v, vdist, a, dist, n, batch, dst, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1093,6 +1110,7 @@ __device__ __forceinline__ void dht_post_body(const T *v, int64_t vdist, T *a, i
 
 template <typename T>
 __global__ void dht_post_kernel(const T *v, int64_t vdist, T *a, int64_t dist, int64_t n, int64_t batch, T mult) {
+    pdl_begin();
     dht_post_body<T>(v, vdist, a, dist, n, batch, mult, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1103,6 +1121,7 @@ __global__ void dht_post_kernel(const T *v, int64_t vdist, T *a, int64_t dist, i
 // pass of realForward, -1 before the column pass of realInverse.
 template <typename T>
 __global__ void rdft2d_kernel(T *a, int64_t dist, int64_t rows, int64_t cols, int64_t batch, int isgn) {
+    pdl_begin();
     const int64_t n1h = rows >> 1;
     const int64_t q = n1h > 1 ? n1h - 1 : 0;
     int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1133,6 +1152,7 @@ __global__ void rdft2d_kernel(T *a, int64_t dist, int64_t rows, int64_t cols, in
 // pairs are disjoint, so any order gives the reference's result.
 template <typename T>
 __global__ void rdft3d_kernel(T *a, int64_t dist, int64_t slices, int64_t rows, int64_t cols, int64_t batch, int isgn) {
+    pdl_begin();
     const int64_t n1h = slices >> 1, n2h = rows >> 1, ss = rows * cols, rs = cols;
     const int64_t per = n1h * n2h * 2;
     int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1183,6 +1203,7 @@ __global__ void rdft3d_kernel(T *a, int64_t dist, int64_t slices, int64_t rows, 
 // order; they never share elements with other quadruples.
 template <typename T>
 __global__ void ytransform2_kernel(T *a, int64_t rows, int64_t cols) {
+    pdl_begin();
     int64_t nr = rows / 2 + 1, nc = cols / 2 + 1;
     int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (idx >= nr * nc) return;
@@ -1200,6 +1221,7 @@ __global__ void ytransform2_kernel(T *a, int64_t rows, int64_t cols) {
 // DHT yTransform, 3D (dht/DoubleDHT_3D.java:2314-2356)
 template <typename T>
 __global__ void ytransform3_kernel(T *a, int64_t slices, int64_t rows, int64_t cols) {
+    pdl_begin();
     int64_t ns = slices / 2 + 1, nr = rows / 2 + 1, nc = cols / 2 + 1;
     int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (idx >= ns * nr * nc) return;
@@ -1231,6 +1253,7 @@ __global__ void ytransform3_kernel(T *a, int64_t slices, int64_t rows, int64_t c
 // The right half of the spectrum of real data: F[-s][-r][C - k] = conj
 // F[s][r][k], 0 < k < C / 2 (C even), per array of S x R x C.
 template <typename T> __global__ void fill_symmetric_kernel(C2 *a, int64_t S, int64_t R, int64_t C, int64_t batch) {
+    pdl_begin();
     const int64_t q = C / 2 - 1, idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (idx >= batch * S * R * q) return;
     int64_t k, r, s;
@@ -1245,6 +1268,7 @@ template <typename T> __global__ void fill_symmetric_kernel(C2 *a, int64_t S, in
 // elements (E = 4, 8 or 16), 32x32 tiles through shared memory.
 template <typename E>
 __global__ void transpose_kernel(const E *in, E *out, int64_t R, int64_t C, int64_t outer) {
+    pdl_begin();
     __shared__ E tile[32][33];
     int64_t tilesC = (C + 31) / 32, tilesR = (R + 31) / 32;
     int64_t t = blockIdx.x;
@@ -1273,6 +1297,7 @@ template <typename T> __device__ __forceinline__ void scale_body(T *a, int64_t d
 }
 
 template <typename T> __global__ void scale_kernel(T *a, int64_t dist, int64_t len, int64_t batch, T s) {
+    pdl_begin();
     scale_body(a, dist, len, batch, s, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1284,6 +1309,7 @@ template <typename T> __device__ __forceinline__ void copy_real_body(const T *sr
 }
 
 template <typename T> __global__ void copy_real_kernel(const T *src, int64_t sdist, T *dst, int64_t ddist, int64_t len, int64_t batch) {
+    pdl_begin();
     copy_real_body(src, sdist, dst, ddist, len, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 

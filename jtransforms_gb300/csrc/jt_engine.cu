@@ -135,7 +135,7 @@ static inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
         if (!(ctx).dry && (total) > 0) {                                               \
             int64_t g_ = cdiv((total), 256);                                           \
             auto kfn_ = kernel;                                                        \
-            kfn_<<<(unsigned)g_, 256, 0, (ctx).s>>>(__VA_ARGS__);                      \
+            pdl_launch(kfn_, (unsigned)g_, 256, 0, (ctx).s, __VA_ARGS__);              \
             g_launches++;                                                              \
         }                                                                              \
     } while (0)
@@ -1062,9 +1062,9 @@ template <typename T> struct Fft1 {
         if (grid > 0x7fffffff) return JT_ETOOBIG;
         const int threads = (int)std::min<int64_t>(512, std::max<int64_t>(64, cdiv((int64_t)C * nB / 16, 32) * 32));
         if (sign < 0)
-            blue_tile_kernel<-1, T><<<(unsigned)grid, threads, per_line * C, ctx.s>>>(in, out, p, pbl->W, bk1, bk2);
+            pdl_launch(blue_tile_kernel<-1, T>, (unsigned)grid, threads, per_line * C, ctx.s, in, out, p, pbl->W, bk1, bk2);
         else
-            blue_tile_kernel<1, T><<<(unsigned)grid, threads, per_line * C, ctx.s>>>(in, out, p, pbl->W, bk1, bk2);
+            pdl_launch(blue_tile_kernel<1, T>, (unsigned)grid, threads, per_line * C, ctx.s, in, out, p, pbl->W, bk1, bk2);
         g_launches++;
         return JT_OK;
     }
@@ -1230,9 +1230,9 @@ template <typename T> struct Fft1 {
         int64_t grid = cdiv(nlines, C);
         if (grid > 0x7fffffff) return JT_ETOOBIG;
         if (sign < 0)
-            fft_tile_kernel<-1, T><<<(unsigned)grid, threads, smem, ctx.s>>>(in, out, p, W, Whi_, Wlo_);
+            pdl_launch(fft_tile_kernel<-1, T>, (unsigned)grid, threads, smem, ctx.s, in, out, p, W, Whi_, Wlo_);
         else
-            fft_tile_kernel<1, T><<<(unsigned)grid, threads, smem, ctx.s>>>(in, out, p, W, Whi_, Wlo_);
+            pdl_launch(fft_tile_kernel<1, T>, (unsigned)grid, threads, smem, ctx.s, in, out, p, W, Whi_, Wlo_);
         g_launches++;
         return JT_OK;
     }
@@ -1735,11 +1735,11 @@ static int r2r_fused(Ctx &ctx, int op, const Real1<T> *rf, const T *in, T *out, 
     const int threads = (int)std::min<int64_t>(512, std::max<int64_t>(64, cdiv((int64_t)C * h / 8, 32) * 32));
     const size_t smem = per_line * C;
     const C2 *W = rf->half->W;
-    if (op == R2R_DCT2) r2r_tile_kernel<R2R_DCT2, T><<<(unsigned)grid, threads, smem, ctx.s>>>(in, out, p, W, rf->Wr, Wd);
-    else if (op == R2R_DCT3) r2r_tile_kernel<R2R_DCT3, T><<<(unsigned)grid, threads, smem, ctx.s>>>(in, out, p, W, rf->Wr, Wd);
-    else if (op == R2R_DHT) r2r_tile_kernel<R2R_DHT, T><<<(unsigned)grid, threads, smem, ctx.s>>>(in, out, p, W, rf->Wr, Wd);
-    else if (op == R2R_RFWD) r2r_tile_kernel<R2R_RFWD, T><<<(unsigned)grid, threads, smem, ctx.s>>>(in, out, p, W, rf->Wr, Wd);
-    else r2r_tile_kernel<R2R_RINV, T><<<(unsigned)grid, threads, smem, ctx.s>>>(in, out, p, W, rf->Wr, Wd);
+    if (op == R2R_DCT2) pdl_launch(r2r_tile_kernel<R2R_DCT2, T>, (unsigned)grid, threads, smem, ctx.s, in, out, p, W, rf->Wr, Wd);
+    else if (op == R2R_DCT3) pdl_launch(r2r_tile_kernel<R2R_DCT3, T>, (unsigned)grid, threads, smem, ctx.s, in, out, p, W, rf->Wr, Wd);
+    else if (op == R2R_DHT) pdl_launch(r2r_tile_kernel<R2R_DHT, T>, (unsigned)grid, threads, smem, ctx.s, in, out, p, W, rf->Wr, Wd);
+    else if (op == R2R_RFWD) pdl_launch(r2r_tile_kernel<R2R_RFWD, T>, (unsigned)grid, threads, smem, ctx.s, in, out, p, W, rf->Wr, Wd);
+    else pdl_launch(r2r_tile_kernel<R2R_RINV, T>, (unsigned)grid, threads, smem, ctx.s, in, out, p, W, rf->Wr, Wd);
     g_launches++;
     return JT_OK;
 }
@@ -1975,7 +1975,7 @@ template <typename T> struct PlanImpl {
     template <typename E> void transpose(Ctx &ctx, const E *in, E *out, int64_t outer, int64_t R, int64_t Cc) const {
         if (ctx.dry || outer * R * Cc == 0) return;
         int64_t blocks = outer * cdiv(R, 32) * cdiv(Cc, 32);
-        transpose_kernel<E><<<(unsigned)blocks, dim3(32, 8), 0, ctx.s>>>(in, out, R, Cc, outer);
+        pdl_launch(transpose_kernel<E>, (unsigned)blocks, dim3(32, 8), 0, ctx.s, in, out, R, Cc, outer);
         g_launches++;
     }
 

@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::NT,
     typedef typename F::S S;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t red[F::RED];
+    pdl_begin();
     Fx *xs = reinterpret_cast<Fx *>(smem_raw);
     const int tid = threadIdx.x, NT = blockDim.x, C = NT / F::TL;
     const int c = MODE == 0 ? tid / F::TL : tid & (C - 1), t = MODE == 0 ? tid % F::TL : tid / C;
@@ -318,7 +319,7 @@ template <int L> struct FixLaunch {
         }
         const int C = fix_lines(p.nlines, CM, std::min(CM, std::max(F::CMIN, MODE == 0 ? 1 : 4)), sms);
         const int64_t ntiles = (p.nlines + C - 1) / C;
-        kern<<<(unsigned)ntiles, C * F::TL, (size_t)C * F::stride(C) * sizeof(Fx), s>>>(in, out, p, W, Whi, Wlo, Wq, Whiq, Wloq);
+        pdl_launch(kern, (unsigned)ntiles, C * F::TL, (size_t)C * F::stride(C) * sizeof(Fx), s, in, out, p, W, Whi, Wlo, Wq, Whiq, Wloq);
     }
     template <int MODE, int SIGN, typename... A> static void tw(const double2 *in, double2 *out, const StockParams &p, A... a) {
         if constexpr (MODE == 1) {

@@ -14,6 +14,7 @@ __device__ __noinline__ void fixmix_fp64(const double2 *in, double2 *out, const 
 
 __global__ void __launch_bounds__(JT_FIXMIX_THREADS, 1) fixmix_kernel(const double2 *in, double2 *out, FixMixParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_begin();
     const int64_t b0 = (int64_t)blockIdx.x * p.m.C;
     const int lines = (int)min((int64_t)p.m.C, p.m.nlines - b0), nbuf = p.m.npass > 2 ? 2 : 1;
     Fx *A = reinterpret_cast<Fx *>(smem_raw);
@@ -43,7 +44,7 @@ void fixmix_table(int4 *out, const MixParams &p, int count, cudaStream_t s) {
 }
 
 void fixmix_launch(const double2 *in, double2 *out, const FixMixParams &p, unsigned grid, int threads, size_t smem, cudaStream_t s) {
-    fixmix_kernel<<<grid, threads, smem, s>>>(in, out, p);
+    pdl_launch(fixmix_kernel, grid, threads, smem, s, in, out, p);
 }
 
 }  // namespace jt

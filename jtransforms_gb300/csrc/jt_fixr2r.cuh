@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
     auto pad = [](int i) { return F::pad(i); };
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t red[F::RED];
+    pdl_begin();
     Fx *xs = reinterpret_cast<Fx *>(smem_raw);
     double2 *xd = reinterpret_cast<double2 *>(smem_raw);
     const int tid = threadIdx.x, NT = blockDim.x, C = NT / TL;
@@ -388,8 +389,8 @@ template <int H> struct FixR2rLaunch {
         }
         p.C = fix_lines(p.nlines, G::CM, std::min(G::CM, std::max(F::CMIN, MODE == 0 ? 1 : 4)), sms);
         const int64_t grid = (p.nlines + p.C - 1) / p.C;
-        fix_r2r_kernel<H, MODE, OP><<<(unsigned)grid, p.C * F::TL, (size_t)p.C * F::stride(p.C) * sizeof(Fx), s>>>(in, out, p, fs, Wp, Wr, Wd,
-                                                                                                           Wpq, Wrq, Wdq);
+        pdl_launch(fix_r2r_kernel<H, MODE, OP>, (unsigned)grid, p.C * F::TL, (size_t)p.C * F::stride(p.C) * sizeof(Fx), s, in, out, p, fs,
+                   Wp, Wr, Wd, Wpq, Wrq, Wdq);
     }
     template <int MODE, typename... A> static void op(int op, A... a) {
         if (op == R2R_DCT2) one<MODE, R2R_DCT2>(a...);

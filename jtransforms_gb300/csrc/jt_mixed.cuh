@@ -348,6 +348,7 @@ template <int SIGN, int MODE>
 __global__ void __launch_bounds__(JT_MIX_THREADS, 2) mix_kernel(const float2 *in, float2 *out, MixParams p, const float2 *__restrict__ tw,
                                                                 const float2 *__restrict__ Whi, const float2 *__restrict__ Wlo) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_begin();
     const int64_t b0 = (int64_t)blockIdx.x * p.C;
     float2 *A = reinterpret_cast<float2 *>(smem_raw);
     MixTile<SIGN, MODE>{in, out, p, tw, Whi, Wlo, b0, (int)min((int64_t)p.C, p.nlines - b0), MixBlue{}}.run(A, A + p.C * p.Lp);

@@ -6,9 +6,9 @@ namespace jt {
 
 void mix_launch_inv(int mode, const float2 *in, float2 *out, const MixParams &p, const float2 *tw, const float2 *Whi,
                      const float2 *Wlo, unsigned grid, int threads, size_t smem, cudaStream_t s) {
-    if (mode == 0) mix_kernel<1, 0><<<grid, threads, smem, s>>>(in, out, p, tw, Whi, Wlo);
-    else if (mode == 1) mix_kernel<1, 1><<<grid, threads, smem, s>>>(in, out, p, tw, Whi, Wlo);
-    else mix_kernel<1, 2><<<grid, threads, smem, s>>>(in, out, p, tw, Whi, Wlo);
+    if (mode == 0) pdl_launch(mix_kernel<1, 0>, grid, threads, smem, s, in, out, p, tw, Whi, Wlo);
+    else if (mode == 1) pdl_launch(mix_kernel<1, 1>, grid, threads, smem, s, in, out, p, tw, Whi, Wlo);
+    else pdl_launch(mix_kernel<1, 2>, grid, threads, smem, s, in, out, p, tw, Whi, Wlo);
 }
 
 void mix_setup_inv(int smem_optin) {

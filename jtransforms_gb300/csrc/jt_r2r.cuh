@@ -333,6 +333,7 @@ template <int OP, typename T>
 __global__ void __launch_bounds__(512) r2r_tile_kernel(const T *in, T *out, R2rParams p, const C2 *__restrict__ W,
                                                        const C2 *__restrict__ Wr, const C2 *__restrict__ Wd) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_begin();
     r2r_tile_body<OP, T>(in, out, p, W, Wr, Wd, (int64_t)blockIdx.x, smem_raw);
 }
 
@@ -521,6 +522,7 @@ __global__ void __launch_bounds__(R2rReg<T, H, OP>::S::NT)
     r2r_reg_kernel(const T *in, T *out, R2rParams p, const C2 *__restrict__ Wp, const C2 *__restrict__ Wr,
                    const C2 *__restrict__ Wd) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_begin();
     r2r_reg_body<T, H, OP>(in, out, p, Wp, Wr, Wd, smem_raw);
 }
 
@@ -538,7 +540,7 @@ template <typename T, int H> struct R2rRegLaunch {
         // p.C lines per CTA (1 .. S::C): p.C * TL threads, p.C rows of shared memory
         const int64_t grid = (p.nlines + p.C - 1) / p.C;
         const size_t smem = (size_t)p.C * G::RX * sizeof(typename V2<T>::t);
-        r2r_reg_kernel<T, H, OP><<<(unsigned)grid, p.C * G::S::TL, smem, s>>>(in, out, p, Wp, Wr, Wd);
+        pdl_launch(r2r_reg_kernel<T, H, OP>, (unsigned)grid, p.C * G::S::TL, smem, s, in, out, p, Wp, Wr, Wd);
     }
     static void go(int op, const T *in, T *out, const R2rParams &p, const C2 *Wp, const C2 *Wr, const C2 *Wd, cudaStream_t s) {
         if (op == R2R_DCT2) one<R2R_DCT2>(in, out, p, Wp, Wr, Wd, s);

@@ -419,6 +419,7 @@ __global__ void __launch_bounds__(Stockham<T, L, MODE, SIGN>::NT)
                     const typename V2<T>::t *__restrict__ W, const typename V2<T>::t *__restrict__ Whi,
                     const typename V2<T>::t *__restrict__ Wlo) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_begin();
     stockham_body<T, L, MODE, SIGN>(in, out, p, W, Whi, Wlo, (int64_t)blockIdx.x, smem_raw);
 }
 
@@ -436,6 +437,7 @@ __global__ void __launch_bounds__(Stockham<T, L, MODE, SIGN>::NT, Stockham<T, L,
     typedef Stockham<T, L, MODE, SIGN> S;
     typedef typename V2<T>::t C2;
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    pdl_begin();
     C2 *stage0 = reinterpret_cast<C2 *>(smem_raw);
     C2 *stage1 = stage0 + S::STAGE;
     uint64_t *bar = reinterpret_cast<uint64_t *>(stage1 + S::STAGE);
@@ -652,6 +654,7 @@ __global__ void __launch_bounds__(Stockham<T, L, 0, SIGN>::NT, 1)
     constexpr int MP = S::BIG_MP;
     constexpr uint32_t PBYTES = (uint32_t)(MP * S::TL * sizeof(C2));
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    pdl_begin();
     C2 *xs = reinterpret_cast<C2 *>(smem_raw);
     C2 *pst = reinterpret_cast<C2 *>(smem_raw + S::BIG_X);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw + S::BIG_X + PBYTES);
@@ -733,7 +736,9 @@ template <typename T, int L> struct StockLaunch {
             }
         }
         const int64_t grid = std::min<int64_t>(ntiles, (int64_t)sms * per_sm);
-        kern<<<(unsigned)grid, S::NT, S::PIPE_SMEM, s>>>(in, out, p, tmap, W, Whi, Wlo, err);
+        // persistent blocks that each walk many tiles gain nothing from an early
+        // start (64 transforms of 2^20 took 867 us with it, 833 without)
+        pdl_launch_if(ntiles <= 4 * grid, kern, (unsigned)grid, S::NT, S::PIPE_SMEM, s, in, out, p, tmap, W, Whi, Wlo, err);
     }
     template <int MODE, int SIGN> static void one(const C2 *in, C2 *out, const StockParams &p, const CUtensorMap *tmap,
                                                   const C2 *W, const C2 *Whi, const C2 *Wlo, int *err, int sms,
@@ -749,7 +754,7 @@ template <typename T, int L> struct StockLaunch {
                 big_attr = true;
             }
             const int64_t grid = std::min<int64_t>(ntiles, (int64_t)sms);
-            kern<<<(unsigned)grid, S::NT, S::BIG_SMEM, s>>>(in, out, p, W, err);
+            pdl_launch_if(ntiles <= 4 * grid, kern, (unsigned)grid, S::NT, S::BIG_SMEM, s, in, out, p, W, err);
             return;
         }
         if constexpr (S::PIPE_OK) if (tmap) {
@@ -763,7 +768,7 @@ template <typename T, int L> struct StockLaunch {
             cudaFuncSetAttribute(stockham_kernel<T, L, MODE, SIGN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
             attr = true;
         }
-        stockham_kernel<T, L, MODE, SIGN><<<(unsigned)ntiles, S::NT, S::SMEM, s>>>(in, out, p, W, Whi, Wlo);
+        pdl_launch(stockham_kernel<T, L, MODE, SIGN>, (unsigned)ntiles, S::NT, S::SMEM, s, in, out, p, W, Whi, Wlo);
     }
     static void go(int mode, int sign, const C2 *in, C2 *out, const StockParams &p, const CUtensorMap *tmap, const C2 *W,
                    const C2 *Whi, const C2 *Wlo, int *err, int sms, cudaStream_t s) {
