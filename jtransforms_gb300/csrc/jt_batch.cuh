@@ -18,10 +18,13 @@
 #include "jt_stockham.cuh"
 #include "jt_r2r.cuh"
 #include "jt_chirp.cuh"
+#include "jt_bluemix.cuh"
+#include "jt_batchmix_params.cuh"
+#include "jt_fixmix.cuh"
 
 namespace jt {
 
-enum BOpType { BOP_TILE = 0, BOP_ELEM = 2, BOP_R2R = 3, BOP_BLUE = 4 };
+enum BOpType { BOP_TILE = 0, BOP_MIX = 1, BOP_ELEM = 2, BOP_R2R = 3, BOP_BLUE = 4, BOP_FIX = 5 };
 
 enum ElemKind {
     EK_COPY_COMPLEX = 0,
@@ -61,6 +64,8 @@ struct BOp {
         TileParams tp;
         R2rParams rp;   // DCT/DST/DHT and packed real lines in one step (kind: the R2rOp)
         BlueParams bp;  // a Bluestein transform in one step (W, Whi, Wlo: roots, bk1, bk2)
+        BatchMix mp;    // float lines and convolutions on register passes
+        FixMixParams fm;  // double lines (jt_fixmix.cuh)
     };
     const void *in;
     void *out;
@@ -78,166 +83,11 @@ struct BTask {
 // A batch CTA has 256 threads and at most JT_BATCH_SMEM_CAP bytes of shared
 // memory per task, so that three CTAs share an SM and their loads overlap one
 // another's arithmetic (lines whose tile would need more are recorded as two
-// passes of shorter lines).  Measured on the 10,000-transform workload: two
-// CTAs per SM (110 KB) 12.1 ms, three (72 KB, 80 registers) 9.4 ms, four
-// (54 KB, 64 registers, heavy spilling) 10.6 ms.
+// passes of shorter lines).  Each precision has a kernel and a queue of its
+// own: the double lines' fixed-point passes take 128 registers a thread (two
+// CTAs per SM), the float ones 80.
 #define JT_BATCH_THREADS 256
 #define JT_BATCH_ELEMS_PER_TASK (JT_BATCH_THREADS * 4)
 #define JT_BATCH_SMEM_CAP (72 * 1024)
-
-template <typename T> __device__ void elem_dispatch(const BOp &o, int64_t idx) {
-    typedef typename V2<T>::t C2;
-    const EArgs &e = o.e;
-    switch (o.kind) {
-        case EK_COPY_COMPLEX:
-            copy_complex_body<T>((const C2 *)e.p[0], e.i[0], (C2 *)e.p[1], e.i[1], e.i[2], e.i[3], (T)e.d[0], e.f, idx);
-            break;
-        case EK_BLUE_PRE:
-            if (o.sign < 0)
-                bluestein_pre_body<-1, T>((const C2 *)e.p[0], e.i[0], (C2 *)e.p[1], (const C2 *)e.p[2], e.i[1], e.i[2], e.i[3], idx);
-            else
-                bluestein_pre_body<1, T>((const C2 *)e.p[0], e.i[0], (C2 *)e.p[1], (const C2 *)e.p[2], e.i[1], e.i[2], e.i[3], idx);
-            break;
-        case EK_BLUE_MUL:
-            if (o.sign < 0) bluestein_mul_body<-1, T>((C2 *)e.p[0], (const C2 *)e.p[1], e.i[0], e.i[1], idx);
-            else bluestein_mul_body<1, T>((C2 *)e.p[0], (const C2 *)e.p[1], e.i[0], e.i[1], idx);
-            break;
-        case EK_BLUE_POST:
-            if (o.sign < 0)
-                bluestein_post_body<-1, T>((C2 *)e.p[0], e.i[0], (const C2 *)e.p[1], (const C2 *)e.p[2], e.i[1], e.i[2], e.i[3],
-                                           (T)e.d[0], idx);
-            else
-                bluestein_post_body<1, T>((C2 *)e.p[0], e.i[0], (const C2 *)e.p[1], (const C2 *)e.p[2], e.i[1], e.i[2], e.i[3],
-                                          (T)e.d[0], idx);
-            break;
-        case EK_REAL_POST_PACKED:
-            real_post_packed_body<T>((T *)e.p[0], e.i[0], e.i[1], e.i[2], (const C2 *)e.p[1], idx);
-            break;
-        case EK_REAL_POST_FULL:
-            if (o.sign < 0)
-                real_post_full_body<-1, T>((const T *)e.p[0], e.i[0], (T *)e.p[1], e.i[1], e.i[2], e.i[3], (const C2 *)e.p[2],
-                                           (T)e.d[0], idx);
-            else
-                real_post_full_body<1, T>((const T *)e.p[0], e.i[0], (T *)e.p[1], e.i[1], e.i[2], e.i[3], (const C2 *)e.p[2],
-                                          (T)e.d[0], idx);
-            break;
-        case EK_REAL_PRE_INV:
-            real_pre_inverse_body<T>((T *)e.p[0], e.i[0], e.i[1], e.i[2], (const C2 *)e.p[1], (T)e.d[0], idx);
-            break;
-        case EK_R2C: real_to_complex_body<T>((const T *)e.p[0], e.i[0], (C2 *)e.p[1], e.i[1], e.i[2], idx); break;
-        case EK_PACK_FULL: pack_from_full_body<T>((const C2 *)e.p[0], (T *)e.p[1], e.i[0], e.i[1], e.i[2], idx); break;
-        case EK_UNPACK_FULL: unpack_to_full_body<T>((const T *)e.p[0], e.i[0], (C2 *)e.p[1], e.i[1], e.i[2], idx); break;
-        case EK_REAL_PART: real_part_body<T>((const C2 *)e.p[0], (T *)e.p[1], e.i[0], e.i[1], e.i[2], (T)e.d[0], idx); break;
-        case EK_DCT2_PRE:
-            dct2_pre_body<T>((const T *)e.p[0], e.i[0], (T *)e.p[1], e.i[1], e.i[2], e.i[3], e.f, idx);
-            break;
-        case EK_DCT2_POST:
-            dct2_post_body<T>((const T *)e.p[0], e.i[0], (T *)e.p[1], e.i[1], e.i[2], e.i[3], (const C2 *)e.p[2], (T)e.d[0],
-                              (T)e.d[1], e.f, idx);
-            break;
-        case EK_DCT3_PRE:
-            dct3_pre_body<T>((const T *)e.p[0], e.i[0], (T *)e.p[1], e.i[1], e.i[2], e.i[3], (const C2 *)e.p[2], (T)e.d[0],
-                             (T)e.d[1], e.f, idx);
-            break;
-        case EK_DCT3_POST:
-            dct3_post_body<T>((const T *)e.p[0], e.i[0], (T *)e.p[1], e.i[1], e.i[2], e.i[3], e.f, idx);
-            break;
-        case EK_DHT_POST:
-            dht_post_body<T>((const T *)e.p[0], e.i[0], (T *)e.p[1], e.i[1], e.i[2], e.i[3], (T)e.d[0], idx);
-            break;
-        case EK_SCALE: scale_body<T>((T *)e.p[0], e.i[0], e.i[1], e.i[2], (T)e.d[0], idx); break;
-        case EK_COPY_REAL: copy_real_body<T>((const T *)e.p[0], e.i[0], (T *)e.p[1], e.i[1], e.i[2], e.i[3], idx); break;
-    }
-}
-
-template <typename T> __device__ void r2r_dispatch(const BOp &o, int idx, unsigned char *smem) {
-    typedef typename V2<T>::t C2;
-    const T *in = (const T *)o.in;
-    T *out = (T *)o.out;
-    const C2 *W = (const C2 *)o.W, *Wr = (const C2 *)o.Whi, *Wd = (const C2 *)o.Wlo;
-    if (o.kind == R2R_DCT2) r2r_tile_body<R2R_DCT2, T>(in, out, o.rp, W, Wr, Wd, idx, smem);
-    else if (o.kind == R2R_DCT3) r2r_tile_body<R2R_DCT3, T>(in, out, o.rp, W, Wr, Wd, idx, smem);
-    else if (o.kind == R2R_DHT) r2r_tile_body<R2R_DHT, T>(in, out, o.rp, W, Wr, Wd, idx, smem);
-    else if (o.kind == R2R_RFWD) r2r_tile_body<R2R_RFWD, T>(in, out, o.rp, W, Wr, Wd, idx, smem);
-    else r2r_tile_body<R2R_RINV, T>(in, out, o.rp, W, Wr, Wd, idx, smem);
-}
-
-__device__ __forceinline__ int ld_acquire_gpu(const int *p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// wait_polls: polls of a dependency wait (64 ns apart) before it gives up;
-// the library's default, 2^24, is about a second
-__global__ void __launch_bounds__(JT_BATCH_THREADS, 3)
-    batch_kernel(const BOp *__restrict__ ops, const BTask *__restrict__ tasks, int ntasks, int *head, int *done, int *err,
-                 int wait_polls) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_task;
-    __shared__ int s_ok;
-    const int tid = threadIdx.x;
-    for (;;) {
-        if (tid == 0) s_task = atomicAdd(head, 1);
-        __syncthreads();
-        const int ti = s_task;
-        if (ti >= ntasks) break;
-        const BTask tk = tasks[ti];
-        const BOp &o = ops[tk.op];
-        if (tid == 0) {
-            int ok = 1;
-            if (o.dep >= 0) {
-                const int need = ops[o.dep].ntasks;
-                int it = 0;
-                while (ld_acquire_gpu(&done[o.dep]) < need) {
-                    if (++it > wait_polls) {
-                        ok = 0;
-                        atomicExch(err, 1);
-                        break;
-                    }
-                    __nanosleep(64);
-                }
-            }
-            s_ok = ok;
-        }
-        __syncthreads();
-        if (s_ok) {
-            if (o.type == BOP_TILE) {
-                if (o.prec == 0) {
-                    if (o.sign < 0) tile_fft_body<-1, float>((const float2 *)o.in, (float2 *)o.out, o.tp, (const float2 *)o.W, (const float2 *)o.Whi, (const float2 *)o.Wlo, tk.idx, smem_raw);
-                    else tile_fft_body<1, float>((const float2 *)o.in, (float2 *)o.out, o.tp, (const float2 *)o.W, (const float2 *)o.Whi, (const float2 *)o.Wlo, tk.idx, smem_raw);
-                } else {
-                    if (o.sign < 0) tile_fft_body<-1, double>((const double2 *)o.in, (double2 *)o.out, o.tp, (const double2 *)o.W, (const double2 *)o.Whi, (const double2 *)o.Wlo, tk.idx, smem_raw);
-                    else tile_fft_body<1, double>((const double2 *)o.in, (double2 *)o.out, o.tp, (const double2 *)o.W, (const double2 *)o.Whi, (const double2 *)o.Wlo, tk.idx, smem_raw);
-                }
-            } else if (o.type == BOP_BLUE) {
-                if (o.prec == 0) {
-                    if (o.sign < 0) blue_tile_body<-1, float>((const float2 *)o.in, (float2 *)o.out, o.bp, (const float2 *)o.W, (const float2 *)o.Whi, (const float2 *)o.Wlo, tk.idx, smem_raw);
-                    else blue_tile_body<1, float>((const float2 *)o.in, (float2 *)o.out, o.bp, (const float2 *)o.W, (const float2 *)o.Whi, (const float2 *)o.Wlo, tk.idx, smem_raw);
-                } else {
-                    if (o.sign < 0) blue_tile_body<-1, double>((const double2 *)o.in, (double2 *)o.out, o.bp, (const double2 *)o.W, (const double2 *)o.Whi, (const double2 *)o.Wlo, tk.idx, smem_raw);
-                    else blue_tile_body<1, double>((const double2 *)o.in, (double2 *)o.out, o.bp, (const double2 *)o.W, (const double2 *)o.Whi, (const double2 *)o.Wlo, tk.idx, smem_raw);
-                }
-            } else if (o.type == BOP_R2R) {
-                if (o.prec == 0) r2r_dispatch<float>(o, tk.idx, smem_raw);
-                else r2r_dispatch<double>(o, tk.idx, smem_raw);
-            } else {
-                const int64_t base = (int64_t)tk.idx * JT_BATCH_ELEMS_PER_TASK;
-                for (int k = tid; k < JT_BATCH_ELEMS_PER_TASK; k += JT_BATCH_THREADS) {
-                    const int64_t idx = base + k;
-                    if (idx < o.total) {
-                        if (o.prec == 0) elem_dispatch<float>(o, idx);
-                        else elem_dispatch<double>(o, idx);
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            atomicAdd(&done[tk.op], 1);
-        }
-    }
-}
 
 }  // namespace jt

@@ -197,6 +197,11 @@ void fixmix_setup(int smem_optin);
 void fixmix_table(int4 *out, const MixParams &p, int count, cudaStream_t s);
 void fixmix_launch(const double2 *in, double2 *out, const FixMixParams &p, unsigned grid, int threads, size_t smem, cudaStream_t s);
 
+// The batch kernel (jt_batch.cu).
+cudaError_t batch_setup(int prec, int smem, int *per_sm);
+void batch_launch(int prec, const BOp *ops, const BTask *tasks, int ntasks, int *head, int *done, int *err, int wait_polls, int grid,
+                  int smem, cudaStream_t s);
+
 // Float Bluestein lines (jt_bluemix.cu).
 void blue_setup(int smem_optin);
 void blue_mid(bool one, const float2 *in, float2 *out, const BlueMid &q, unsigned grid, int threads, size_t smem, cudaStream_t s);
@@ -642,9 +647,8 @@ template <typename T> struct Fft1 {
     int init_direct() {
         algo = ALG_DIRECT;
         JT_TRY(set_reg(reg_ok(n)));
-        if (reg) return make_roots(&W, n, 1, n, sizeof(T) == 8);
-        radix = direct_radices(n, radix_order(n, sizeof(T) == 4));
-        if constexpr (sizeof(T) == 4) {
+        if (!reg) radix = direct_radices(n, radix_order(n, sizeof(T) == 4));
+        if constexpr (sizeof(T) == 4) {  // (power-of-two lines run it in batches)
             const std::vector<int> R = mix_radices(n);
             const int count = R.empty() ? 0 : mix_plan((int)n, R, &mix);
             JT_TRY(make_roots(&W, n, 1, n, false, count + 1));
@@ -679,29 +683,15 @@ template <typename T> struct Fft1 {
         }
     }
 
-    // Line pass of the doubles' mixed-radix kernel.  C lines per CTA: a first
-    // pass of 256 butterflies for rows, 512 for strided lines (up to 8: 128-byte
-    // runs), fewer (down to 2 columns) while the grid has fewer CTAs than two
-    // per SM.
-    int exec_fixmix(Ctx &ctx, const C2 *in, C2 *out, int64_t nlines, const Layout &lin, const Layout &lout, int sign, double scale,
-                    int64_t tw_n, int64_t tw_inner, const C2 *Whi_, const C2 *Wlo_, int tw_lo_bits) const {
-        FixMixParams p;
+    // What a fixmix step needs but its lines per CTA.
+    void fill_fixmix(FixMixParams &p, int64_t nlines, const Layout &lin, const Layout &lout, int sign, double scale, int64_t tw_n,
+                     int64_t tw_inner, const C2 *Whi_, const C2 *Wlo_, int tw_lo_bits) const {
         memset(&p, 0, sizeof(p));
         p.m = mix;
         p.psh = psh;
         p.cols_in = lin.estride != 1;
         p.cols_out = lout.estride != 1;
         p.inv = sign > 0;
-        const bool strided = p.cols_in || p.cols_out;
-        const int nb = (int)n / mix.R[0];
-        const size_t per_line = (size_t)mix.Lp * sizeof(C2) * (mix.npass > 2 ? 2 : 1) + tile_words<T>();
-        int C = std::max(1, (strided ? JT_FIXMIX_THREADS : 256) / nb);
-        if (strided) C = std::min(C, std::max(8, 128 / nb));
-        C = std::min(C, (int)std::max<size_t>(1, (size_t)g_smem_optin / per_line));
-        while (C > (strided ? 2 : 1) && C * nb > 32 && cdiv(nlines, C) < 2 * (int64_t)g_sms) C /= 2;
-        if ((int64_t)C > nlines) C = (int)nlines;
-        p.m.C = C;
-        p.m.mC = C > 1 ? (uint32_t)(((uint64_t)1 << 32) / (uint64_t)C + 1) : 0;
         p.m.nlines = nlines;
         p.m.lin = lin;
         p.m.lout = lout;
@@ -718,8 +708,9 @@ template <typename T> struct Fft1 {
         p.Whiq = (const int4 *)(Whi_ ? Whi_ + nhi : nullptr);
         p.Wloq = (const int4 *)(Wlo_ ? Wlo_ + nlo : nullptr);
         p.fp.L = (int)n;
-        p.fp.npass = (int)radix.size();
-        for (int i = 0; i < p.fp.npass; i++) p.fp.radix[i] = radix[i];
+        const std::vector<int> rr = radix.empty() ? direct_radices(n) : radix;
+        p.fp.npass = (int)rr.size();
+        for (int i = 0; i < p.fp.npass; i++) p.fp.radix[i] = rr[i];
         p.fp.C = 1;
         p.fp.nlines = nlines;
         p.fp.lin = lin;
@@ -732,11 +723,37 @@ template <typename T> struct Fft1 {
         p.W = W;
         p.Whi = Whi_;
         p.Wlo = Wlo_;
+    }
+    static void set_fixmix_lines(FixMixParams &p, int C) {
+        p.m.C = C;
+        p.m.mC = C > 1 ? (uint32_t)(((uint64_t)1 << 32) / (uint64_t)C + 1) : 0;
+    }
+    // shared memory of C lines: their buffers and words, or one line's FP64 tile
+    size_t fixmix_smem(int C) const {
+        return std::max(((size_t)mix.Lp * sizeof(C2) * (mix.npass > 2 ? 2 : 1) + tile_words<T>()) * C, 2 * (size_t)padded_len((int)n) * sizeof(C2));
+    }
+
+    // Line pass of the doubles' mixed-radix kernel.  C lines per CTA: a first
+    // pass of 256 butterflies for rows, 512 for strided lines (up to 8: 128-byte
+    // runs), fewer (down to 2 columns) while the grid has fewer CTAs than two
+    // per SM.
+    int exec_fixmix(Ctx &ctx, const C2 *in, C2 *out, int64_t nlines, const Layout &lin, const Layout &lout, int sign, double scale,
+                    int64_t tw_n, int64_t tw_inner, const C2 *Whi_, const C2 *Wlo_, int tw_lo_bits) const {
+        FixMixParams p;
+        fill_fixmix(p, nlines, lin, lout, sign, scale, tw_n, tw_inner, Whi_, Wlo_, tw_lo_bits);
+        const bool strided = p.cols_in || p.cols_out;
+        const int nb = (int)n / mix.R[0];
+        const size_t per_line = (size_t)mix.Lp * sizeof(C2) * (mix.npass > 2 ? 2 : 1) + tile_words<T>();
+        int C = std::max(1, (strided ? JT_FIXMIX_THREADS : 256) / nb);
+        if (strided) C = std::min(C, std::max(8, 128 / nb));
+        C = std::min(C, (int)std::max<size_t>(1, (size_t)g_smem_optin / per_line));
+        while (C > (strided ? 2 : 1) && C * nb > 32 && cdiv(nlines, C) < 2 * (int64_t)g_sms) C /= 2;
+        if ((int64_t)C > nlines) C = (int)nlines;
+        set_fixmix_lines(p, C);
         if (ctx.dry) return JT_OK;
         const int64_t grid = cdiv(nlines, C);
         if (grid > 0x7fffffff) return JT_ETOOBIG;
-        const size_t smem = std::max(per_line * C, 2 * (size_t)padded_len((int)n) * sizeof(C2));
-        fixmix_launch(in, out, p, (unsigned)grid, (int)cdiv(C * nb, 32) * 32, smem, ctx.s);
+        fixmix_launch(in, out, p, (unsigned)grid, (int)cdiv(C * nb, 32) * 32, fixmix_smem(C), ctx.s);
         g_launches++;
         return JT_OK;
     }
@@ -1069,6 +1086,70 @@ template <typename T> struct Fft1 {
         return JT_OK;
     }
 
+    // Lines per task of a register-pass step: about 2048 numbers, at least 16
+    // columns where the cap allows them.
+    static int batch_mix_lines(const MixParams &p, bool strided, int64_t nlines) {
+        int C = std::max(strided ? 16 : 1, 2048 / p.L);
+        C = std::min(C, (int)((size_t)JT_BATCH_SMEM_CAP / (2 * (size_t)p.Lp * sizeof(C2))));
+        return (int)std::max<int64_t>(1, std::min<int64_t>(C, nlines));
+    }
+    static void set_batch_mix(MixParams &p, int C, int64_t nlines) {
+        p.C = C;
+        p.mC = C > 1 ? (uint32_t)(((uint64_t)1 << 32) / (uint64_t)C + 1) : 0;
+        p.nlines = nlines;
+    }
+    // Bluestein in a batch (one transform): the kernels of exec_blue as steps.
+    bool record_blue_ok() const {
+        return bn1 > 0 && bf.npass > 1 &&
+               2 * (size_t)bf.Lp * sizeof(C2) <= (size_t)JT_BATCH_SMEM_CAP;
+    }
+    int record_blue(Ctx &ctx, const C2 *in, C2 *out, int64_t batch, int64_t din, int64_t dout, int sign, double scale) const {
+        const int64_t N = (int64_t)bn1 * bn2;
+        C2 *tmp = bn1 > 1 ? (C2 *)ctx.ws->get(sizeof(C2) * batch * N, !ctx.rec) : nullptr;
+        if (!ctx.rec) return JT_OK;
+        auto step = [&](const MixParams &p, bool cols, int64_t lines, const C2 *src, C2 *dst) {
+            BOp o;
+            memset(&o, 0, sizeof(o));
+            o.type = BOP_MIX;
+            o.in = src;
+            o.out = dst;
+            BatchMix &q = o.mp;
+            q.f = p;
+            q.twf = btab;
+            q.n1 = bn1;
+            q.cols_in = q.cols_out = cols;
+            q.bl = MixBlue{(int)n, bn2, sign > 0, din, dout, (float)scale, bk1, btab + btw};
+            const int C = batch_mix_lines(p, cols, lines);
+            set_batch_mix(q.f, C, lines);
+            q.f.lin = q.f.lout = cols ? Layout{bn2, N, 1, bn2} : Layout{1, bn2, 0, 1};
+            o.ntasks = (int)cdiv(lines, C);
+            o.smem = (int)(2 * (size_t)p.Lp * sizeof(C2) * C);
+            return o;
+        };
+        if (bn1 > 1) {
+            BOp o = step(bcol, true, batch * bn2, in, tmp);
+            o.mp.chirp_in = 2;
+            emit(ctx, o);
+        }
+        BOp o = step(bf, false, batch * bn1, bn1 > 1 ? tmp : in, bn1 > 1 ? tmp : out);
+        o.mp.turn = 1;
+        o.mp.twf = btab + boff_f;
+        o.mp.g = bg;
+        set_batch_mix(o.mp.g, o.mp.f.C, batch * bn1);
+        o.mp.g.lin = o.mp.g.lout = o.mp.f.lin;
+        o.mp.twg = btab + boff_g;
+        o.mp.Bp = bspec;
+        o.mp.chirp_in = o.mp.chirp_out = bn1 == 1;
+        emit(ctx, o);
+        if (bn1 > 1) {
+            BOp e = step(bcol, true, batch * bn2, tmp, out);
+            e.mp.inv = 1;
+            e.mp.chirp_out = 2;
+            emit(ctx, e);
+        }
+        return JT_OK;
+    }
+
     // Batch recording of a line pass: the generic tile kernel (any layout,
     // lengths up to the tile kernel's limit; longer one-pass lengths are
     // recorded through their two-pass alternate, make_rec_alt).
@@ -1083,6 +1164,45 @@ template <typename T> struct Fft1 {
         o.W = W;
         o.Whi = Whi_;
         o.Wlo = Wlo_;
+        if constexpr (sizeof(T) == 4) {
+            if (mix.npass > 1 && 2 * (size_t)mix.Lp * sizeof(C2) <= (size_t)JT_BATCH_SMEM_CAP) {
+                o.type = BOP_MIX;
+                BatchMix &q = o.mp;
+                q.f = mix;
+                q.twf = Wm;
+                q.n1 = 1;
+                q.cols_in = lin.estride != 1;
+                q.cols_out = lout.estride != 1;
+                q.inv = sign > 0;
+                const int C = batch_mix_lines(mix, q.cols_in || q.cols_out, nlines);
+                set_batch_mix(q.f, C, nlines);
+                q.f.lin = lin;
+                q.f.lout = lout;
+                q.f.scale = (float)scale;
+                q.f.do_scale = scale != 1.0;
+                q.f.tw_n = tw_n;
+                q.f.tw_inner = tw_inner;
+                q.f.tw_lo_bits = tw_lo_bits;
+                o.ntasks = (int)cdiv(nlines, C);
+                o.smem = (int)(2 * (size_t)mix.Lp * sizeof(C2) * C);
+                emit(ctx, o);
+                return JT_OK;
+            }
+        } else {
+            const int nb = mix.npass ? (int)n / mix.R[0] : 0;
+            if (nb && nb <= JT_BATCH_THREADS && fixmix_smem(1) <= (size_t)JT_BATCH_SMEM_CAP) {
+                o.type = BOP_FIX;
+                fill_fixmix(o.fm, nlines, lin, lout, sign, scale, tw_n, tw_inner, Whi_, Wlo_, tw_lo_bits);
+                int C = JT_BATCH_THREADS / nb;  // the first pass: one butterfly per thread
+                while (C > 1 && fixmix_smem(C) > (size_t)JT_BATCH_SMEM_CAP) C--;
+                C = (int)std::min<int64_t>(C, nlines);
+                set_fixmix_lines(o.fm, C);
+                o.ntasks = (int)cdiv(nlines, C);
+                o.smem = (int)fixmix_smem(C);
+                emit(ctx, o);
+                return JT_OK;
+            }
+        }
         if (generic_ok(n)) {
             const int L = (int)n;
             const bool strided = lin.estride != 1 || lout.estride != 1;
@@ -1300,6 +1420,10 @@ template <typename T> struct Fft1 {
                 return JT_OK;
             }
             case ALG_BLUESTEIN: {
+                if constexpr (sizeof(T) == 4) {
+                    if ((ctx.rec || ctx.rec_sizing) && record_blue_ok())
+                        return record_blue(ctx, in, out, batch, din, dout, sign, scale);
+                }
                 if ((ctx.rec || ctx.rec_sizing) && rec_alt) return rec_alt->exec(ctx, in, din, out, dout, batch, sign, scale);
                 if constexpr (sizeof(T) == 4) {
                     if (bn1 && !ctx.rec && !ctx.rec_sizing) return exec_blue(ctx, in, din, out, dout, batch, sign, scale);
@@ -2850,11 +2974,16 @@ struct jt_batch {
     std::vector<int> ops, scales;
     std::vector<void *> ptrs;
     // recorded steps, on the device
-    int nops = 0, ntasks = 0, smem = 0, grid = 0;
+    int nops = 0;
+    // a queue for each precision: its tasks follow one another in d_tasks
+    int ntasks[2] = {0, 0}, smem[2] = {0, 0}, grid[2] = {0, 0};
     BOp *d_ops = nullptr;
     BTask *d_tasks = nullptr;
     int *d_done = nullptr;  // completed tasks per step
-    int *d_head = nullptr;  // queue head
+    int *d_head = nullptr;  // queue heads
+    // the double queue's kernel runs beside the float one's
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     char *scratch = nullptr;    // float transforms' scratch
     char *scratch_d = nullptr;  // double transforms' scratch
     cudaGraphExec_t graph = nullptr;
@@ -2862,6 +2991,9 @@ struct jt_batch {
     int wait_polls = 1 << 24;  // polls of a dependency wait before it gives up
     ~jt_batch() {
         if (graph) cudaGraphExecDestroy(graph);
+        if (side) cudaStreamDestroy(side);
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
         for (void *p : {(void *)d_ops, (void *)d_tasks, (void *)d_done, (void *)d_head, (void *)scratch, (void *)scratch_d})
             if (p) cudaFree(p);
     }
@@ -2960,45 +3092,64 @@ int jt_batch_create(int count, jt_plan *const *plans, const int *ops, void *cons
     std::vector<BTask> tasks;
     size_t maxlen = 0;
     for (auto &c : chains) maxlen = std::max(maxlen, c.size());
-    int smem = 0;
-    for (size_t s = 0; s < maxlen; s++)
-        for (auto &c : chains)
-            if (s < c.size()) {
-                const BOp &o = rec[c[s]];
-                smem = std::max(smem, o.smem);
-                for (int k = 0; k < o.ntasks; k++) tasks.push_back(BTask{c[s], k});
-            }
+    for (int prec = 0; prec < 2; prec++) {
+        const size_t before = tasks.size();
+        for (size_t s = 0; s < maxlen; s++)
+            for (auto &c : chains)
+                if (s < c.size() && rec[c[s]].prec == prec) {
+                    const BOp &o = rec[c[s]];
+                    b->smem[prec] = std::max(b->smem[prec], std::max(o.smem, 1));
+                    for (int k = 0; k < o.ntasks; k++) tasks.push_back(BTask{c[s], k});
+                }
+        b->ntasks[prec] = (int)(tasks.size() - before);
+        if (!b->ntasks[prec]) continue;
+        int per_sm = 0;
+        JT_CU(batch_setup(prec, b->smem[prec], &per_sm));
+        b->grid[prec] = std::max(1, per_sm) * g_sms;
+    }
     b->nops = (int)rec.size();
-    b->ntasks = (int)tasks.size();
-    b->smem = smem;
     if (b->nops) {
         JT_CU(cudaMalloc(&b->d_ops, sizeof(BOp) * rec.size()));
         JT_CU(cudaMemcpy(b->d_ops, rec.data(), sizeof(BOp) * rec.size(), cudaMemcpyHostToDevice));
         JT_CU(cudaMalloc(&b->d_done, sizeof(int) * rec.size()));
     }
-    if (b->ntasks) {
+    if (!tasks.empty()) {
         JT_CU(cudaMalloc(&b->d_tasks, sizeof(BTask) * tasks.size()));
         JT_CU(cudaMemcpy(b->d_tasks, tasks.data(), sizeof(BTask) * tasks.size(), cudaMemcpyHostToDevice));
     }
-    JT_CU(cudaMalloc(&b->d_head, sizeof(int)));
-    JT_CU(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(smem, 1)));
-    JT_CU(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    int per_sm = 0;
-    JT_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, JT_BATCH_THREADS, std::max(smem, 1)));
-    b->grid = std::max(1, per_sm) * g_sms;
+    JT_CU(cudaMalloc(&b->d_head, 2 * sizeof(int)));
+    if (b->ntasks[0] && b->ntasks[1]) {
+        JT_CU(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
+        JT_CU(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+        JT_CU(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
+    }
     *out = b.release();
     return JT_OK;
 }
 
 int jt_batch_run(jt_batch *b, void *stream) {
     if (!b) return JT_EINVAL;
-    if (!b->ntasks) return JT_OK;
+    if (!b->ntasks[0] && !b->ntasks[1]) return JT_OK;
     cudaStream_t s = (cudaStream_t)stream;
     JT_CU(cudaMemsetAsync(b->d_done, 0, sizeof(int) * b->nops, s));
-    JT_CU(cudaMemsetAsync(b->d_head, 0, sizeof(int), s));
-    batch_kernel<<<b->grid, JT_BATCH_THREADS, std::max(b->smem, 1), s>>>(b->d_ops, b->d_tasks, b->ntasks, b->d_head, b->d_done,
-                                                                          g_err_dev, b->wait_polls);
-    g_launches++;
+    JT_CU(cudaMemsetAsync(b->d_head, 0, 2 * sizeof(int), s));
+    // the double queue takes longer: its kernel first, the float one fills in
+    cudaStream_t ds = s;
+    if (b->side) {
+        ds = b->side;
+        JT_CU(cudaEventRecord(b->fork, s));
+        JT_CU(cudaStreamWaitEvent(ds, b->fork, 0));
+    }
+    for (int prec = 1; prec >= 0; prec--) {
+        if (!b->ntasks[prec]) continue;
+        batch_launch(prec, b->d_ops, b->d_tasks + (prec ? b->ntasks[0] : 0), b->ntasks[prec], b->d_head + prec, b->d_done, g_err_dev,
+                     b->wait_polls, b->grid[prec], b->smem[prec], prec ? ds : s);
+        g_launches++;
+    }
+    if (b->side) {
+        JT_CU(cudaEventRecord(b->join, ds));
+        JT_CU(cudaStreamWaitEvent(s, b->join, 0));
+    }
     JT_CU(cudaGetLastError());
     return JT_OK;
 }

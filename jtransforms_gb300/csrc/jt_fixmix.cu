@@ -3,23 +3,10 @@
 
 namespace jt {
 
-__device__ __noinline__ void fixmix_fp64(const double2 *in, double2 *out, const FixMixParams &p, int64_t b0, int lines,
-                                                unsigned char *smem) {
-    for (int l = 0; l < lines; l++) {
-        __syncthreads();
-        if (p.inv) tile_fft_body<1, double, true>(in, out, p.fp, p.W, p.Whi, p.Wlo, b0 + l, smem);
-        else tile_fft_body<-1, double, true>(in, out, p.fp, p.W, p.Whi, p.Wlo, b0 + l, smem);
-    }
-}
-
 __global__ void __launch_bounds__(JT_FIXMIX_THREADS, 1) fixmix_kernel(const double2 *in, double2 *out, FixMixParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     pdl_begin();
-    const int64_t b0 = (int64_t)blockIdx.x * p.m.C;
-    const int lines = (int)min((int64_t)p.m.C, p.m.nlines - b0), nbuf = p.m.npass > 2 ? 2 : 1;
-    Fx *A = reinterpret_cast<Fx *>(smem_raw);
-    uint32_t *words = reinterpret_cast<uint32_t *>(A + nbuf * p.m.C * p.m.Lp);
-    if (!FixMixTile{in, out, p, b0, lines, words}.run(A, A + p.m.C * p.m.Lp)) fixmix_fp64(in, out, p, b0, lines, smem_raw);
+    fixmix_body(in, out, p, (int64_t)blockIdx.x, smem_raw);
 }
 
 // Pass P >= 1: factor k (1..R-1) as Ns entries w_{Ns R}^{jm k} from toff[P] on.

@@ -271,4 +271,22 @@ struct FixMixTile {
     }
 };
 
+static __device__ __noinline__ void fixmix_fp64(const double2 *in, double2 *out, const FixMixParams &p, int64_t b0, int lines,
+                                                unsigned char *smem) {
+    for (int l = 0; l < lines; l++) {
+        __syncthreads();
+        if (p.inv) tile_fft_body<1, double, true>(in, out, p.fp, p.W, p.Whi, p.Wlo, b0 + l, smem);
+        else tile_fft_body<-1, double, true>(in, out, p.fp, p.W, p.Whi, p.Wlo, b0 + l, smem);
+    }
+}
+
+// Tile `blk`, at smem_raw: one or two buffers of C lines and their words.
+__device__ __forceinline__ void fixmix_body(const double2 *in, double2 *out, const FixMixParams &p, int64_t blk, unsigned char *smem_raw) {
+    const int64_t b0 = blk * p.m.C;
+    const int lines = (int)min((int64_t)p.m.C, p.m.nlines - b0), nbuf = p.m.npass > 2 ? 2 : 1;
+    Fx *A = reinterpret_cast<Fx *>(smem_raw);
+    uint32_t *words = reinterpret_cast<uint32_t *>(A + nbuf * p.m.C * p.m.Lp);
+    if (!FixMixTile{in, out, p, b0, lines, words}.run(A, A + p.m.C * p.m.Lp)) fixmix_fp64(in, out, p, b0, lines, smem_raw);
+}
+
 }  // namespace jt
