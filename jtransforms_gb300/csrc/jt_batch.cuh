@@ -87,7 +87,7 @@ struct BTask {
 // own: the double lines' fixed-point passes take 128 registers a thread (two
 // CTAs per SM), the float ones 80.
 #define JT_BATCH_THREADS 256
-#define JT_BATCH_ELEMS_PER_TASK (JT_BATCH_THREADS * 4)
+#define JT_BATCH_ELEMS_PER_TASK (JT_BATCH_THREADS * 8)
 #define JT_BATCH_SMEM_CAP (72 * 1024)
 
 }  // namespace jt

@@ -37,6 +37,7 @@
 #include <memory>
 #include <mutex>
 #include <new>
+#include <queue>
 #include <string>
 #include <tuple>
 #include <thread>
@@ -3052,6 +3053,75 @@ int batch_record(jt_batch *bt, std::vector<BOp> &ops, std::vector<std::vector<in
     return JT_OK;
 }
 
+// Time of one task of a step, in the units of a small one: fixed costs (claim,
+// wait, first loads) and passes over its numbers.
+double batch_task_cost(const BOp &o) {
+    double points = 0, passes = 1;
+    switch (o.type) {
+        case BOP_TILE: points = (double)o.tp.C * o.tp.L; passes = o.tp.npass + 1; break;
+        case BOP_MIX: points = (double)o.mp.f.C * o.mp.f.L; passes = o.mp.f.npass * (o.mp.turn ? 2 : 1); break;
+        case BOP_FIX: points = (double)o.fm.m.C * o.fm.m.L; passes = 2.0 * o.fm.m.npass; break;
+        case BOP_R2R: points = (double)o.rp.C * o.rp.n / 2; passes = o.rp.npass + 3; break;
+        case BOP_BLUE: points = (double)o.bp.C * o.bp.nB; passes = 2.0 * o.bp.npass + 3; break;
+        default: points = JT_BATCH_ELEMS_PER_TASK; break;
+    }
+    return 1.0 + points * passes / 3000.0 * (o.prec == 1 ? 1.5 : 1.0);
+}
+
+// Appends the tasks of the chains' steps in the order in which `workers` CTAs
+// would start them if a free one always took the ready step with the longest
+// rest of its chain.  (Steps after steps, each stage of all transforms before
+// the next, left the long chains to run by themselves at the end.)  A step's
+// tasks come after all tasks of the step it waits for, so the kernel's waits end.
+void batch_order(const std::vector<BOp> &rec, const std::vector<std::vector<int>> &chains, int workers, std::vector<BTask> &tasks) {
+    struct Ready {
+        double rest;
+        int chain, step, next;
+        bool operator<(const Ready &r) const { return rest < r.rest; }
+    };
+    std::vector<std::vector<double>> rest(chains.size());
+    std::priority_queue<Ready> ready;
+    for (size_t c = 0; c < chains.size(); c++) {
+        rest[c].resize(chains[c].size());
+        double r = 0;
+        for (int s = (int)chains[c].size() - 1; s >= 0; s--) {
+            const BOp &o = rec[chains[c][s]];
+            r += batch_task_cost(o) * (1.0 + o.ntasks / (double)workers);
+            rest[c][s] = r;
+        }
+        if (!chains[c].empty()) ready.push(Ready{rest[c][0], (int)c, 0, 0});
+    }
+    typedef std::pair<double, int> Event;  // time, worker's chain (-1: none yet)
+    std::priority_queue<Event, std::vector<Event>, std::greater<Event>> busy;
+    std::vector<int> left(chains.size(), 0), at(chains.size(), 0);
+    int idle = workers;
+    double now = 0;
+    for (;;) {
+        while (idle > 0 && !ready.empty()) {
+            const Ready r = ready.top();
+            ready.pop();
+            const BOp &o = rec[chains[r.chain][r.step]];
+            if (r.next == 0) left[r.chain] = o.ntasks;
+            const double end = now + batch_task_cost(o);
+            const int k = std::min(idle, o.ntasks - r.next);
+            for (int i = 0; i < k; i++) {
+                tasks.push_back(BTask{chains[r.chain][r.step], r.next + i});
+                busy.push(Event(end, r.chain));
+            }
+            idle -= k;
+            if (r.next + k < o.ntasks) ready.push(Ready{r.rest, r.chain, r.step, r.next + k});
+        }
+        if (busy.empty()) break;
+        now = busy.top().first;
+        while (!busy.empty() && busy.top().first <= now) {
+            const int c = busy.top().second;
+            busy.pop();
+            idle++;
+            if (--left[c] == 0 && ++at[c] < (int)chains[c].size()) ready.push(Ready{rest[c][at[c]], c, at[c], 0});
+        }
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -3088,24 +3158,22 @@ int jt_batch_create(int count, jt_plan *const *plans, const int *ops, void *cons
         for (auto &c : chains)
             if (!c.empty()) rec[c[0]].dep = phantom;
     }
-    // tasks, stage by stage: every transform's first step, then the second...
+    // the queues, each in the order of a schedule with as many workers as the
+    // kernel has CTAs
     std::vector<BTask> tasks;
-    size_t maxlen = 0;
-    for (auto &c : chains) maxlen = std::max(maxlen, c.size());
     for (int prec = 0; prec < 2; prec++) {
         const size_t before = tasks.size();
-        for (size_t s = 0; s < maxlen; s++)
-            for (auto &c : chains)
-                if (s < c.size() && rec[c[s]].prec == prec) {
-                    const BOp &o = rec[c[s]];
-                    b->smem[prec] = std::max(b->smem[prec], std::max(o.smem, 1));
-                    for (int k = 0; k < o.ntasks; k++) tasks.push_back(BTask{c[s], k});
-                }
-        b->ntasks[prec] = (int)(tasks.size() - before);
-        if (!b->ntasks[prec]) continue;
+        std::vector<std::vector<int>> mine;
+        for (auto &c : chains)
+            if (!c.empty() && rec[c[0]].prec == prec) mine.push_back(c);
+        for (auto &c : mine)
+            for (int o : c) b->smem[prec] = std::max(b->smem[prec], std::max(rec[o].smem, 1));
+        if (mine.empty()) continue;
         int per_sm = 0;
         JT_CU(batch_setup(prec, b->smem[prec], &per_sm));
         b->grid[prec] = std::max(1, per_sm) * g_sms;
+        batch_order(rec, mine, b->grid[prec], tasks);
+        b->ntasks[prec] = (int)(tasks.size() - before);
     }
     b->nops = (int)rec.size();
     if (b->nops) {
