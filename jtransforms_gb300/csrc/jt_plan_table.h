@@ -14,8 +14,8 @@ static const signed char kSplitF32[31][3] = {
 
 static const signed char kSplitF64[31][3] = {
     {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1},
-    {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {7, 7, 0}, {8, 7, 0},
-    {8, 8, 0}, {11, 6, 0}, {11, 7, 0}, {11, 8, 0}, {11, 9, 0}, {11, 10, 0}, {11, 11, 0}, {12, 11, 0},
+    {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {8, 6, 0}, {6, 9, 0},
+    {6, 10, 0}, {6, 11, 0}, {8, 10, 0}, {9, 10, 0}, {10, 10, 0}, {10, 11, 0}, {11, 11, 0}, {8, 8, 7},
     {8, 8, 8}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1},
 };
 
