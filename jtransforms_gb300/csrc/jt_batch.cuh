@@ -1,15 +1,15 @@
-// jt_batch.cuh -- one persistent launch for a batch of transforms of mixed
-// sizes and kinds.
+// jt_batch.cuh -- one persistent launch per precision for a batch of
+// transforms of mixed sizes and kinds.
 //
-// The host records each transform as the chain of steps the single-transform
-// path would launch (generic tile FFT passes and elementwise pre/post steps),
-// into a table of ops.  Each op is split into tasks of one CTA's work; the
-// task queue holds every transform's first step, then every second step, and
-// so on.  batch_kernel's CTAs pull tasks with an atomic counter, wait
-// (bounded) until the task's previous step in the same transform has
-// finished, run it and count it done.  Because a step's tasks are all queued
-// before any task of the next step, every awaited task is already held by a
-// running CTA and the waits end.  Producer CTAs publish with a gpu-scope
+// The host records each transform as a chain of steps (line passes of
+// jt_batchmix.cuh, jt_fixmix.cuh and jt_device.cuh, one-step real, DCT and
+// Bluestein lines, elementwise pre/post steps) into a table of ops.  Each op
+// is split into tasks of one CTA's work; the queue holds them in the order of
+// a schedule made beforehand.  batch_kernel's CTAs pull tasks with an atomic
+// counter, wait (bounded) until the task's previous step in the same transform
+// has finished, run it and count it done.  Because a step's tasks are all
+// queued before any task of the next step, every awaited task is already held
+// by a running CTA and the waits end.  Producer CTAs publish with a gpu-scope
 // fence before the counter update; consumers read the counter with acquire
 // semantics before their threads touch the data.
 #pragma once

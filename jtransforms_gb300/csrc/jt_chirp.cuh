@@ -1,12 +1,12 @@
-// jt_chirp.cuh -- Bluestein (chirp-z) transforms in one CTA tile.
+// jt_chirp.cuh -- Bluestein (chirp-z) transforms as one batch step.
 //
-// For a length n whose padded length nB = nextPow2(2n - 1) fits a tile (the
-// tile kernel's limit), a CTA runs the whole chirp-z transform of C lines in
-// shared memory: the chirp premultiply and zero pad on the load, the nB-point
-// forward FFT, the multiply by the transformed chirp, the nB-point inverse
-// FFT, and the chirp postmultiply (times the scale) on the store.  The
-// chirp tables are the FP64-built bk1 (n) and bk2 (nB) of the plan, the
-// same ones the separate pre/mul/post kernels of jt_device.cuh use.
+// For a length n whose convolution of nB >= 2n - 1 points fits a batch task, a
+// CTA runs the whole chirp-z transform of C lines in shared memory: the chirp
+// premultiply and zero pad on the load, the nB-point forward FFT, the multiply
+// by the transformed chirp, the nB-point inverse FFT, and the chirp
+// postmultiply (times the scale) on the store.  The chirp tables are the
+// FP64-built bk1 (n) and bk2 (nB) of the plan, the same ones the separate
+// pre/mul/post kernels of jt_device.cuh use.
 // Reference: fft/DoubleFFT_1D.java:1864-1890 (bluesteini), :1920-2107
 // (bluestein_complex).
 #pragma once
@@ -71,14 +71,6 @@ __device__ void blue_tile_body(const C2 *in, C2 *out, const BlueParams &p, const
         if (sc != (T)1) v = cscale<T>(v, sc);
         out[line_off(p.lout, b0 + c) + (int64_t)i * p.lout.estride] = v;
     }
-}
-
-template <int SIGN, typename T>
-__global__ void __launch_bounds__(512) blue_tile_kernel(const C2 *in, C2 *out, BlueParams p, const C2 *__restrict__ W,
-                                                        const C2 *__restrict__ bk1, const C2 *__restrict__ bk2) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    pdl_begin();
-    blue_tile_body<SIGN, T>(in, out, p, W, bk1, bk2, (int64_t)blockIdx.x, smem_raw);
 }
 
 #undef C2

@@ -3,18 +3,20 @@
 //
 // Algorithm choice per complex length n (GPU-first, not the reference's
 // split-radix / FFTPACK / Bluestein choice, which only fixes the results):
-//   DIRECT    n <= 8192 (f32) / 4096 (f64) with prime factors <= 63: one
-//             shared-memory tile kernel per batch of lines; powers of two in
-//             registers, floats in FP32 (jt_stockham.cuh), doubles in 64-bit
-//             fixed point (jt_fix64.cuh).
+//   DIRECT    n <= 8192 (f32) / 4096 (f64) with prime factors <= 63, one kernel
+//             per batch of lines: powers of two in registers, floats in FP32
+//             (jt_stockham.cuh), doubles in 64-bit fixed point (jt_fix64.cuh);
+//             small prime factors in few register passes (jt_mixed.cuh,
+//             jt_fixmix.cuh); the rest in shared-memory tile passes.
 //   TWOPASS   n = n1 * n2 with both DIRECT: column pass with the four-step
 //             twiddle fused into its store, then a row pass that writes the
 //             transposed (natural-order) result.  The batch is processed in
 //             chunks of up to 1 GiB: one launch per pass and chunk (long
 //             launches measured faster than L2-sized chunks).
-//   BLUESTEIN everything else: chirp-z with a power-of-two convolution of
-//             nextPow2(2n-1) points (fft/DoubleFFT_1D.java:1864-2107), chirp
-//             tables generated in FP64 on the device.
+//   BLUESTEIN everything else: chirp-z (fft/DoubleFFT_1D.java:1864-2107), chirp
+//             tables generated in FP64 on the device; floats around a convolution
+//             just above 2n - 1 in one kernel or three (jt_bluemix.cuh), doubles
+//             (and long floats) around one of nextPow2(2n - 1) points.
 #include "jt_device.cuh"
 #include "jt_stockham.cuh"
 #include "jt_batch.cuh"
@@ -246,10 +248,6 @@ static int device_init() {
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT2, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT3, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DHT, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
-        cudaFuncSetAttribute(blue_tile_kernel<-1, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
-        cudaFuncSetAttribute(blue_tile_kernel<1, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
-        cudaFuncSetAttribute(blue_tile_kernel<-1, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
-        cudaFuncSetAttribute(blue_tile_kernel<1, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_RFWD, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_RINV, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_RFWD, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
@@ -989,11 +987,10 @@ template <typename T> struct Fft1 {
     // kernel's limit or the batch's shared-memory cap) is recorded as the
     // same transform in two passes of shorter lines: the balanced split with
     // both lengths fitting, if there is one.
-    // A Bluestein length records its convolution at the smallest 7-smooth
-    // length >= 2n - 1 instead of the power of two: batch steps run every
-    // line on the mixed-radix tile passes, so the shorter convolution is
-    // less work there (up to 2x); single calls keep the power of two, whose
-    // register-kernel passes are faster.  Only for convolutions up to 2^20.
+    // A Bluestein length that has no register-pass steps (record_blue) records
+    // its convolution at the smallest 7-smooth length >= 2n - 1 instead of the
+    // power of two: less work (up to 2x) on the batch's mixed-radix steps.
+    // Only for convolutions up to 2^20.
     int64_t rec_length() const {
         const int64_t nS = next_smooth(2 * n - 1);
         return nB > ((int64_t)1 << 20) || (nS >= nB && !bn1) ? 0 : nS;
@@ -1030,16 +1027,15 @@ template <typename T> struct Fft1 {
         return rec_alt->init_twopass(best);
     }
 
-    // Bluestein in one CTA tile (jt_chirp.cuh) when the padded length fits
-    // the tile passes: always inside batches, and for float calls (double
-    // calls keep the register-kernel FFTs of the FP64-bound convolution)
+    // Bluestein as one batch step (jt_chirp.cuh) when the convolution fits a
+    // task; floats only where record_blue's lines do not
     bool blue_fused_ok(const Ctx &ctx) const {
-        const bool rec = ctx.rec || ctx.rec_sizing;
-        return pbl && pbl->algo == ALG_DIRECT && pbl->W && generic_ok(nB) && (rec || sizeof(T) == 4) &&
-               (!rec || batch_line_ok<T>(nB));
+        return (ctx.rec || ctx.rec_sizing) && pbl && pbl->algo == ALG_DIRECT && pbl->W && generic_ok(nB) &&
+               batch_line_ok<T>(nB);
     }
     int exec_blue_fused(Ctx &ctx, const C2 *in, int64_t din, C2 *out, int64_t dout, int64_t batch, int sign,
                         double scale) const {
+        if (!ctx.rec) return JT_OK;  // no scratch
         BlueParams p;
         memset(&p, 0, sizeof(p));
         p.n = (int)n;
@@ -1049,7 +1045,7 @@ template <typename T> struct Fft1 {
         p.npass = (int)rr.size();
         for (int i = 0; i < p.npass; i++) p.radix[i] = rr[i];
         const size_t per_line = tile_line<T>((int)nB);
-        int C = (int)std::max<int64_t>(1, (ctx.rec ? kBatchTileElems : (sizeof(T) == 4 ? 4096 : 2048)) / nB);
+        int C = (int)std::max<int64_t>(1, kBatchTileElems / nB);
         C = std::min(C, (int)std::max<size_t>(1, (size_t)g_smem_optin / per_line));
         if ((int64_t)C > batch) C = (int)batch;
         p.C = C;
@@ -1058,32 +1054,20 @@ template <typename T> struct Fft1 {
         p.lout = Layout{1, dout, 0, 1};
         p.scale = scale;
         p.scalef = (float)scale;
-        if (ctx.rec) {
-            BOp o;
-            memset(&o, 0, sizeof(o));
-            o.type = BOP_BLUE;
-            o.prec = sizeof(T) == 4 ? 0 : 1;
-            o.sign = sign;
-            o.in = in;
-            o.out = out;
-            o.W = pbl->W;
-            o.Whi = bk1;
-            o.Wlo = bk2;
-            o.bp = p;
-            o.ntasks = (int)cdiv(batch, C);
-            o.smem = (int)(per_line * C);
-            emit(ctx, o);
-            return JT_OK;
-        }
-        if (ctx.dry) return JT_OK;  // no scratch
-        const int64_t grid = cdiv(batch, C);
-        if (grid > 0x7fffffff) return JT_ETOOBIG;
-        const int threads = (int)std::min<int64_t>(512, std::max<int64_t>(64, cdiv((int64_t)C * nB / 16, 32) * 32));
-        if (sign < 0)
-            pdl_launch(blue_tile_kernel<-1, T>, (unsigned)grid, threads, per_line * C, ctx.s, in, out, p, pbl->W, bk1, bk2);
-        else
-            pdl_launch(blue_tile_kernel<1, T>, (unsigned)grid, threads, per_line * C, ctx.s, in, out, p, pbl->W, bk1, bk2);
-        g_launches++;
+        BOp o;
+        memset(&o, 0, sizeof(o));
+        o.type = BOP_BLUE;
+        o.prec = sizeof(T) == 4 ? 0 : 1;
+        o.sign = sign;
+        o.in = in;
+        o.out = out;
+        o.W = pbl->W;
+        o.Whi = bk1;
+        o.Wlo = bk2;
+        o.bp = p;
+        o.ntasks = (int)cdiv(batch, C);
+        o.smem = (int)(per_line * C);
+        emit(ctx, o);
         return JT_OK;
     }
 
@@ -1207,7 +1191,7 @@ template <typename T> struct Fft1 {
         if (generic_ok(n)) {
             const int L = (int)n;
             const bool strided = lin.estride != 1 || lout.estride != 1;
-            int64_t target = kBatchTileElems;  // the batch CTA has 512 threads: 512 radix-16 butterflies
+            int64_t target = kBatchTileElems;  // a radix-16 butterfly for each thread
             int C = (int)std::max<int64_t>(1, target / L);
             if (strided) C = std::max(C, sizeof(T) == 4 ? 16 : 8);
             size_t per_line = tile_line<T>(L);

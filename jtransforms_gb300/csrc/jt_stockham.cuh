@@ -86,14 +86,6 @@ template <typename T> struct StockCfg {
     static constexpr int C(int L, int mode) { return mode == 0 ? rows_C(L) : mode == 2 ? rows2_C(L) : cols_C(L); }
 };
 
-// Pass twiddle table of a length-L line (one per length, built by
-// passtw_kernel): pass P >= 1 of radix R after NS = 16^P owns NS * R slots
-// holding w_{NS R}^{jm k} for jm < NS, k = 1..R-1, factor-major so that the
-// threads of a warp (consecutive jm) read consecutive addresses.  Float
-// tables: factor 1 as NS entries, then factors (2,3), (4,5), ... as NS
-// 16-byte pairs each; double tables: factor k as NS entries.  Passes are
-// radix 16 (E = 16 elements per thread) with a last pass of the remaining
-// radix.
 // Numbers per thread of a length-L line of doubles (jt_fix64.cuh).  Eight
 // (radix-8 passes, 64 registers, twice the threads) where that takes no more
 // passes than sixteen: at 64 = 8 x 8 one pass over 2^16 points took 4.7 us
@@ -103,6 +95,15 @@ template <typename T> struct StockCfg {
 // of 1024 112 -> 141, 4096 11.7 -> 12.7 and 214 -> 243.
 __host__ __device__ constexpr int fx_elems(int L) { return L == 64 || L == 512 ? 8 : 16; }
 
+// Pass twiddle table of a length-L line (one per length, built by
+// passtw_kernel): pass P >= 1 of radix R after NS = 16^P owns NS * R slots
+// holding w_{NS R}^{jm k} for jm < NS, k = 1..R-1, factor-major so that the
+// threads of a warp (consecutive jm) read consecutive addresses.  Float
+// tables: factor 1 as NS entries, then factors (2,3), (4,5), ... as NS
+// 16-byte pairs each; double tables: factor k as NS entries.  Passes are
+// radix E (elements per thread: 16, or fx_elems) with a last pass of the
+// remaining radix.  Double tables are followed by the same entries in fixed
+// point (int4, fx_twiddle below).
 // E: elements per thread, 0 for the usual 16.
 __host__ __device__ inline int stock_tw_count(int L, int E = 0) {
     if (E == 0) E = L >= 16 ? 16 : L;
@@ -120,9 +121,6 @@ __host__ __device__ inline int stock_tw_count(int L, int E = 0) {
     return tot;
 }
 
-//
-// Double tables are followed by the same entries in fixed point (int4,
-// fx_twiddle below).
 template <typename T> __global__ void passtw_kernel(typename V2<T>::t *out, int L, int E) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     int logl = 0, loge = 0;
@@ -229,10 +227,8 @@ template <typename T, int L, int MODE, int SIGN, int EL = (L >= 16 ? 16 : L)> st
     static constexpr size_t BIG_SMEM = BIG_X + (size_t)BIG_MP * TL * sizeof(C2) + 16;
     static constexpr bool BIG_OK = MODE == 0 && C == 1 && !PIPE_OK && BIG_MP >= E / 2;
     // blocks per SM the register budget is sized for (about 24 warps)
-    // (double lines need twice the registers: no cap beyond one block at 256+)
     // (single-warp blocks of short lines get more registers per thread: 18 warps)
-    static constexpr int MINB = sizeof(T) == 4 ? (NT >= 512 || NT < 32 ? 1 : NT < 64 ? 576 / NT : 768 / NT)
-                                               : (NT >= 256 || NT < 64 ? 1 : 384 / NT);
+    static constexpr int MINB = NT >= 512 || NT < 32 ? 1 : NT < 64 ? 576 / NT : 768 / NT;
 
     template <int P> struct Pass {
         static constexpr int R = P < NFULL ? E : REM;
