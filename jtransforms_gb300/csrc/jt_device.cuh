@@ -9,7 +9,10 @@
 //                       two-pass (four-step) scheme.  Replaces the Ooura
 //                       split-radix tree (utils/CommonUtils.java:708-5749),
 //                       bitrv2* and the FFTPACK passes (fft/DoubleFFT_1D.java:
-//                       6630-7842).
+//                       6630-7842).  Lines that no register kernel takes
+//                       (jt_stockham.cuh, jt_fix64.cuh, jt_mixed.cuh,
+//                       jt_fixmix.cuh); doubles of 48 points and more compute in
+//                       fixed point (tile_passes_fx).
 //   real_*              real-FFT pack/unpack around a half-length complex FFT
 //                       (replaces rftfsub/rftbsub, utils/CommonUtils.java:5750-5830).
 //   bluestein_*         chirp multiplies (fft/DoubleFFT_1D.java:1920-2107).
@@ -18,6 +21,8 @@
 //                       dht/DoubleDHT_1D.java).
 //   rdft2d_kernel, ytransform*_kernel   2D real packing fix-up and DHT nD
 //                       combine (fft/DoubleFFT_2D.java:2544, dht/DoubleDHT_3D.java:2314).
+//   fill_symmetric_kernel   the right half of a real array's full spectrum
+//                       (fillSymmetric, fft/DoubleFFT_2D.java, fft/DoubleFFT_3D.java).
 //   transpose_kernel    batched tiled transpose for axis passes.
 //   table kernels       FP64 twiddle/chirp generation with sincospi.
 #pragma once

@@ -4,10 +4,10 @@
 // A CTA holds C lines of n reals as C complex lines of h = n/2 in shared
 // memory and runs the h-point complex FFT on them: in registers with the
 // Stockham core for power-of-two h from 16 to 4096 (r2r_reg_kernel, floats;
-// doubles: jt_fixr2r.cuh), else with the tile passes of jt_device.cuh (r2r_tile_kernel, also the batch's
-// one-step form).  Contiguous lines whose scalar pairs are aligned complex
-// values move as pairs, the rest one scalar at a time.  Around the FFT
-// (Makhoul's reordering, the standard real-FFT split and the DCT
+// doubles: jt_fixr2r.cuh), else with the tile passes of jt_device.cuh
+// (r2r_tile_kernel, also the batch's one-step form).  Contiguous lines whose
+// scalar pairs are aligned complex values move as pairs, the rest one scalar at
+// a time.  Around the FFT (Makhoul's reordering, the standard real-FFT split and the DCT
 // quarter-wave twiddle):
 //   forward DCT/DST   load:  v_j = x_2j, v_{n-1-j} = x_2j+1 (DST: odd
 //                            inputs negated), z_m = v_2m + i v_2m+1
