@@ -746,7 +746,7 @@ __device__ __forceinline__ void bluestein_pre_body(const C2 *a, int64_t dist, C2
 template <int SIGN, typename T>
 __global__ void bluestein_pre_kernel(const C2 *a, int64_t dist, C2 *tmp, const C2 *__restrict__ bk1, int64_t n, int64_t nB,
                                      int64_t batch) {
-    pdl_begin();
+    pdl_begin_few();
     bluestein_pre_body<SIGN, T>(a, dist, tmp, bk1, n, nB, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -759,7 +759,7 @@ __device__ __forceinline__ void bluestein_mul_body(C2 *tmp, const C2 *__restrict
 
 template <int SIGN, typename T>
 __global__ void bluestein_mul_kernel(C2 *tmp, const C2 *__restrict__ bk2, int64_t nB, int64_t total) {
-    pdl_begin();
+    pdl_begin_few();
     bluestein_mul_body<SIGN, T>(tmp, bk2, nB, total, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -777,7 +777,7 @@ __device__ __forceinline__ void bluestein_post_body(C2 *a, int64_t dist, const C
 template <int SIGN, typename T>
 __global__ void bluestein_post_kernel(C2 *a, int64_t dist, const C2 *tmp, const C2 *__restrict__ bk1, int64_t n, int64_t nB,
                                       int64_t batch, T scale) {
-    pdl_begin();
+    pdl_begin_few();
     bluestein_post_body<SIGN, T>(a, dist, tmp, bk1, n, nB, batch, scale, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -825,7 +825,7 @@ __device__ __forceinline__ void real_post_packed_body(T *a, int64_t dist, int64_
 
 template <typename T>
 __global__ void real_post_packed_kernel(T *a, int64_t dist, int64_t n, int64_t batch, const C2 *__restrict__ Wr) {
-    pdl_begin();
+    pdl_begin_few();
     real_post_packed_body<T>(a, dist, n, batch, Wr, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -866,7 +866,7 @@ __device__ __forceinline__ void real_post_full_body(const T *zin, int64_t zdist,
 template <int SIGN, typename T>
 __global__ void real_post_full_kernel(const T *zin, int64_t zdist, T *out, int64_t odist, int64_t n, int64_t batch,
                                       const C2 *__restrict__ Wr, T scale) {
-    pdl_begin();
+    pdl_begin_few();
     real_post_full_body<SIGN, T>(zin, zdist, out, odist, n, batch, Wr, scale, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -906,7 +906,7 @@ __device__ __forceinline__ void real_pre_inverse_body(T *a, int64_t dist, int64_
 
 template <typename T>
 __global__ void real_pre_inverse_kernel(T *a, int64_t dist, int64_t n, int64_t batch, const C2 *__restrict__ Wr, T mult) {
-    pdl_begin();
+    pdl_begin_few();
     real_pre_inverse_body<T>(a, dist, n, batch, Wr, mult, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -921,7 +921,7 @@ __device__ __forceinline__ void real_to_complex_body(const T *a, int64_t dist, C
 
 template <typename T>
 __global__ void real_to_complex_kernel(const T *a, int64_t dist, C2 *tmp, int64_t n, int64_t batch) {
-    pdl_begin();
+    pdl_begin_few();
     real_to_complex_body<T>(a, dist, tmp, n, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -943,7 +943,7 @@ __device__ __forceinline__ void pack_from_full_body(const C2 *F, T *a, int64_t d
 
 template <typename T>
 __global__ void pack_from_full_kernel(const C2 *F, T *a, int64_t dist, int64_t n, int64_t batch) {
-    pdl_begin();
+    pdl_begin_few();
     pack_from_full_body<T>(F, a, dist, n, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -965,7 +965,7 @@ __device__ __forceinline__ void unpack_to_full_body(const T *a, int64_t dist, C2
 
 template <typename T>
 __global__ void unpack_to_full_kernel(const T *a, int64_t dist, C2 *F, int64_t n, int64_t batch) {
-    pdl_begin();
+    pdl_begin_few();
     unpack_to_full_body<T>(a, dist, F, n, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -979,7 +979,7 @@ __device__ __forceinline__ void real_part_body(const C2 *F, T *a, int64_t dist, 
 
 template <typename T>
 __global__ void real_part_kernel(const C2 *F, T *a, int64_t dist, int64_t n, int64_t batch, T mult) {
-    pdl_begin();
+    pdl_begin_few();
     real_part_body<T>(F, a, dist, n, batch, mult, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -998,7 +998,7 @@ __device__ __forceinline__ void copy_complex_body(const C2 *src, int64_t sdist, 
 template <typename T>
 __global__ void copy_complex_kernel(const C2 *src, int64_t sdist, C2 *dst, int64_t ddist, int64_t len, int64_t batch,
                                     T scale, int conj) {
-    pdl_begin();
+    pdl_begin_few();
     copy_complex_body<T>(src, sdist, dst, ddist, len, batch, scale, conj, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1019,7 +1019,7 @@ __device__ __forceinline__ void dct2_pre_body(const T *a, int64_t dist, T *v, in
 
 template <typename T>
 __global__ void dct2_pre_kernel(const T *a, int64_t dist, T *v, int64_t vdist, int64_t n, int64_t batch, int dst) {
-    pdl_begin();
+    pdl_begin_few();
     dct2_pre_body<T>(a, dist, v, vdist, n, batch, dst, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1050,7 +1050,7 @@ __device__ __forceinline__ void dct2_post_body(const T *v, int64_t vdist, T *a, 
 template <typename T>
 __global__ void dct2_post_kernel(const T *v, int64_t vdist, T *a, int64_t dist, int64_t n, int64_t batch,
                                  const C2 *__restrict__ Wd, T mult, T mult0, int dst) {
-    pdl_begin();
+    pdl_begin_few();
     dct2_post_body<T>(v, vdist, a, dist, n, batch, Wd, mult, mult0, dst, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1083,7 +1083,7 @@ __device__ __forceinline__ void dct3_pre_body(const T *a, int64_t dist, T *v, in
 template <typename T>
 __global__ void dct3_pre_kernel(const T *a, int64_t dist, T *v, int64_t vdist, int64_t n, int64_t batch,
                                 const C2 *__restrict__ Wd, T mult, T mult0, int dst) {
-    pdl_begin();
+    pdl_begin_few();
     dct3_pre_body<T>(a, dist, v, vdist, n, batch, Wd, mult, mult0, dst, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1100,7 +1100,7 @@ __device__ __forceinline__ void dct3_post_body(const T *v, int64_t vdist, T *a, 
 
 template <typename T>
 __global__ void dct3_post_kernel(const T *v, int64_t vdist, T *a, int64_t dist, int64_t n, int64_t batch, int dst) {
-    pdl_begin();
+    pdl_begin_few();
     dct3_post_body<T>(v, vdist, a, dist, n, batch, dst, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1115,7 +1115,7 @@ __device__ __forceinline__ void dht_post_body(const T *v, int64_t vdist, T *a, i
 
 template <typename T>
 __global__ void dht_post_kernel(const T *v, int64_t vdist, T *a, int64_t dist, int64_t n, int64_t batch, T mult) {
-    pdl_begin();
+    pdl_begin_few();
     dht_post_body<T>(v, vdist, a, dist, n, batch, mult, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1126,7 +1126,7 @@ __global__ void dht_post_kernel(const T *v, int64_t vdist, T *a, int64_t dist, i
 // pass of realForward, -1 before the column pass of realInverse.
 template <typename T>
 __global__ void rdft2d_kernel(T *a, int64_t dist, int64_t rows, int64_t cols, int64_t batch, int isgn) {
-    pdl_begin();
+    pdl_begin_few();
     const int64_t n1h = rows >> 1;
     const int64_t q = n1h > 1 ? n1h - 1 : 0;
     int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1157,7 +1157,7 @@ __global__ void rdft2d_kernel(T *a, int64_t dist, int64_t rows, int64_t cols, in
 // pairs are disjoint, so any order gives the reference's result.
 template <typename T>
 __global__ void rdft3d_kernel(T *a, int64_t dist, int64_t slices, int64_t rows, int64_t cols, int64_t batch, int isgn) {
-    pdl_begin();
+    pdl_begin_few();
     const int64_t n1h = slices >> 1, n2h = rows >> 1, ss = rows * cols, rs = cols;
     const int64_t per = n1h * n2h * 2;
     int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1208,7 +1208,7 @@ __global__ void rdft3d_kernel(T *a, int64_t dist, int64_t slices, int64_t rows, 
 // order; they never share elements with other quadruples.
 template <typename T>
 __global__ void ytransform2_kernel(T *a, int64_t rows, int64_t cols) {
-    pdl_begin();
+    pdl_begin_few();
     int64_t nr = rows / 2 + 1, nc = cols / 2 + 1;
     int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (idx >= nr * nc) return;
@@ -1226,7 +1226,7 @@ __global__ void ytransform2_kernel(T *a, int64_t rows, int64_t cols) {
 // DHT yTransform, 3D (dht/DoubleDHT_3D.java:2314-2356)
 template <typename T>
 __global__ void ytransform3_kernel(T *a, int64_t slices, int64_t rows, int64_t cols) {
-    pdl_begin();
+    pdl_begin_few();
     int64_t ns = slices / 2 + 1, nr = rows / 2 + 1, nc = cols / 2 + 1;
     int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (idx >= ns * nr * nc) return;
@@ -1258,7 +1258,7 @@ __global__ void ytransform3_kernel(T *a, int64_t slices, int64_t rows, int64_t c
 // The right half of the spectrum of real data: F[-s][-r][C - k] = conj
 // F[s][r][k], 0 < k < C / 2 (C even), per array of S x R x C.
 template <typename T> __global__ void fill_symmetric_kernel(C2 *a, int64_t S, int64_t R, int64_t C, int64_t batch) {
-    pdl_begin();
+    pdl_begin_few();
     const int64_t q = C / 2 - 1, idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (idx >= batch * S * R * q) return;
     int64_t k, r, s;
@@ -1302,7 +1302,7 @@ template <typename T> __device__ __forceinline__ void scale_body(T *a, int64_t d
 }
 
 template <typename T> __global__ void scale_kernel(T *a, int64_t dist, int64_t len, int64_t batch, T s) {
-    pdl_begin();
+    pdl_begin_few();
     scale_body(a, dist, len, batch, s, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
@@ -1314,7 +1314,7 @@ template <typename T> __device__ __forceinline__ void copy_real_body(const T *sr
 }
 
 template <typename T> __global__ void copy_real_kernel(const T *src, int64_t sdist, T *dst, int64_t ddist, int64_t len, int64_t batch) {
-    pdl_begin();
+    pdl_begin_few();
     copy_real_body(src, sdist, dst, ddist, len, batch, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 

@@ -138,7 +138,7 @@ static inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
         if (!(ctx).dry && (total) > 0) {                                               \
             int64_t g_ = cdiv((total), 256);                                           \
             auto kfn_ = kernel;                                                        \
-            pdl_launch(kfn_, (unsigned)g_, 256, 0, (ctx).s, __VA_ARGS__);              \
+            pdl_launch_if(g_ <= JT_PDL_BLOCKS, kfn_, (unsigned)g_, 256, 0, (ctx).s, __VA_ARGS__); \
             g_launches++;                                                              \
         }                                                                              \
     } while (0)
