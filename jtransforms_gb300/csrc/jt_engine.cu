@@ -2152,7 +2152,7 @@ template <typename T> struct PlanImpl {
         const bool sc = sign > 0 && scale;
         const double s = sc ? 1.0 / (double)n : 1.0;
         C2 *c = (C2 *)a, *tmp = (C2 *)ctx.ws->get(sizeof(C2) * rows * h, ctx.dry);
-        JT_TRY(r->half->exec(ctx, c, h, tmp, h, rows, sign, 1.0));
+        JT_TRY(half_rows(ctx, r->half.get(), c, tmp, batch, S * R, sign));
         if (sign < 0) LAUNCH1D(ctx, rows * (h / 2 + 1), (real_post_full_kernel<-1, T>), (const T *)tmp, n, a, 2 * n, n, rows, r->Wr, s);
         else LAUNCH1D(ctx, rows * (h / 2 + 1), (real_post_full_kernel<1, T>), (const T *)tmp, n, a, 2 * n, n, rows, r->Wr, s);
         // columns 0..h, to the next 16 (whole tiles of the column kernels); the
@@ -2167,6 +2167,19 @@ template <typename T> struct PlanImpl {
                 JT_TRY(half_columns(ctx, fs, c + b * S * R * n, R, S, w, n, n, R * n, sign, sc ? 1.0 / (double)S : 1.0));
         }
         LAUNCH1D(ctx, rows * (h - 1), fill_symmetric_kernel<T>, c, S, R, n, batch);
+        return JT_OK;
+    }
+    // Half-length FFTs of the real rows of `batch` arrays (each N reals, the
+    // arrays 2N apart) into `out`, row after row.
+    int half_rows(Ctx &ctx, Fft1<T> *f, const C2 *a, C2 *out, int64_t batch, int64_t rows, int sign) {
+        const int64_t h = f->n;
+        if (f->algo == ALG_DIRECT)
+            return f->exec_direct(ctx, a, out, batch * rows, Layout{rows, N, h, 1}, Layout{1, h, 0, 1}, sign, 1.0);
+        const size_t mark = ctx.ws->used;
+        for (int64_t b = 0; b < batch; b++) {
+            ctx.ws->used = mark;  // the arrays run in order on one stream: one scratch region
+            JT_TRY(f->exec(ctx, a + b * N, h, out + b * rows * h, h, rows, sign, 1.0));
+        }
         return JT_OK;
     }
     // FFTs of length len over the first w columns of `blocks` blocks (stride
