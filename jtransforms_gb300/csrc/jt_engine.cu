@@ -2163,8 +2163,11 @@ template <typename T> struct PlanImpl {
         JT_TRY(half_columns(ctx, fr, c, batch * S, R, w, n, R * n, n, sign, s1));
         if (nd == 3) {
             Fft1<T> *fs = fft.at(S).get();
-            for (int64_t b = 0; b < batch; b++)
+            const size_t mark = ctx.ws->used;
+            for (int64_t b = 0; b < batch; b++) {
+                ctx.ws->used = mark;  // the arrays run in order on one stream: one scratch region
                 JT_TRY(half_columns(ctx, fs, c + b * S * R * n, R, S, w, n, n, R * n, sign, sc ? 1.0 / (double)S : 1.0));
+            }
         }
         LAUNCH1D(ctx, rows * (h - 1), fill_symmetric_kernel<T>, c, S, R, n, batch);
         return JT_OK;

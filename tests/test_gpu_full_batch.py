@@ -45,3 +45,28 @@ def test_full_of_several_arrays(prec, shape, op, batch, where):
         want = np.fft.fftn(z) if op == "forward" else np.fft.ifftn(z) * (1 if op == "inverse scaled" else size)
         got = np.ascontiguousarray(out[b, :2 * size]).astype(np.float64).view(np.complex128).reshape(shape)
         assert rel_l2(got, want) <= tol(size, dt)
+
+
+def test_slices_of_several_arrays_share_scratch():
+    """71 slices run through a transposed copy (0.6 MB an array) and a
+    convolution of 256 (2.1 MB an array): beside the reals of all arrays
+    (2.3 MB) that is 5 MB for eight arrays as for one, and 24 MB if each array
+    had its own."""
+    import torch
+    import jtransforms_gb300 as J
+    from jtransforms_gb300 import _native as N
+    shape, batch = (71, 8, 64), 8
+    size = int(np.prod(shape))
+    f = J.DoubleFFT_3D(*shape)
+    x = np.random.default_rng(0).standard_normal((batch,) + shape)
+    a = np.zeros((batch, 2 * size))
+    a[:, :size] = x.reshape(batch, -1)
+    dev = torch.from_numpy(a.ravel()).cuda()
+    prev = N.set_option(N.OPT_ARENA_LIMIT_MB, 8)
+    try:
+        f.plan.execute(N.REAL_FORWARD_FULL, dev, 0, False, batch=batch, dist=2 * size)
+    finally:
+        N.set_option(N.OPT_ARENA_LIMIT_MB, prev)
+    got = dev.cpu().numpy().view(np.complex128).reshape((batch,) + shape)
+    for b in range(batch):
+        assert rel_l2(got[b], np.fft.fftn(x[b])) <= tol(size, np.float64)
