@@ -253,15 +253,14 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::NT,
         const Fx r = fx_mul<-1>(f, __ldg(&Wloq[x & ((1u << p.tw_lo_bits) - 1u)]));
         return Fx{r.x << 2, r.y << 2};
     };
-    auto factor = [](Fx a) { return make_int4(fx_hi(a.x), fx_lo(a.x), fx_hi(a.y), fx_lo(a.y)); };
     typedef typename S::template Pass<F::NPASS - 1> LP_;
     Fx wq{0, 0}, w{0, 0};
     int4 g1 = make_int4(0, 0, 0, 0), gn = g1;
     if constexpr (TW) {
         const uint32_t g = (uint32_t)F::TL * j2;
         wq = two_level((uint32_t)t * j2);
-        g1 = factor(two_level(g));
-        gn = LP_::NB > 1 ? factor(two_level((uint32_t)LP_::NB * g)) : g1;
+        g1 = fx_as_factor(two_level(g));
+        gn = LP_::NB > 1 ? fx_as_factor(two_level((uint32_t)LP_::NB * g)) : g1;
     }
     auto times = [](Fx a, int4 b) {
         const Fx r = fx_mul<-1>(a, b);
@@ -281,7 +280,7 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::NT,
                 } else {
                     w = times(w, gn);
                 }
-                u[k] = fx_mul<SIGN>(u[k], factor(w));
+                u[k] = fx_mul<SIGN>(u[k], fx_as_factor(w));
             }
             r[k] = make_double2(fx_to(u[k].x, ex), fx_to(u[k].y, ex));
         }

@@ -39,6 +39,14 @@ template <int SIGN> __device__ __forceinline__ Fx fx_mul(Fx v, int4 w) {
     return r;
 }
 
+// A factor formed at run time (a product of two), with values at 2^62.  fx_mul
+// negates the sine's low half, which the lowest int does not survive: it is
+// moved by one, as in the tables (fx_split).
+__device__ __forceinline__ int4 fx_as_factor(Fx a) {
+    if ((int)a.y == INT32_MIN) a.y++;
+    return make_int4(fx_hi(a.x), fx_lo(a.x), fx_hi(a.y), fx_lo(a.y));
+}
+
 // v k / 2^64 rounded, for a constant |k| < 2^63: v times a factor in (-1/2, 1/2)
 __device__ __forceinline__ long long fx_mulk(long long v, long long k) {
     const int vh = fx_hi(v), vl = fx_lo(v), kh = (int)((k + (1ll << 31)) >> 32), kl = (int)k;

@@ -202,7 +202,7 @@ struct FixMixTile {
                         const int4 a = __ldg(&p.Whiq[x >> m.tw_lo_bits]);
                         Fx w = fx_mul<-1>(Fx{((long long)a.x << 32) + a.y, ((long long)a.z << 32) + a.w}, __ldg(&p.Wloq[x & mask]));
                         w = Fx{w.x << 2, w.y << 2};
-                        v[k] = fx_mul<-1>(v[k], make_int4(fx_hi(w.x), fx_lo(w.x), fx_hi(w.y), fx_lo(w.y)));
+                        v[k] = fx_mul<-1>(v[k], fx_as_factor(w));
                         x += dx;
                     }
                 }
