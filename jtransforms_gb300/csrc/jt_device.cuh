@@ -475,8 +475,13 @@ __device__ __forceinline__ void fx_pass_r(const Fx *src, Fx *dst, int lines, int
     }
 }
 
-// A generic odd radix (11..63): one thread per output, whose R products by
-// roots divide by 4 (after the twiddles' 4, if there are any).
+// A generic odd radix (11..63): one thread per output, whose R products by roots
+// are summed with 24 bits below the unit, over 4 (after twiddles that divide by
+// nothing).  Its numbers have fx_room's bits less than 60, so that the sum fits.
+// (Rounded product by product it was 1.4 to 6 times as far off as FP64 on lines
+// with one large number.)
+__host__ __device__ constexpr bool fx_generic(int R) { return !(R == 2 || R == 3 || R == 4 || R == 5 || R == 7 || R == 8 || R == 16); }
+__host__ __device__ constexpr int fx_room(int R) { return R > 32 ? 2 : R > 16 ? 1 : 0; }
 template <int SIGN>
 __device__ void fx_pass_generic(const Fx *src, Fx *dst, int lines, int L, int Lp, int Ns, int R, const int4 *__restrict__ Wq,
                                 const uint32_t *bin, uint32_t *bout) {
@@ -486,21 +491,30 @@ __device__ void fx_pass_generic(const Fx *src, Fx *dst, int lines, int L, int Lp
         const int c = idx / L, e0 = idx - c * L, k = e0 / nb, j = e0 - k * nb;
         const Fx *s = src + c * Lp;
         const int jm = j % Ns;
-        int sh = Ns > 1 ? fx_norm_shift(bin[c]) : 0;
+        int sh = Ns > 1 ? fx_norm_shift(bin[c]) + fx_room(R) : 0;
         const int left = sh < 0 ? -sh : 0;
         sh = sh < 0 ? 0 : sh;
-        const long long r1 = fx_half(sh), r0 = fx_half(sh + 2);
-        Fx sum{0, 0};
+        const long long r1 = fx_half(sh);
+        Fx hi{0, 0}, mid{0, 0};  // of weight 4 and 2^-30 (mid: over 2^8)
         int e = 0;  // k m mod R
         for (int m = 0; m < R; m++) {
             Fx x = s[pad(j + m * nb)];
             x = Fx{x.x << left, x.y << left};
-            if (Ns > 1) x = m == 0 ? fx_shr(x, sh + 2, r0) : fx_mul<SIGN>(fx_shr(x, sh, r1), __ldg(&Wq[jm * m * step]));
-            x = m == 0 ? fx_shr(x, 2, 2) : fx_mul<SIGN>(x, __ldg(&Wq[e * rstep]));
-            sum = fx_add(sum, x);
+            if (Ns > 1) {
+                x = fx_shr(x, sh, r1);
+                if (m > 0) x = fx_mul_full<SIGN>(x, __ldg(&Wq[jm * m * step]));
+            }
+            const int4 w = __ldg(&Wq[e * rstep]);
+            const int xh = fx_hi(x.x), xl = fx_lo(x.x), yh = fx_hi(x.y), yl = fx_lo(x.y);
+            const int ph = SIGN < 0 ? w.z : -w.z, pl = SIGN < 0 ? w.w : -w.w;
+            hi.x = fx_madw(yh, -ph, fx_madw(xh, w.x, hi.x));
+            hi.y = fx_madw(xh, ph, fx_madw(yh, w.x, hi.y));
+            mid.x += fx_madw(yl, -ph, fx_madw(yh, -pl, fx_madw(xl, w.x, fx_madw(xh, w.y, 0)))) >> 8;
+            mid.y += fx_madw(xl, ph, fx_madw(xh, pl, fx_madw(yl, w.x, fx_madw(yh, w.y, 0)))) >> 8;
             e += k;
             if (e >= R) e -= R;
         }
+        const Fx sum{hi.x + ((mid.x + (1 << 23)) >> 24), hi.y + ((mid.y + (1 << 23)) >> 24)};
         dst[c * Lp + pad((j - jm) * R + jm + k * Ns)] = sum;
         fx_join<false>(bout, c, fx_bits(sum.x) | fx_bits(sum.y));
     }
@@ -527,8 +541,7 @@ __device__ __noinline__ double2 *tile_passes_fx(double2 *src, double2 *dst, int 
         fx_join<true>(b0, c, m);
     }
     if (__syncthreads_or(special)) return tile_passes_fp<SIGN, double>(src, dst, lines, L, Lp, npass, radix, W);
-    // a generic first radix sums up to 63 numbers: it starts two bits lower
-    const int low = radix[0] > 16 || radix[0] == 11 || radix[0] == 13 || radix[0] == 15 ? 2 : 0;
+    const int low = fx_generic(radix[0]) ? fx_room(radix[0]) - 2 : 0;  // against 58 bits
     for (int c = tid; c < lines; c += nt) {
         const FxLine l = fx_line(b0[c]);
         ex[c] = l.ex + low;
@@ -547,9 +560,10 @@ __device__ __noinline__ double2 *tile_passes_fx(double2 *src, double2 *dst, int 
     for (int ps = 0; ps < npass; ps++) {
         __syncthreads();
         const int R = radix[ps];
-        const bool gen = !(R == 2 || R == 3 || R == 4 || R == 5 || R == 7 || R == 8 || R == 16);
+        const bool gen = fx_generic(R);
         for (int c = tid; c < lines; c += nt) {
-            ex[c] += (Ns > 1 ? fx_norm_shift(b0[c]) + 2 : 0) + (gen ? 2 : 0);
+            if (Ns > 1) ex[c] += fx_norm_shift(b0[c]) + 2 + (gen ? fx_room(R) : 0);
+            else if (gen) ex[c] += 2;
             b2[c] = 0;
         }
         switch (R) {

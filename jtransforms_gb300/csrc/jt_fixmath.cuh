@@ -39,6 +39,21 @@ template <int SIGN> __device__ __forceinline__ Fx fx_mul(Fx v, int4 w) {
     return r;
 }
 
+// The same without the division, for what no butterfly follows: |v| below 2^62,
+// results below 2^63.  (Two units off at most.)
+template <int SIGN> __device__ __forceinline__ Fx fx_mul_full(Fx v, int4 w) {
+    const int xh = fx_hi(v.x), xl = fx_lo(v.x), yh = fx_hi(v.y), yl = fx_lo(v.y);
+    const int ph = SIGN < 0 ? w.z : -w.z, pl = SIGN < 0 ? w.w : -w.w;
+    const int nh = SIGN < 0 ? -w.z : w.z, nl = SIGN < 0 ? -w.w : w.w;
+    const long long half = 1ll << 29;
+    long long m = fx_madw(yl, nh, fx_madw(yh, nl, fx_madw(xl, w.x, fx_madw(xh, w.y, half))));
+    Fx r;
+    r.x = (fx_madw(yh, nh, fx_madw(xh, w.x, 0)) << 2) + (m >> 30);
+    m = fx_madw(xl, ph, fx_madw(xh, pl, fx_madw(yl, w.x, fx_madw(yh, w.y, half))));
+    r.y = (fx_madw(xh, ph, fx_madw(yh, w.x, 0)) << 2) + (m >> 30);
+    return r;
+}
+
 // A factor formed at run time (a product of two), with values at 2^62.  fx_mul
 // negates the sine's low half, which the lowest int does not survive: it is
 // moved by one, as in the tables (fx_split).
@@ -52,6 +67,12 @@ __device__ __forceinline__ long long fx_mulk(long long v, long long k) {
     const int vh = fx_hi(v), vl = fx_lo(v), kh = (int)((k + (1ll << 31)) >> 32), kl = (int)k;
     const long long m = fx_madw(vl, kh, fx_madw(vh, kl, 1ll << 31));
     return fx_madw(vh, kh, m >> 32);
+}
+// v k / 2^62, rounded, for 0 < k < 2^62
+__device__ __forceinline__ long long fx_mulk_full(long long v, long long k) {
+    const int vh = fx_hi(v), vl = fx_lo(v), kh = fx_hi(k), kl = fx_lo(k);
+    const long long m = fx_madw(vl, kh, fx_madw(vh, kl, 1ll << 29));
+    return (fx_madw(vh, kh, 0) << 2) + (m >> 30);
 }
 // round(f 2^64) for -1/2 < f < 1/2: cos(pi/4) - 1, sqrt(2) - 1, tan(pi/16), sin(pi/8)
 static constexpr long long kFxHm1 = -5402926248376769404ll;
@@ -231,26 +252,30 @@ struct FxLine {
     int pre;   // 0, or +-512: the doubles were multiplied by 2^pre first
 };
 
-#define JT_FX_BIAS 1080  // a double of the line's largest exponent eb is v 2^(eb - 1080), v < 2^58
-
-// From the line's largest (high word << 1) over all its numbers.
+// From the line's largest (high word << 1) over all its numbers: v below 1.4 x
+// 2^58 and the largest at least 1.4 x 2^57.  A 16-point DFT of such components
+// stays below 16 sqrt(2) 1.4 x 2^58 = 1.98 x 2^62; exponents alone would leave
+// lines whose largest is 1.0 (normalised images, constants) a bit less.
+#define JT_FX_BIAS 1081
 __device__ __forceinline__ FxLine fx_line(uint32_t m) {
-    const int eb = (int)(m >> 21);
+    const int eb = (int)((m + 1258291u) >> 21);  // mantissas of 1.4 and more (0.6 2^21) count as the next exponent
     FxLine l;
     l.pre = eb < 123 ? 512 : eb > 1923 ? -512 : 0;  // (lines of zeros too: subnormals may have no high word)
     l.ex = max(eb, 1) + l.pre - JT_FX_BIAS;
     return l;
 }
-// The line's numbers below 2^BITS (l.ex is for 58).
+// The line's numbers below 1.4 x 2^BITS (l.ex is for 58), rounded to nearest
+// (cut off, they were more than FP64's rounding off in lines of 4096 and more
+// with one large number).
 template <int BITS = 58> __device__ __forceinline__ long long fx_from(double d, const FxLine &l) {
     const int hi = __double2hiint(d), lo = __double2loint(d);
     const int e = (hi >> 20) & 0x7ff;
     const uint32_t mh = ((uint32_t)hi & 0xfffffu) | 0x100000u;
-    const int r = min(l.ex + JT_FX_BIAS + 63 - BITS - e, 63);  // at least 63 - BITS; zeros (and far smaller numbers) go to 0
-    unsigned long long u = (((unsigned long long)mh << 32) | (uint32_t)lo) << 10;
-    u >>= r;
-    const long long s = (long long)(hi >> 31);
-    return ((long long)u ^ s) - s;
+    const int r = min(l.ex + JT_FX_BIAS + 61 - BITS - e, 63);  // at least 61 - BITS; zeros (and far smaller numbers) go to 0
+    const unsigned long long u = (((unsigned long long)mh << 32) | (uint32_t)lo) << 10;
+    // (negative: -u - 1, a last place of the double's off, before the shift; one
+    // more of the result's halves after it, which rounds)
+    return (((long long)(u ^ (long long)(hi >> 31)) >> r) + 1) >> 1;
 }
 __device__ __forceinline__ double fx_to(long long v, int ex) {
     const double d = __ll2double_rn(v);

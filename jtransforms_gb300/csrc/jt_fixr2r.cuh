@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
         for (int m = 0; m < EH; m++) {
             const int k = t + m * TL;
             const bool z = m == 0 && t == 0;
-            Fx X{fx_from<61>(d[m].x, ln), fx_from<61>(d[m].y, ln)}, Y{fx_from<61>(d[EH + m].x, ln), fx_from<61>(d[EH + m].y, ln)};
+            constexpr int BITS = OP == R2R_DCT3 ? 61 : 59;
+            Fx X{fx_from<BITS>(d[m].x, ln), fx_from<BITS>(d[m].y, ln)}, Y{fx_from<BITS>(d[EH + m].x, ln), fx_from<BITS>(d[EH + m].y, ln)};
             Fx X0{0, 0};  // k = 0: (X_0, X_H)
             if (OP == R2R_DCT3) {
                 // V = e^{+i pi k/2n} (C_k - i C_{n-k}) / 4
@@ -177,23 +178,18 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
                     X = fx_mul<1>(Fx{X.x, -X.y}, __ldg(&Wdq[k]));
                     Y = fx_mul<1>(Fx{Y.x, -Y.y}, __ldg(&Wdq[H - k]));
                 }
-            } else {
-                X = fx_shr(X, 2, 2);
-                Y = fx_shr(Y, 2, 2);
-                if (z) {
-                    X0 = X;
-                    X = Y;
-                }
+            } else if (z) {
+                X0 = X;
+                X = Y;
             }
+            // (59 bits here and sums of four numbers: no division until all are known)
             const Fx s{X.x + Y.x, X.y - Y.y}, dd{X.x - Y.x, X.y + Y.y};
-            const Fx w = fx_mul<1>(dd, __ldg(&Wrq[z ? H / 2 : k]));  // e^{+2 pi i k/n} d / 4
-            const Fx s4 = fx_shr(s, 2, 2);
-            v[m] = Fx{s4.x - w.y, s4.y + w.x};
-            Fx u{s4.x + w.y, w.x - s4.y};
+            const Fx w = fx_mul_full<1>(dd, __ldg(&Wrq[z ? H / 2 : k]));  // e^{+2 pi i k/n} d
+            v[m] = Fx{s.x - w.y, s.y + w.x};
+            Fx u{s.x + w.y, w.x - s.y};
             if (z) {
                 u = v[m];
-                const Fx e{X0.x + X0.y, X0.x - X0.y};
-                v[m] = fx_shr(e, 2, 2);
+                v[m] = Fx{X0.x + X0.y, X0.x - X0.y};
             }
             bits |= fx_bits(v[m].x) | fx_bits(v[m].y) | fx_bits(u.x) | fx_bits(u.y);
             xs[base + pad(partner(m))] = u;
@@ -204,8 +200,8 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
         F::line_sync();
         const int s = fx_norm_shift<58>(bits);
         fx_norm<E>(v, s);
-        // from 61 bits, over 4 twice, and the half of Z
-        ln.ex += -3 + 4 - 1 + s;
+        // from 59 bits (the DCT's from 61, over 4), and the half of Z
+        ln.ex += -1 - 1 + s;
     } else {
 #pragma unroll
         for (int m = 0; m < E; m++) v[m] = Fx{fx_from(d[m].x, ln), fx_from(d[m].y, ln)};
@@ -224,12 +220,12 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
         for (int m = 0; m < E; m++) v[m] = z[m];
     }
     const int nk = fs.k != 0;
-    auto real_out = [&](long long x) -> long long { return nk ? fx_mulk(x, fs.k) : x; };  // over 4 if nk
+    auto real_out = [&](long long x) -> long long { return nk ? fx_mulk_full(x, fs.k) : x; };
     const bool mul = scaled;
     const double f = fx_pre(-ln.pre);
     // ---- output ---------------------------------------------------------
     if constexpr (OP == R2R_RINV) {
-        const int ex = ln.ex + fs.e2 + (nk ? 2 : 0);
+        const int ex = ln.ex + fs.e2;
         double2 r[E];
 #pragma unroll
         for (int m = 0; m < E; m++) r[m] = make_double2(fx_to(real_out(v[m].x), ex), fx_to(real_out(v[m].y), ex));
@@ -253,7 +249,7 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
     }
     if constexpr (F::NPASS > 1) F::line_sync();  // the last exchange is read
     if constexpr (OP == R2R_DCT3) {
-        const int ex = ln.ex + fs.e2 + (nk ? 2 : 0);
+        const int ex = ln.ex + fs.e2;
 #pragma unroll
         for (int m = EH; m < E; m++) xs[base + pad(t + m * TL)] = v[m];
         F::line_sync();
@@ -295,8 +291,10 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
     for (int m = EH; m < E; m++) xs[base + pad(t + m * TL)] = v[m];
     bits = F::template line_red<false>(bits, F::NPASS, c, tid, C, red);
     const int s = fx_norm_shift(bits);
-    // V / 4 with the half of a and d
-    const int ex0 = ln.ex + s + 2 - 1 + (OP == R2R_DCT2 ? 2 : 0), ex = ex0 + fs.e2 + (nk ? 2 : 0);
+    // V doubled, below 2^62 (60 bits before, |A|, |B| below sqrt(2) 2^60): no
+    // division by the last products either.  (Each one's 2 bits made a line with
+    // one large coefficient, as an image's, up to 5 times as far off as FP64.)
+    const int ex0 = ln.ex + s - 1, ex = ex0 + fs.e2;
 #pragma unroll
     for (int m = 0; m < EH; m++) {
         const int k = t + m * TL;
@@ -306,13 +304,13 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
         Fx A = zz[0], B = zz[1];
         if (z) A = B;  // Z_{H/2}; Z_0 below
         const Fx a{A.x + B.x, A.y - B.y}, dd{A.x - B.x, A.y + B.y};
-        const Fx wd = fx_mul<-1>(dd, __ldg(&Wrq[z ? H / 2 : k])), a4 = fx_shr(a, 2, 2);
-        Fx V{a4.x + wd.y, a4.y - wd.x};     // V_k / 4 (doubled), k = 0: V_{H/2}
-        Fx U{a4.x - wd.y, -a4.y - wd.x};    // V_{H-k} / 4
+        const Fx wd = fx_mul_full<-1>(dd, __ldg(&Wrq[z ? H / 2 : k]));
+        Fx V{a.x + wd.y, a.y - wd.x};     // V_k (doubled), k = 0: V_{H/2}
+        Fx U{a.x - wd.y, -a.y - wd.x};    // V_{H-k}
         if (z) {
             U = V;
-            const Fx g = fx_shr(zz[0], 1, 1);  // V_0 = Z_0.x + Z_0.y, V_H = Z_0.x - Z_0.y (doubled)
-            V = Fx{g.x + g.y, g.x - g.y};
+            // V_0 = Z_0.x + Z_0.y, V_H = Z_0.x - Z_0.y (doubled)
+            V = Fx{(zz[0].x + zz[0].y) << 1, (zz[0].x - zz[0].y) << 1};
         }
         long long q0, q1, q2, q3;  // of k, n - k, H - k, H + k (k = 0: 0, 3H/2, H/2, H)
         if constexpr (OP == R2R_DHT) {
@@ -330,21 +328,21 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
             q2 = U.x;
             q3 = U.y;
         } else {
-            const Fx y = fx_mul<-1>(U, __ldg(&Wdq[z ? H / 2 : H - k]));
+            const Fx y = fx_mul_full<-1>(U, __ldg(&Wdq[z ? H / 2 : H - k]));
             q2 = y.x;
             q3 = -y.y;
             if (z) {
-                q0 = (V.x + 2) >> 2;
+                q0 = V.x;
                 q1 = -y.y;
-                q3 = (fx_mulh(V.y) + 2) >> 2;  // C_H = cos(pi/4) V_H
+                q3 = fx_mulh(V.y);  // C_H = cos(pi/4) V_H
             } else {
-                const Fx x = fx_mul<-1>(V, __ldg(&Wdq[k]));
+                const Fx x = fx_mul_full<-1>(V, __ldg(&Wdq[k]));
                 q0 = x.x;
                 q1 = -x.y;
             }
         }
         double r0 = fx_to(real_out(q0), ex), r1 = fx_to(real_out(q1), ex), r2 = fx_to(real_out(q2), ex), r3 = fx_to(real_out(q3), ex);
-        if (OP == R2R_DCT2 && z) r0 = fx_to(fs.k0 ? fx_mulk(q0, fs.k0) : q0, ex0 + fs.e20 + (fs.k0 ? 2 : 0));
+        if (OP == R2R_DCT2 && z) r0 = fx_to(fs.k0 ? fx_mulk_full(q0, fs.k0) : q0, ex0 + fs.e20);
         if (mul) {
             r0 *= f;
             r1 *= f;
