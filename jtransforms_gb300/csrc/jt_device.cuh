@@ -691,20 +691,39 @@ __global__ void __launch_bounds__(512) fft_tile_kernel(const C2 *in, C2 *out, Ti
 // Table generation (FP64, sincospi), rounded to T.
 // ---------------------------------------------------------------------------
 // A root's cosine or sine times 2^62 as two signed halves, high and low (the
-// low half is negated in products: never the lowest int): the factors of
-// jt_fix64.cuh.
-__device__ __forceinline__ int2 fx_split(double c) {
-    long long v = __double2ll_rn(c * 4611686018427387904.0);
+// low half is negated in products: never the lowest int).
+__device__ __forceinline__ int2 fx_split(long long v) {
     if ((int)v == INT32_MIN) v++;
     return make_int2((int)(v >> 32) + (int)((uint32_t)v >> 31), (int)v);
 }
-__device__ __forceinline__ int4 fx_twiddle(double c, double s) {
-    const int2 a = fx_split(c), b = fx_split(s);
-    return make_int4(a.x, a.y, b.x, b.y);
+// e^{-2 pi i num / den}, 0 <= num < den < 2^60, right to a unit or two of 2^-62: the
+// factors of jt_fixmath.cuh.  (Taken from doubles they were 2^-54 off, which the
+// four-step store's powers of one factor multiplied by up to 15: lines of 2^14
+// points were half as far off again as in FP64.)  The angle within its octant
+// is a fraction of pi/4, cosine and sine are their power series to x^20 and
+// x^21, nested, in 64-bit fractions.
+__device__ __forceinline__ int4 fx_root(int64_t num, int64_t den) {
+    const int oct = (int)(8 * num / den);
+    int64_t rem = 8 * num - oct * den;
+    if (oct & 1) rem = den - rem;
+    const unsigned long long f = rem == den ? ~0ull : (unsigned long long)(((unsigned __int128)rem << 64) / (unsigned long long)den);
+    const unsigned long long x = __umul64hi(f, 0xC90FDAA22168C235ull), y = __umul64hi(x, x), one = 1ull << 63;
+    unsigned long long c = one, s = one;
+#pragma unroll
+    for (int k = 10; k >= 1; k--) {
+        c = one - __umul64hi(y, c) / (unsigned)((2 * k - 1) * (2 * k));
+        s = one - __umul64hi(y, s) / (unsigned)((2 * k) * (2 * k + 1));
+    }
+    s = __umul64hi(x, s);
+    const long long a = (long long)((c + 1) >> 1), b = (long long)((s + 1) >> 1);
+    const bool swap = ((oct + 1) >> 1) & 1;  // octants 1, 2, 5, 6
+    const long long co = swap ? b : a, si = swap ? a : b;
+    const int2 u = fx_split(oct >= 2 && oct < 6 ? -co : co), v = fx_split(oct >= 4 ? si : -si);
+    return make_int4(u.x, u.y, v.x, v.y);
 }
 
 // out[t] = e^{-2 pi i t * num / den} for t < count; fixed (double): the same
-// roots as fx_twiddle's after them
+// roots as fx_root's after them
 template <typename T> __global__ void roots_kernel(C2 *out, int64_t count, int64_t num, int64_t den, bool fixed) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= count) return;
@@ -713,7 +732,7 @@ template <typename T> __global__ void roots_kernel(C2 *out, int64_t count, int64
     double s, c;
     sincospi(-2.0 * (double)r / (double)den, &s, &c);
     out[t] = mk<T>((T)c, (T)s);
-    if (sizeof(T) == 8 && fixed) reinterpret_cast<int4 *>(out + count)[t] = fx_twiddle(c, s);
+    if (sizeof(T) == 8 && fixed) reinterpret_cast<int4 *>(out + count)[t] = fx_root(r, den);
 }
 
 // Bluestein chirp bk1[i] = e^{i pi (i^2 mod 2n) / n} (fft/DoubleFFT_1D.java:1864-1879)

@@ -11,7 +11,7 @@
 // passes the line is shifted so that its largest number again has 60 bits.
 // The error of a pass is a fraction of 2^-58 of the line's largest value,
 // below that of the same pass in FP64 (2^-54 of each value); the twiddles are
-// the FP64 tables' own values.  The result is rounded to double once.
+// right to 2^-62 (fx_root).  The result is rounded to double once.
 //
 // Measured (GB300, DoubleFFT_3D(256^3).complexForward and inverse, 268 MB):
 // 888 us where the FP64 passes took 4617; DoubleFFT_1D(4096) x 256, both

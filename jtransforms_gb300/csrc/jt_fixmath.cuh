@@ -22,7 +22,7 @@ __device__ __forceinline__ long long fx_madw(int a, int b, long long c) {
 __device__ __forceinline__ int fx_hi(long long v) { return (int)(v >> 32) + (int)((uint32_t)v >> 31); }
 __device__ __forceinline__ int fx_lo(long long v) { return (int)v; }
 
-// Fixed-point factors w are fx_twiddle's (x, y: cosine's halves; z, w: sine's).
+// Fixed-point factors w are fx_root's (x, y: cosine's halves; z, w: sine's).
 // v w / 4 (SIGN < 0) or v conj(w) / 4, rounded to nearest.  |v| below 2^62.5:
 // the partial sums stay below 2^63.  The low x low product is left out (a
 // quarter of a unit at most).

@@ -17,9 +17,7 @@ __global__ void fixmix_table_kernel(int4 *out, MixParams p, int count) {
     while (ps + 1 < p.npass && idx >= p.toff[ps + 1]) ps++;
     const int r = idx - p.toff[ps], Ns = p.Ns[ps], jm = r % Ns, k = r / Ns + 1;
     const int64_t den = (int64_t)Ns * p.R[ps], num = ((int64_t)jm * k) % den;
-    double s, c;
-    sincospi(-2.0 * (double)num / (double)den, &s, &c);
-    out[idx] = fx_twiddle(c, s);
+    out[idx] = fx_root(num, den);
 }
 
 void fixmix_setup(int smem_optin) {

@@ -103,7 +103,7 @@ __host__ __device__ constexpr int fx_elems(int L) { return L == 64 || L == 512 ?
 // 16-byte pairs each; double tables: factor k as NS entries.  Passes are
 // radix E (elements per thread: 16, or fx_elems) with a last pass of the
 // remaining radix.  Double tables are followed by the same entries in fixed
-// point (int4, fx_twiddle below).
+// point (int4, fx_root).
 // E: elements per thread, 0 for the usual 16.
 __host__ __device__ inline int stock_tw_count(int L, int E = 0) {
     if (E == 0) E = L >= 16 ? 16 : L;
@@ -150,7 +150,7 @@ template <typename T> __global__ void passtw_kernel(typename V2<T>::t *out, int 
                 double s, c;
                 sincospi(-2.0 * (double)num / (double)den, &s, &c);
                 out[idx] = mk<T>((T)c, (T)s);
-                if constexpr (sizeof(T) == 8) reinterpret_cast<int4 *>(out + stock_tw_count(L, E))[idx] = fx_twiddle(c, s);
+                if constexpr (sizeof(T) == 8) reinterpret_cast<int4 *>(out + stock_tw_count(L, E))[idx] = fx_root(num, den);
                 return;
             }
             off += ns * R;

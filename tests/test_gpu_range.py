@@ -104,3 +104,36 @@ def test_packed_real(n, kind):
     G[:, 0], G[:, n // 2] = x[:, 0], x[:, 1]
     G[:, 1:n // 2] = x[:, 2::2] + 1j * x[:, 3::2].astype(CLD)
     _check(dev.cpu().numpy().reshape(B, n).astype(LD), sfft.irfft(G, n, axis=1), n)
+
+
+# one pass, two passes whose columns' outputs take a four-step factor (of 256,
+# 64, 256 and, with mixed radices, 200 points), and three
+@pytest.mark.parametrize("n,passes", [(256, 1), (4096, 1), (8192, 1), (1000, 1), (3000, 1), (1331, 1),
+                                      (1 << 14, 2), (1 << 15, 2), (1 << 18, 2), (50000, 2), (1 << 23, 3)])
+def test_impulses(n, passes):
+    """An impulse of 1 at j has the roots e^{-2 pi i jk/n} themselves as its
+    spectrum. A pass over memory rounds each part to a double, 2^-54 at most,
+    and the passes after it turn that error, which makes it sqrt(2) of that at
+    most. All else stays below 2^-55: twiddles are right to 2^-62, butterflies
+    round at 2^-58, four-step factors, powers of one, add 15 units of 2^-60."""
+    bound = (1 + np.sqrt(2) * (passes - 1)) * 2.0 ** -54 + 2.0 ** -55
+    import torch
+    import jtransforms_gb300 as J
+    from jtransforms_gb300 import _native as N
+    rows = B if n < 1 << 20 else 1
+    j = np.random.default_rng(n).integers(0, n, rows)
+    z = np.zeros((rows, n), np.complex128)
+    z[np.arange(rows), j] = 1
+    dev = torch.from_numpy(z.view(np.float64).ravel()).cuda()
+    J.DoubleFFT_1D(n).plan.execute(N.COMPLEX_FORWARD, dev, 0, False, batch=rows, dist=2 * n)
+    got = dev.cpu().numpy().view(np.complex128).reshape(rows, n)
+    for g, at in zip(got, j):
+        # eighths of a turn and a rest, so that the argument is exact
+        r = (int(at) * np.arange(n)) % n
+        o = (8 * r + n // 2) // n
+        t = (8 * r - o * n).astype(LD) / LD(4 * n) * LD("3.14159265358979323846264338327950288")
+        c, s, h = np.cos(t), np.sin(t), np.sqrt(LD(0.5))
+        co = np.array([1, h, 0, -h, -1, -h, 0, h, 1], LD)[o]
+        si = np.array([0, h, 1, h, 0, -h, -1, -h, 0], LD)[o]
+        assert np.abs(g.real - (co * c - si * s)).max() <= bound
+        assert np.abs(g.imag + (si * c + co * s)).max() <= bound
