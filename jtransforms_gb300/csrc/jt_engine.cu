@@ -2335,12 +2335,13 @@ template <typename T> struct PlanImpl {
             double mult = (!fwd && scale) ? 1.0 / (double)dims[0] : 1.0;
             return h->lines(ctx, a, batch, Layout{1, dist, 0, 1}, mult);
         }
-        // the inverse's 1/N rides on the last axis
+        // the inverse's 1/N and the half of 3D arrays' joining step ride on the last axis
+        const double last = (nd == 3 ? 0.5 : 1.0) * (!fwd && scale ? 1.0 / (double)N : 1.0);
         int left = nd;
         JT_TRY(real_axes(
             ctx, a, batch,
             [&](Ctx &c, int64_t len, T *x, int64_t nb, const Layout &l) {
-                return dht.at(len)->lines(c, x, nb, l, --left == 0 && !fwd && scale ? 1.0 / (double)N : 1.0);
+                return dht.at(len)->lines(c, x, nb, l, --left == 0 ? last : 1.0);
             },
             [&](int64_t len) { return dht.at(len)->strided_ok(ctx); }));
         for (int64_t b = 0; b < batch; b++) {
