@@ -154,14 +154,26 @@ __global__ void __launch_bounds__(JT_BATCH_THREADS, sizeof(T) == 4 ? 3 : 2)
     }
 }
 
-// Blocks per SM with `smem` bytes each; sets the kernel of prec (0: float, 1:
-// double) up for them.
-cudaError_t batch_setup(int prec, int smem, int *per_sm) {
-    const void *k = prec == 0 ? (const void *)batch_kernel<float> : (const void *)batch_kernel<double>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, JT_BATCH_THREADS, smem);
-    return e;
+static const void *batch_function(int prec) {
+    return prec == 0 ? (const void *)batch_kernel<float> : (const void *)batch_kernel<double>;
+}
+// Once per process: both kernels may take the most there is. (Set to what one
+// batch needs, it was too little for another made before.)
+cudaError_t batch_setup(int smem_optin) {
+    for (int prec = 0; prec < 2; prec++) {
+        const void *k = batch_function(prec);
+        cudaFuncAttributes at;
+        cudaError_t e = cudaFuncGetAttributes(&at, k);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - (int)at.sharedSizeBytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+// Blocks per SM of the kernel of prec (0: float, 1: double) with `smem` bytes each.
+cudaError_t batch_occupancy(int prec, int smem, int *per_sm) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, batch_function(prec), JT_BATCH_THREADS, smem);
 }
 
 void batch_launch(int prec, const BOp *ops, const BTask *tasks, int ntasks, int *head, int *done, int *err, int wait_polls, int grid,

@@ -201,7 +201,8 @@ void fixmix_table(int4 *out, const MixParams &p, int count, cudaStream_t s);
 void fixmix_launch(const double2 *in, double2 *out, const FixMixParams &p, unsigned grid, int threads, size_t smem, cudaStream_t s);
 
 // The batch kernel (jt_batch.cu).
-cudaError_t batch_setup(int prec, int smem, int *per_sm);
+cudaError_t batch_setup(int smem_optin);
+cudaError_t batch_occupancy(int prec, int smem, int *per_sm);
 void batch_launch(int prec, const BOp *ops, const BTask *tasks, int ntasks, int *head, int *done, int *err, int wait_polls, int grid,
                   int smem, cudaStream_t s);
 
@@ -242,6 +243,7 @@ static int device_init() {
         mix_setup_inv(g_smem_optin);
         blue_setup(g_smem_optin);
         fixmix_setup(g_smem_optin);
+        if (batch_setup(g_smem_optin) != cudaSuccess) g_dev_status = JT_ECUDA;
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DCT3, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
         cudaFuncSetAttribute(r2r_tile_kernel<R2R_DHT, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin);
@@ -3195,7 +3197,7 @@ int jt_batch_create(int count, jt_plan *const *plans, const int *ops, void *cons
             for (int o : c) b->smem[prec] = std::max(b->smem[prec], std::max(rec[o].smem, 1));
         if (mine.empty()) continue;
         int per_sm = 0;
-        JT_CU(batch_setup(prec, b->smem[prec], &per_sm));
+        JT_CU(batch_occupancy(prec, b->smem[prec], &per_sm));
         b->grid[prec] = std::max(1, per_sm) * g_sms;
         batch_order(rec, mine, b->grid[prec], tasks);
         b->ntasks[prec] = (int)(tasks.size() - before);
