@@ -2065,16 +2065,21 @@ template <typename T> struct PlanImpl {
 
     // Builds (or takes from the cache) every table `op` needs, under the
     // mutex; when anything was built, waits for the setup stream.
-    int prepare(int op) {
+    int prepare(int op, cudaStream_t s = nullptr) {
         const uint64_t seq0 = g_setup_seq.load();
-        int st = prepare_locked(op);
+        int st = prepare_locked(op, s);
         if (st == JT_OK && g_setup_seq.load() != seq0) {
             JT_CU(cudaStreamSynchronize(g_setup));
             JT_CU(cudaGetLastError());
         }
         return st;
     }
-    int prepare_locked(int op) {
+    static bool capturing(cudaStream_t s) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &st) != cudaSuccess) cudaGetLastError();
+        return st != cudaStreamCaptureStatusNone;
+    }
+    int prepare_locked(int op, cudaStream_t s) {
         std::lock_guard<std::mutex> g(mu);
         Fft1<T> *f;
         Real1<T> *r;
@@ -2092,7 +2097,10 @@ template <typename T> struct PlanImpl {
                 JT_TRY(get_fft(dims[1], &f));
                 return get_fft(dims[0], &f);
             }
-            if (nd > 1 && (op == JT_REAL_FORWARD_FULL || op == JT_REAL_INVERSE_FULL) && dims[nd - 1] % 2 == 0)
+            // (no tables can be built while the stream is captured: a plan whose
+            // first full spectrum is captured runs the complex transform)
+            if (nd > 1 && (op == JT_REAL_FORWARD_FULL || op == JT_REAL_INVERSE_FULL) && dims[nd - 1] % 2 == 0 &&
+                (real.count(dims[nd - 1]) || !capturing(s)))
                 JT_TRY(get_real(dims[nd - 1], &r));
             for (int a = 0; a < nd; a++) JT_TRY(get_fft(dims[a], &f));
             return JT_OK;
@@ -2262,7 +2270,7 @@ template <typename T> struct PlanImpl {
                 case JT_COMPLEX_INVERSE: return complex_nd(ctx, (C2 *)a, batch, 1, scale);
                 case JT_REAL_FORWARD_FULL:
                 case JT_REAL_INVERSE_FULL: {
-                    if (dims[nd - 1] % 2 == 0)
+                    if (dims[nd - 1] % 2 == 0 && real.count(dims[nd - 1]))
                         return real_full_nd(ctx, a, batch, op == JT_REAL_FORWARD_FULL ? -1 : 1, op == JT_REAL_INVERSE_FULL && scale);
                     T *tmp = (T *)ctx.ws->get(sizeof(T) * batch * N, ctx.dry);
                     LAUNCH1D(ctx, batch * N, copy_real_kernel<T>, a, dist, tmp, N, N, batch);
@@ -2466,7 +2474,7 @@ int check_err_flag() {
 template <typename T>
 int run_device(jt_plan *p, int op, T *a, int64_t batch, int64_t dist, bool scale, cudaStream_t s) {
     PlanImpl<T> *im = impl_of<T>(p);
-    JT_TRY(im->prepare(op));
+    JT_TRY(im->prepare(op, s));
     Ctx c;
     c.s = s;
     c.tc = p->mode == JT_MODE_TC_SPLIT;
