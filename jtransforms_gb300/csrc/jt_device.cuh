@@ -520,27 +520,15 @@ __device__ void fx_pass_generic(const Fx *src, Fx *dst, int lines, int L, int Lp
     }
 }
 
-// Doubles in `src` to doubles in the returned buffer.  `words`: JT_FX_WORDS
-// per line; Wq: the roots in fixed point.  Tiles with an infinity or a NaN run
-// tile_passes_fp.
+// `lines` finite lines of doubles in `src` to doubles in the returned buffer.
+// Wq: the roots in fixed point.  words: each line's largest number, zero and
+// three more (JT_FX_WORDS), each `ws` words apart.
 template <int SIGN>
-__device__ __noinline__ double2 *tile_passes_fx(double2 *src, double2 *dst, int lines, int L, int Lp, int npass, const int *radix,
-                                                const double2 *__restrict__ W, uint32_t *words) {
-    const int4 *Wq = reinterpret_cast<const int4 *>(W + L);
-    uint32_t *b0 = words, *b1 = words + lines, *b2 = words + 2 * lines;
-    int *ex = reinterpret_cast<int *>(words + 3 * lines), *pre = ex + lines;
+__device__ __forceinline__ double2 *tile_lines_fx(double2 *src, double2 *dst, int lines, int L, int Lp, int npass, const int *radix,
+                                                  const int4 *__restrict__ Wq, uint32_t *words, int ws) {
+    uint32_t *b0 = words, *b1 = words + ws, *b2 = words + 2 * ws;
+    int *ex = reinterpret_cast<int *>(words + 3 * ws), *pre = ex + ws;
     const int tid = threadIdx.x, nt = blockDim.x, tot = lines * L;
-    for (int c = tid; c < lines; c += nt) b0[c] = b1[c] = 0;
-    __syncthreads();
-    bool special = false;
-    for (int i = tid; i < tot; i += nt) {
-        const int c = i / L;
-        const double2 d = src[c * Lp + pad(i - c * L)];
-        const uint32_t m = max((uint32_t)__double2hiint(d.x) << 1, (uint32_t)__double2hiint(d.y) << 1);
-        special |= m >= 0xffe00000u;
-        fx_join<true>(b0, c, m);
-    }
-    if (__syncthreads_or(special)) return tile_passes_fp<SIGN, double>(src, dst, lines, L, Lp, npass, radix, W);
     const int low = fx_generic(radix[0]) ? fx_room(radix[0]) - 2 : 0;  // against 58 bits
     for (int c = tid; c < lines; c += nt) {
         const FxLine l = fx_line(b0[c]);
@@ -595,6 +583,35 @@ __device__ __noinline__ double2 *tile_passes_fx(double2 *src, double2 *dst, int 
         r[at] = y;
     }
     __syncthreads();
+    return r;
+}
+
+// Doubles in `src` to doubles in the returned buffer.  `words`: JT_FX_WORDS
+// per line.  A line with an infinity or a NaN runs tile_passes_fp; its tile
+// then goes line by line, so that no finite line's result depends on it.
+template <int SIGN>
+__device__ __noinline__ double2 *tile_passes_fx(double2 *src, double2 *dst, int lines, int L, int Lp, int npass, const int *radix,
+                                                const double2 *__restrict__ W, uint32_t *words) {
+    const int tid = threadIdx.x, nt = blockDim.x, tot = lines * L;
+    for (int c = tid; c < 2 * lines; c += nt) words[c] = 0;
+    __syncthreads();
+    bool special = false;
+    for (int i = tid; i < tot; i += nt) {
+        const int c = i / L;
+        const double2 d = src[c * Lp + pad(i - c * L)];
+        const uint32_t m = max((uint32_t)__double2hiint(d.x) << 1, (uint32_t)__double2hiint(d.y) << 1);
+        special |= m >= 0xffe00000u;
+        fx_join<true>(words, c, m);
+    }
+    const bool one = __syncthreads_or(special);
+    const int step = one ? 1 : lines;
+    double2 *r = src;
+    for (int c = 0; c < lines; c += step) {
+        double2 *s = src + c * Lp, *d = dst + c * Lp;
+        r = one && words[c] >= 0xffe00000u ? tile_passes_fp<SIGN, double>(s, d, 1, L, Lp, npass, radix, W)
+                                           : tile_lines_fx<SIGN>(s, d, step, L, Lp, npass, radix, reinterpret_cast<const int4 *>(W + L), words + c, lines);
+        r -= c * Lp;
+    }
     return r;
 }
 

@@ -751,9 +751,10 @@ template <typename T> struct Fft1 {
         p.m.C = C;
         p.m.mC = C > 1 ? (uint32_t)(((uint64_t)1 << 32) / (uint64_t)C + 1) : 0;
     }
-    // shared memory of C lines: their buffers and words, or one line's FP64 tile
+    // shared memory of C lines: their buffers, or one line's FP64 tile, and words
     size_t fixmix_smem(int C) const {
-        return std::max(((size_t)mix.Lp * sizeof(C2) * (mix.npass > 2 ? 2 : 1) + tile_words<T>()) * C, 2 * (size_t)padded_len((int)n) * sizeof(C2));
+        return std::max((size_t)mix.Lp * sizeof(C2) * (mix.npass > 2 ? 2 : 1) * C, 2 * (size_t)padded_len((int)n) * sizeof(C2)) +
+               tile_words<T>() * C;
     }
 
     // Line pass of the doubles' mixed-radix kernel.  C lines per CTA: a first

@@ -24,7 +24,7 @@
 // with four CTAs of 128 registers a thread per SM.
 //
 // Range: lines whose largest exponent leaves no room (below 2^-900 or above
-// 2^900) are scaled by 2^+-512 around the transform, which is exact; a tile
+// 2^900) are scaled by 2^+-512 around the transform, which is exact; a line
 // with an infinity or a NaN runs the FP64 passes of jt_stockham.cuh, so those
 // spread as they always did.
 #pragma once
@@ -158,6 +158,35 @@ template <int L, int MODE, int SIGN, int CM> struct FxStock {
     }
 };
 
+// The tile's lines with an infinity or a NaN (`bad`: the thread's line b is one)
+// by the FP64 passes, after the others: a finite line's result does not depend
+// on its neighbours.
+template <int L, int MODE, int SIGN, bool TW>
+__device__ __noinline__ void fix_fp64_lines(const double2 *in, double2 *out, const StockParams &p, const double2 *W, const double2 *Whi,
+                                            const double2 *Wlo, int64_t b, int t, int c, bool bad, unsigned char *smem) {
+    typedef FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)> F;
+    typedef typename F::S S;
+    if (!bad) b = 0;
+    const double2 *src = in + line_off(p.lin, b);
+    double2 *dst = out + line_off(p.lout, b);
+    double2 d[F::E];
+#pragma unroll
+    for (int m = 0; m < F::E; m++) d[m] = bad ? src[(t + m * F::TL) * p.lin.estride] : make_double2(0, 0);
+    int64_t j2 = 0;
+    if constexpr (TW) div_fast(b, p.tw_inner, &j2);
+    auto store = [&](int pos, double2 val, int) {
+        if (TW) {
+            const double2 w = tw_lookup<double>(Whi, Wlo, (uint32_t)pos * (uint32_t)j2, p);
+            val = SIGN < 0 ? cmul<double>(val, w) : cmulc<double>(val, w);
+        }
+        if (p.do_scale) val = cscale<double>(val, p.scale);
+        if (bad) dst[(int64_t)pos * p.lout.estride] = val;
+    };
+    PadIdx xi{c * S::LP};
+    __syncthreads();  // the exchange buffer
+    S::run_all(d, t, reinterpret_cast<double2 *>(smem), xi, W, store);
+}
+
 // One tile of C = blockDim / TL lines per CTA (several CTAs share an SM:
 // their loads overlap each other's arithmetic).
 template <int L, int MODE, int SIGN, bool TW>
@@ -220,20 +249,15 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::NT,
     int64_t j2l = 0;
     if constexpr (TW) div_fast(valid ? b : 0, p.tw_inner, &j2l);
     const uint32_t j2 = (uint32_t)j2l;
-    if (fp) {
-        auto store = [&](int pos, double2 val, int) {
-            if (TW) {
-                const double2 w = tw_lookup<double>(Whi, Wlo, (uint32_t)pos * j2, p);
-                val = SIGN < 0 ? cmul<double>(val, w) : cmulc<double>(val, w);
-            }
-            if (p.do_scale) val = cscale<double>(val, p.scale);
-            if (valid) st_hint(&dst[(int64_t)pos * oes], val, spol);
-        };
-        PadIdx xi{c * S::LP};
-        S::run_all(d, t, reinterpret_cast<double2 *>(smem_raw), xi, W, store);
-        return;
-    }
     if constexpr (!F::WARP_LINE) mx = red[c];
+    bool keep = valid;
+    if (fp && mx >= 0xffe00000u) {
+        // goes through the passes as zeros that are not stored
+        mx = 0;
+        keep = false;
+#pragma unroll
+        for (int m = 0; m < F::E; m++) d[m] = make_double2(0, 0);
+    }
     FxLine ln = fx_line(mx);
     if (__any_sync(0xffffffffu, ln.pre != 0)) {
         const double f = fx_pre(ln.pre);
@@ -288,12 +312,13 @@ __global__ void __launch_bounds__(FxStock<L, MODE, SIGN, FxCfg::C(L, MODE)>::NT,
 #pragma unroll
             for (int k = 0; k < LP_::R; k++) r[k] = cscale<double>(r[k], f);
         }
-        if (valid) {
+        if (keep) {
 #pragma unroll
             for (int k = 0; k < LP_::R; k++) st_hint(&dst[(int64_t)(pos + k * LP_::NS) * oes], r[k], spol);
         }
     };
     F::template run<0>(v, t, c, tid, C, xs, Wq, red, ln, store);
+    if (fp) fix_fp64_lines<L, MODE, SIGN, TW>(in, out, p, W, Whi, Wlo, b, t, c, valid && !keep, smem_raw);
 }
 
 // Lines per CTA: the most that fit, halved while the grid has fewer CTAs than

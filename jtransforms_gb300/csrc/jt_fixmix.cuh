@@ -5,8 +5,8 @@
 // The first pass takes one butterfly per thread: its numbers wait in
 // registers as doubles until the line's largest exponent is known.  Inverse
 // transforms exchange real and imaginary parts on the way in and out, so the
-// passes exist once.  Tiles with an infinity or a NaN run the FP64 passes of
-// jt_device.cuh, line by line.
+// passes exist once.  Lines with an infinity or a NaN run the FP64 passes of
+// jt_device.cuh.
 //
 // Measured (GB300, one direction, FP64 tile passes before): 2 M points of n =
 // 1000 55 us (185), of 96 39 (105), of 3000 73 (228); one transform of n = 1000
@@ -22,6 +22,7 @@ namespace jt {
 
 #define JT_FIXMIX_RADICES(X) X(2) X(3) X(4) X(5) X(7) X(8) X(9) X(10) X(12) X(15) X(16)
 #define JT_FIXMIX_THREADS 512
+#define JT_FX_SPECIAL (1 << 20)  // in the place of a line's scaling (FxLine::pre): an infinity or a NaN among its numbers
 
 struct FixMixParams {
     MixParams m;          // Lp: line stride; tables: factor k of a pass as Ns entries
@@ -111,8 +112,9 @@ struct FixMixTile {
 
     __device__ __forceinline__ int at(int c, int i) const { return c * p.m.Lp + i + (i >> p.psh); }
 
-    // Pass ps.  bin, bout: the lines' bits before and after it.  Returns false
-    // (FIRST) if a value is not finite.
+    // Pass ps.  bin, bout: the lines' bits before and after it.  FIRST: returns
+    // whether a value is not finite; the lines of such values are marked and
+    // go through the passes as zeros that are not stored.
     template <int R, bool FIRST, bool LAST>
     __device__ __forceinline__ bool pass(int ps, const Fx *src, Fx *dst, uint32_t *bin, uint32_t *bout) const {
         const MixParams &m = p.m;
@@ -121,6 +123,7 @@ struct FixMixTile {
         const int total = (cols ? C : lines) * nb;
         const int4 *tw = p.tw + m.toff[ps];
         int *ex = reinterpret_cast<int *>(words + 3 * C), *pre = ex + C;
+        bool found = false;
         for (int q = threadIdx.x; FIRST || q < total; q += blockDim.x) {
             int c, j;
             if (cols) {
@@ -147,9 +150,15 @@ struct FixMixTile {
                 for (int k = 0; k < R; k++)
                     mx = max(mx, max((uint32_t)__double2hiint(d[k].x) << 1, (uint32_t)__double2hiint(d[k].y) << 1));
                 if (ok) fx_join<true>(bin, c, mx);
-                if (__syncthreads_or(mx >= 0xffe00000u)) return false;
-                if (!ok) return true;
-                const FxLine l = fx_line(bin[c]);
+                const bool special = __syncthreads_or(mx >= 0xffe00000u);
+                if (!ok) return special;
+                FxLine l = fx_line(bin[c]);
+                if (special && bin[c] >= 0xffe00000u) {
+                    l = FxLine{0, JT_FX_SPECIAL};
+#pragma unroll
+                    for (int k = 0; k < R; k++) d[k] = make_double2(0, 0);
+                }
+                found = special;
                 if (j == 0) {
                     ex[c] = l.ex;
                     pre[c] = l.pre;
@@ -214,8 +223,10 @@ struct FixMixTile {
 #pragma unroll
                     for (int k = 0; k < R; k++) r[k] = cscale<double>(r[k], f);
                 }
+                if (pre[c] != JT_FX_SPECIAL) {
 #pragma unroll
-                for (int k = 0; k < R; k++) g[k * step] = p.inv ? make_double2(r[k].y, r[k].x) : r[k];
+                    for (int k = 0; k < R; k++) g[k * step] = p.inv ? make_double2(r[k].y, r[k].x) : r[k];
+                }
             } else {
                 uint32_t bits = 0;
 #pragma unroll
@@ -225,9 +236,9 @@ struct FixMixTile {
                 }
                 fx_join<false>(bout, c, bits);
             }
-            if (FIRST) return true;
+            if (FIRST) return found;
         }
-        return true;
+        return false;
     }
 
     template <bool FIRST, bool LAST> __device__ __forceinline__ bool any(int ps, const Fx *src, Fx *dst, uint32_t *bin, uint32_t *bout) const {
@@ -237,17 +248,18 @@ struct FixMixTile {
             JT_FIXMIX_RADICES(JT_FIXMIX)
 #undef JT_FIXMIX
         }
-        return true;
+        return false;
     }
 
     // At least two passes, through the buffers A and B (B for three and more).
+    // Returns whether lines are left for the FP64 passes.
     __device__ __forceinline__ bool run(Fx *A, Fx *B) const {
         const int C = p.m.C;
         uint32_t *b0w = words, *b1w = words + C, *b2w = words + 2 * C;
         int *ex = reinterpret_cast<int *>(words + 3 * C);
         for (int c = threadIdx.x; c < C; c += blockDim.x) b0w[c] = b1w[c] = 0;
         __syncthreads();
-        if (!any<true, false>(0, nullptr, A, b0w, b1w)) return false;
+        const bool special = any<true, false>(0, nullptr, A, b0w, b1w);
         auto next = [&] {
             uint32_t *t = b0w;
             b0w = b1w;
@@ -267,26 +279,30 @@ struct FixMixTile {
         }
         __syncthreads();
         any<false, true>(p.m.npass - 1, A, nullptr, b0w, nullptr);
-        return true;
+        return special;
     }
 };
 
+// The marked lines (pre: their marks, beyond the buffers that this uses)
 static __device__ __noinline__ void fixmix_fp64(const double2 *in, double2 *out, const FixMixParams &p, int64_t b0, int lines,
-                                                unsigned char *smem) {
+                                                const int *pre, unsigned char *smem) {
     for (int l = 0; l < lines; l++) {
+        if (pre[l] != JT_FX_SPECIAL) continue;
         __syncthreads();
         if (p.inv) tile_fft_body<1, double, true>(in, out, p.fp, p.W, p.Whi, p.Wlo, b0 + l, smem);
         else tile_fft_body<-1, double, true>(in, out, p.fp, p.W, p.Whi, p.Wlo, b0 + l, smem);
     }
 }
 
-// Tile `blk`, at smem_raw: one or two buffers of C lines and their words.
+// Tile `blk`, at smem_raw: one or two buffers of C lines (room for one line's
+// FP64 passes at least) and their words.
 __device__ __forceinline__ void fixmix_body(const double2 *in, double2 *out, const FixMixParams &p, int64_t blk, unsigned char *smem_raw) {
     const int64_t b0 = blk * p.m.C;
     const int lines = (int)min((int64_t)p.m.C, p.m.nlines - b0), nbuf = p.m.npass > 2 ? 2 : 1;
     Fx *A = reinterpret_cast<Fx *>(smem_raw);
-    uint32_t *words = reinterpret_cast<uint32_t *>(A + nbuf * p.m.C * p.m.Lp);
-    if (!FixMixTile{in, out, p, b0, lines, words}.run(A, A + p.m.C * p.m.Lp)) fixmix_fp64(in, out, p, b0, lines, smem_raw);
+    uint32_t *words = reinterpret_cast<uint32_t *>(A + max(nbuf * p.m.C * p.m.Lp, 2 * padded_len(p.m.L)));
+    if (FixMixTile{in, out, p, b0, lines, words}.run(A, A + p.m.C * p.m.Lp))
+        fixmix_fp64(in, out, p, b0, lines, reinterpret_cast<const int *>(words + 4 * p.m.C), smem_raw);
 }
 
 }  // namespace jt

@@ -46,25 +46,35 @@ template <int H, int MODE, int OP> struct FixR2r {
     typedef FxStock<H, MODE, SIGN, CM> F;
 };
 
-// The FP64 form of the calling CTA's lines (its p.C and threads).
+// The FP64 form of the calling CTA's lines with an infinity or a NaN (marks),
+// one at a time, after the others: a finite line's result does not depend on
+// its neighbours.
 template <int H, int OP>
 __device__ __noinline__ void fix_r2r_fp64(const double *in, double *out, const R2rParams &p, const double2 *Wp, const double2 *Wr,
-                                          const double2 *Wd, unsigned char *smem) {
-    r2r_reg_body<double, H, OP, fx_elems(H)>(in, out, p, Wp, Wr, Wd, smem);
+                                          const double2 *Wd, const bool *marks, unsigned char *smem) {
+    const int64_t b0 = (int64_t)blockIdx.x * p.C;
+    const int lines = (int)min((int64_t)p.C, p.nlines - b0);
+    R2rParams q = p;
+    q.nlines = b0 + 1;  // one line, in the place of the CTA's first
+    __syncthreads();
+    for (int l = 0; l < lines; l++) {
+        if (!marks[l]) continue;
+        r2r_reg_body<double, H, OP, fx_elems(H)>(in + (line_off(p.lin, b0 + l) - line_off(p.lin, b0)),
+                                                 out + (line_off(p.lout, b0 + l) - line_off(p.lout, b0)), q, Wp, Wr, Wd, smem);
+        __syncthreads();
+    }
 }
 
+// The finite lines of the calling CTA; returns whether others are left (marks).
 template <int H, int MODE, int OP>
-__global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP>::F::MINB)
-    fix_r2r_kernel(const double *in, double *out, R2rParams p, FixR2rScale fs, const double2 *__restrict__ Wp,
-                   const double2 *__restrict__ Wr, const double2 *__restrict__ Wd, const int4 *__restrict__ Wpq,
-                   const int4 *__restrict__ Wrq, const int4 *__restrict__ Wdq) {
+__device__ __forceinline__ bool fix_r2r_lines(const double *in, double *out, const R2rParams &p, const FixR2rScale &fs,
+                                              const int4 *__restrict__ Wpq, const int4 *__restrict__ Wrq,
+                                              const int4 *__restrict__ Wdq, bool *marks, unsigned char *smem_raw) {
     typedef typename FixR2r<H, MODE, OP>::F F;
     typedef typename F::S S;
     constexpr int n = 2 * H, TL = F::TL, E = F::E, EH = E / 2;
     auto pad = [](int i) { return F::pad(i); };
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t red[F::RED];
-    pdl_begin();
     Fx *xs = reinterpret_cast<Fx *>(smem_raw);
     double2 *xd = reinterpret_cast<double2 *>(smem_raw);
     const int tid = threadIdx.x, NT = blockDim.x, C = NT / TL;
@@ -137,14 +147,22 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
         __syncthreads();  // red is zeroed
         if (MODE == 0 ? tid % 32 == 0 : tid % 32 < C) atomicMax(&red[c], mx);
     }
-    if (__syncthreads_or(special)) {
-        fix_r2r_fp64<H, OP>(in, out, p, Wp, Wr, Wd, smem_raw);
-        return;
-    }
+    const bool fp = __syncthreads_or(special);
     if constexpr (!F::WARP_LINE) mx = red[c];
     if constexpr (OP == R2R_DCT2) {
 #pragma unroll
         for (int m = EH; m < E; m++) d[m] = xd[base + pad(t + m * TL)];
+    }
+    bool keep = valid;
+    if (fp) {
+        if (t == 0) marks[c] = mx >= 0xffe00000u;
+        if (mx >= 0xffe00000u) {
+            // goes through the passes as zeros that are not stored
+            mx = 0;
+            keep = false;
+#pragma unroll
+            for (int m = 0; m < E; m++) d[m] = make_double2(0, 0);
+        }
     }
     FxLine ln = fx_line(mx);
     const bool scaled = __any_sync(0xffffffffu, ln.pre != 0);
@@ -233,7 +251,7 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
 #pragma unroll
             for (int m = 0; m < E; m++) r[m] = cscale<double>(r[m], f);
         }
-        if (valid) {
+        if (keep) {
 #pragma unroll
             for (int m = 0; m < E; m++) {
                 const int i = 2 * (t + m * TL);
@@ -245,7 +263,7 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
                 }
             }
         }
-        return;
+        return fp;
     }
     if constexpr (F::NPASS > 1) F::line_sync();  // the last exchange is read
     if constexpr (OP == R2R_DCT3) {
@@ -269,7 +287,7 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
                 r2 *= f;
                 r3 *= f;
             }
-            if (valid) {
+            if (keep) {
                 if (vec_out) {
                     *reinterpret_cast<double2 *>(dst + 4 * k) = make_double2(r0, r1);
                     *reinterpret_cast<double2 *>(dst + 4 * k + 2) = make_double2(r2, r3);
@@ -282,7 +300,7 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
                 }
             }
         }
-        return;
+        return fp;
     }
     uint32_t bits = 0;
 #pragma unroll
@@ -349,7 +367,7 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
             r2 *= f;
             r3 *= f;
         }
-        if (!valid) continue;
+        if (!keep) continue;
         if constexpr (OP == R2R_RFWD) {
             const int i = 2 * k, j = 2 * partner(m);
             if (vec_out) {
@@ -370,6 +388,19 @@ __global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP
             put(H + k, r3);
         }
     }
+    return fp;
+}
+
+template <int H, int MODE, int OP>
+__global__ void __launch_bounds__(FixR2r<H, MODE, OP>::F::NT, FixR2r<H, MODE, OP>::F::MINB)
+    fix_r2r_kernel(const double *in, double *out, R2rParams p, FixR2rScale fs, const double2 *__restrict__ Wp,
+                   const double2 *__restrict__ Wr, const double2 *__restrict__ Wd, const int4 *__restrict__ Wpq,
+                   const int4 *__restrict__ Wrq, const int4 *__restrict__ Wdq) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ bool marks[FixR2r<H, MODE, OP>::CM];
+    pdl_begin();
+    if (fix_r2r_lines<H, MODE, OP>(in, out, p, fs, Wpq, Wrq, Wdq, marks, smem_raw))
+        fix_r2r_fp64<H, OP>(in, out, p, Wp, Wr, Wd, marks, smem_raw);
 }
 
 // Launches one (H, op); strided lines up to H = 2048 (longer ones would move
