@@ -82,7 +82,7 @@ template <bool ONE> struct BlueTile {
                 base -= jm * (R - 1);
                 mix_twiddle<R, SIGN>(v, tw, Ns, jm);
             }
-            dft_any<R, SIGN, float>(v);
+            dft_any<R, SIGN, float, true>(v);
             if (TURN) {
                 // v[k]: spectrum number j + k nb; the inverse's first pass has no twiddles
                 int64_t row = 0;
@@ -93,7 +93,7 @@ template <bool ONE> struct BlueTile {
                     const float2 w = __ldg(B + k * nb);
                     v[k] = q.bl.inv ? cmulc<float>(v[k], w) : cmul<float>(v[k], w);
                 }
-                dft_any<R, 1, float>(v);
+                dft_any<R, 1, float, true>(v);
                 base = j * R;
             }
             if (LAST) {
