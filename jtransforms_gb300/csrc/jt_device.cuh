@@ -848,6 +848,40 @@ __device__ __forceinline__ void real_split(C2 zk, C2 zh, C2 w, C2 &xk) {
     xk = mk<T>(a.x + wd.y, a.y - wd.x);  // a - i * wd
 }
 
+// x + y and what its rounding left out
+__device__ __forceinline__ float2 two_sum(float x, float y) {
+    const float s = __fadd_rn(x, y), t = __fsub_rn(s, x);
+    return make_float2(s, __fadd_rn(__fsub_rn(x, __fsub_rn(s, t)), __fsub_rn(y, t)));
+}
+// The split of a pair: X_k and X_{h-k} = conj(a + i w d) of half-length spectra
+// (a, d = Z_k +- conj Z_{h-k}), times s / 2.  Floats carry the roundings of the
+// sums and products along: rounded one by one they made a full spectrum from
+// half-length rows a few percent further off than the complex transform.
+__device__ __forceinline__ void real_split_pair(float2 zk, float2 zh, float2 w, float s, float2 &xk, float2 &xh) {
+    const float2 ax = two_sum(zk.x, zh.x), ay = two_sum(zk.y, -zh.y), dx = two_sum(zk.x, -zh.x), dy = two_sum(zk.y, zh.y);
+    // wd.x = w.x d.x - w.y d.y, wd.y = w.x d.y + w.y d.x as sums of two floats
+    auto dot = [](float a, float2 x, float b, float2 y) {
+        const float p = __fmul_rn(a, x.x), q = __fmul_rn(b, y.x);
+        const float2 t = two_sum(p, q);
+        const float e = fmaf(a, x.x, -p) + fmaf(b, y.x, -q) + t.y;
+        return make_float2(t.x, fmaf(a, x.y, fmaf(b, y.y, e)));
+    };
+    const float2 u = dot(w.x, dx, -w.y, dy), v = dot(w.x, dy, w.y, dx);
+    auto add = [&](float2 a, float2 b) {
+        const float2 t = two_sum(a.x, b.x);
+        return 0.5f * s * (t.x + (t.y + (a.y + b.y)));
+    };
+    auto neg = [](float2 a) { return make_float2(-a.x, -a.y); };
+    xk = make_float2(add(ax, v), add(ay, neg(u)));
+    xh = make_float2(add(ax, neg(v)), -add(ay, u));
+}
+__device__ __forceinline__ void real_split_pair(double2 zk, double2 zh, double2 w, double s, double2 &xk, double2 &xh) {
+    real_split<double>(zk, zh, w, xk);
+    real_split<double>(zh, zk, make_double2(-w.x, w.y), xh);
+    xk = cscale<double>(xk, s);
+    xh = cscale<double>(xh, s);
+}
+
 // In place: a holds Z (h complex); writes the packed realForward layout.
 template <typename T>
 __device__ __forceinline__ void real_post_packed_body(T *a, int64_t dist, int64_t n, int64_t batch, const C2 *__restrict__ Wr, int64_t idx) {
@@ -901,13 +935,10 @@ __device__ __forceinline__ void real_post_full_body(const T *zin, int64_t zdist,
     C2 w = __ldg(&Wr[k]);
     if (SIGN > 0) w.y = -w.y;
     C2 xk, xh;
-    real_split<T>(zk, zh, w, xk);
-    xk = cscale<T>(xk, s);
+    real_split_pair(zk, zh, w, s, xk, xh);
     F[k] = xk;
     F[n - k] = cconj<T>(xk);
     if (k2 != k) {
-        real_split<T>(zh, zk, mk<T>(-w.x, w.y), xh);
-        xh = cscale<T>(xh, s);
         F[k2] = xh;
         F[n - k2] = cconj<T>(xh);
     }
