@@ -90,10 +90,15 @@ template <typename T> struct StockCfg {
 // (radix-8 passes, 64 registers, twice the threads) where that takes no more
 // passes than sixteen: at 64 = 8 x 8 one pass over 2^16 points took 4.7 us
 // instead of 6.3, over 2^24 points 108 instead of 118; at 512 = 8 x 8 x 8 6.1
-// instead of 9.3, and 157 instead of 177.  One pass more costs long batches
+// instead of 9.3, and 157 instead of 177; at 32 = 8 x 4 rows of 2^20 points 10.1
+// instead of 15.0, of 2^24 99 instead of 149.  One pass more costs long batches
 // more than the threads give short ones: 256 7.1 -> 6.1 and 130 -> 145, columns
 // of 1024 112 -> 141, 4096 11.7 -> 12.7 and 214 -> 243.
-__host__ __device__ constexpr int fx_elems(int L) { return L == 64 || L == 512 ? 8 : 16; }
+__host__ __device__ constexpr int fx_elems(int L) {
+    int lg = 0;
+    while ((2 << lg) <= L) lg++;
+    return (lg + 2) / 3 == (lg + 3) / 4 ? 8 : 16;
+}
 
 // Pass twiddle table of a length-L line (one per length, built by
 // passtw_kernel): pass P >= 1 of radix R after NS = 16^P owns NS * R slots
