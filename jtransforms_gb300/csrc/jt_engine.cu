@@ -2396,8 +2396,22 @@ namespace {
 // buffers: copy in (stream h2d), transform (stream), copy out (stream d2h)
 #define JT_HOST_RING 3
 
+// Pinned words that the device error flag is copied to: a thread takes one with
+// its first host call and gives it back when it ends, so there are as many as
+// threads have made such calls at a time.
+struct WordPool {
+    std::mutex mu;
+    std::vector<int *> idle;  // with room for all there are: giving one back allocates nothing
+    size_t all = 0;
+    // (threads may end after static objects do: never destroyed)
+    static WordPool &get() {
+        static WordPool *p = new WordPool;
+        return *p;
+    }
+};
+
 struct ThreadState {
-    int *err_word = nullptr;  // pinned: the device error flag, copied out with the result
+    int *err_word = nullptr;
     cudaStream_t stream = nullptr;
     cudaStream_t h2d = nullptr, d2h = nullptr;
     cudaEvent_t in_done[JT_HOST_RING] = {}, run_done[JT_HOST_RING] = {}, out_done[JT_HOST_RING] = {};
@@ -2406,6 +2420,9 @@ struct ThreadState {
     cudaStream_t last = nullptr;
     ~ThreadState() {
         // device resources are reclaimed at process exit
+        if (!err_word) return;
+        std::lock_guard<std::mutex> g(WordPool::get().mu);
+        WordPool::get().idle.push_back(err_word);
     }
 };
 thread_local ThreadState t_state;
@@ -2419,7 +2436,21 @@ int ensure_stream() {
 }
 
 int ensure_err_word() {
-    if (!t_state.err_word) JT_CU(cudaMallocHost(&t_state.err_word, sizeof(int)));
+    if (t_state.err_word) return JT_OK;
+    WordPool &p = WordPool::get();
+    std::lock_guard<std::mutex> g(p.mu);
+    if (!p.idle.empty()) {
+        t_state.err_word = p.idle.back();
+        p.idle.pop_back();
+        return JT_OK;
+    }
+    try {
+        p.idle.reserve(p.all + 1);
+    } catch (const std::bad_alloc &) {
+        return JT_ENOMEM;
+    }
+    JT_CU(cudaMallocHost(&t_state.err_word, sizeof(int)));
+    p.all++;
     return JT_OK;
 }
 
