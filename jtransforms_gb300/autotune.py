@@ -13,20 +13,20 @@ candidate split:
 Each candidate is installed with jt_set_split before its plan is created.
 Times are CUDA-event medians on the current stream after warm-up, with L2
 flushed before every call. The fastest split per length and precision (of
-those within 3 % the most even one) goes into `jt_plan_table.h`, which the library compiles in (a precision that was
-not tuned keeps its current table rows). All measurements go to
+those within 3 % the most even one) goes into `jt_plan_table.h`, which the
+library compiles in (a precision that was not tuned keeps its current table
+rows). All measurements go to
 `plan_table_f32.json` / `plan_table_f64.json` beside it.
 
 With `--tile` it tunes instead the mixed-radix tile kernel: for each size
-class ceil(log2 L) and precision it times a 3 * 2^k length (a length the tile
-kernel runs) over a 256 MiB batch with each candidate number of elements per
-CTA (which sets the lines and threads per CTA), through JT_OPT_TILE_ELEMS,
-and writes the fastest into kTileElemsF32 / kTileElemsF64
+class ceil(log2 L) and precision it times a length that the tile kernel runs
+(one of `tile_lengths`) over a 256 MiB batch with each candidate number of
+elements per CTA (which sets the lines and threads per CTA), through
+JT_OPT_TILE_ELEMS, and writes the fastest into kTileElemsF32 / kTileElemsF64
 (`plan_table_tile.json`).
 
 With `--radix` it tunes the tile kernel's pass order: for each size class and
-precision it times two lengths of the class, 3 * 2^(k-2) and 7 * 2^(k-3),
-over 256 MiB batches with each of the four orders of JT_OPT_RADIX_ORDER
+precision it times two such lengths over 256 MiB batches with each of the four orders of JT_OPT_RADIX_ORDER
 (power-of-two or odd radices first; 16s or 8s for the power of two), and
 writes the order with the least summed time into kRadixOrderF32 /
 kRadixOrderF64 (`plan_table_radix_<prec>.json`).
@@ -194,12 +194,19 @@ def time_radix(N, J, torch, n, order, prec, flush, steps=5, warmup=3):
         N.set_option(N.OPT_RADIX_ORDER, prev)
 
 
+def tile_lengths(lg: int):
+    """Two lengths with ceil(log2 n) = lg that run the tile kernel in both
+    precisions: with a prime factor above 13 (other lengths have kernels of
+    their own, which read neither table); rows of one pass in the first class."""
+    return [12, 14] if lg == 4 else [17 << (lg - 5), 19 << (lg - 5)]
+
+
 def tune_radix(N, J, torch, precs, flush, out_dir):
     best = {}
     for prec in precs:
         res, tab = {}, {}
         for lg in range(4, 14 if prec == "f32" else 13):
-            lengths = [3 << (lg - 2), 7 << (lg - 3)]  # both with ceil(log2 n) = lg
+            lengths = tile_lengths(lg)
             cand = {}
             for order in range(4):
                 cand[str(order)] = {str(n): time_radix(N, J, torch, n, order, prec, flush) for n in lengths}
@@ -220,7 +227,7 @@ def tune_tiles(N, J, torch, precs, flush, out_dir):
     for prec in precs:
         res, tab = {}, {}
         for lg in range(4, 14 if prec == "f32" else 13):
-            n = 3 << (lg - 2)  # in (2^(lg-1), 2^lg]: ceil(log2 n) = lg
+            n = tile_lengths(lg)[0]
             cand = {}
             for elems in (512, 1024, 2048, 4096, 8192, 16384):
                 if elems < n:
