@@ -465,42 +465,77 @@ static std::vector<int> blue_radices(int n) {
     if (R.size() > 2) std::swap(R[1], R.back());
     return R;
 }
-// Bank conflicts of those strides, as a share of a pass: r's common factor
-// with the 16 banks of a half-warp, over eight.
-static double blue_conflicts(int n) {
-    const std::vector<int> R = blue_radices(n);
-    auto ways = [](int r) { return (r & -r) - 1; };
-    return (ways(R.front()) + ways(R.back())) / 8.0;
+// What blue_split weighs of each length that has such radices, in order.
+struct BlueLength {
+    int n, passes;
+    // bank conflicts of those strides, as a share of a pass: r's common factor
+    // with the 16 banks of a half-warp, over eight
+    double conflicts;
+    // the radices' share of a Bluestein transform's variance by rounding, relative
+    // to its own, in 1e-15 (blue_split)
+    double noise;
+};
+static const std::vector<BlueLength> &blue_lengths() {
+    static const std::vector<BlueLength> t = [] {
+        std::vector<BlueLength> v;
+        for (int n = 2; n <= 8192; n++) {
+            if (!blue_passes()[n]) continue;
+            static const double var[17] = {0, 0, 0, 0, 6.2, 6.9, 8.6, 9.1, 9.1, 9.4, 9.0, 0, 9.6, 0, 0, 0, 11.9};
+            auto ways = [](int r) { return (r & -r) - 1; };
+            const std::vector<int> R = blue_radices(n);
+            double noise = 0;
+            for (int r : R) noise += var[r];
+            v.push_back(BlueLength{n, blue_passes()[n], (ways(R.front()) + ways(R.back())) / 8.0, noise});
+        }
+        return v;
+    }();
+    return t;
 }
 // Convolution N = n1 n2 >= m of a Bluestein transform: n1 = 1 up to 8192 (one
-// kernel), else the n1 x n2 view.  The cheapest by length times memory and
-// passes: a pass counts as half a crossing of memory.
-static bool blue_split(int64_t m, int *n1, int *n2) {
-    const auto &np = blue_passes();
+// kernel), else the n1 x n2 view. The cheapest of those that are no further off
+// than the convolution of the power of two nB that they replace.
+//   error: the shorter a convolution, the more of its rounding falls on the n
+//   numbers that are kept. Variance = (the radices' noise) (0.2 + 0.8 m/N), fitted
+//   to 670 splits of twelve lengths from 97 to 40009 (5 % rms; 4 and 5 rounded
+//   up, and as much allowed); powers of two as they ran before: 2.8 and 3.0 a
+//   bit, 4.1 in two passes.
+//   (By cost alone 4099 took 8400 points for 16384 and was 1.87e-7 off, not
+//   1.60e-7.)
+//   cost: ps a point, fitted to the same splits (11 % rms).
+static bool blue_split(int64_t m, int64_t nB, int *n1, int *n2) {
+    const auto &lens = blue_lengths();
+    int lg = 0;
+    while (((int64_t)1 << lg) < nB) lg++;
+    const double most = 1.04 * lg * (lg <= 11 ? 2.8 : lg <= 14 ? 3.0 : 4.1) * (0.2 + 0.8 * m / nB);
+    auto quiet = [&](double noise, int64_t N) { return N == nB || noise * (0.2 + 0.8 * m / N) <= most; };
     double best = 0;
     if (m <= 8192) {
-        for (int n = (int)std::max<int64_t>(m, 20); n <= 8192; n++) {
-            if (np[n] < 2) continue;
-            const double c = (double)n * (2 + np[n] + blue_conflicts(n));
+        for (const BlueLength &l : lens) {
+            if (l.n < m || l.n < 20 || l.passes < 2 || !quiet(l.noise, l.n)) continue;
+            if (best > 0 && l.n * 5.7 >= best) break;
+            const double c = l.n * (2.3 + 1.7 * l.passes + 0.9 * l.conflicts + (l.n > 7000 ? 1.3 : 0));
             if (best == 0 || c < best) {
                 best = c;
                 *n1 = 1;
-                *n2 = n;
+                *n2 = l.n;
             }
-            if (n * 4.0 >= best) break;
         }
         if (best > 0) return true;
     }
-    for (int b = 64; b <= 4096; b++) {
-        if (np[b] < 2) continue;
-        int64_t a = std::max<int64_t>(cdiv(m, b), 16);
-        while (a <= 1024 && np[a] == 0) a++;
-        if (a > 1024) continue;
-        const double c = (double)a * b * (6 + np[a] + np[b] + blue_conflicts(b) + (a > 512 || b > 2048 ? 1 : 0));
-        if (best == 0 || c < best) {
-            best = c;
-            *n1 = (int)a;
-            *n2 = b;
+    for (const BlueLength &b : lens) {
+        if (b.n < 64 || b.n > 4096 || b.passes < 2) continue;
+        for (const BlueLength &a : lens) {
+            const int64_t N = (int64_t)a.n * b.n;
+            if (a.n < 16 || N < m) continue;
+            if (a.n > 1024 || N * 10 > nB * 11 || (best > 0 && N * 11.9 >= best)) break;
+            if (!quiet(a.noise + b.noise, N)) continue;
+            const double c = N * (7.5 + (a.passes > 2 ? 9.8 : a.passes > 1 ? 5.8 : 0) + (a.n > 256 ? 2 : 0) + 2.2 * b.passes + 0.6 * b.conflicts +
+                                  (b.n < 100 ? 1.1 : b.n > 2048 ? 0.4 : 0) + 1e-6 * a.n);
+            if (best == 0 || c < best) {
+                best = c;
+                *n1 = a.n;
+                *n2 = b.n;
+            }
         }
     }
     return best > 0;
@@ -926,7 +961,7 @@ template <typename T> struct Fft1 {
     // against 539 us, 65521: 333 / 339, 300007: 410 / 605; but 524287: 505 /
     // 369, 1000003: 675 / 395, whose columns take three passes).
     int init_blue() {
-        const bool found = blue_split(2 * n - 1, &bn1, &bn2);
+        const bool found = blue_split(2 * n - 1, nB, &bn1, &bn2);
         const int64_t len = (int64_t)bn1 * bn2;
         if (!found || len > ((int64_t)1 << 20) || (len > 300000 && nB * 5 < len * 7)) {
             bn1 = 0;
