@@ -497,8 +497,9 @@ static const std::vector<BlueLength> &blue_lengths() {
 //   error: the shorter a convolution, the more of its rounding falls on the n
 //   numbers that are kept. Variance = (the radices' noise) (0.2 + 0.8 m/N), fitted
 //   to 670 splits of twelve lengths from 97 to 40009 (5 % rms; 4 and 5 rounded
-//   up, and as much allowed); powers of two as they ran before: 2.8 and 3.0 a
-//   bit, 4.1 in two passes.
+//   up, and as much allowed); powers of two as they ran before: 2.5 a bit up to
+//   1024, 2.8 to 3.0 up to 2^14, 4.1 in two passes.  These kernels run a power
+//   of two otherwise, so it has to be quiet too.
 //   (By cost alone 4099 took 8400 points for 16384 and was 1.87e-7 off, not
 //   1.60e-7.)
 //   cost: ps a point, fitted to the same splits (11 % rms).
@@ -506,8 +507,9 @@ static bool blue_split(int64_t m, int64_t nB, int *n1, int *n2) {
     const auto &lens = blue_lengths();
     int lg = 0;
     while (((int64_t)1 << lg) < nB) lg++;
-    const double most = 1.04 * lg * (lg <= 11 ? 2.8 : lg <= 14 ? 3.0 : 4.1) * (0.2 + 0.8 * m / nB);
-    auto quiet = [&](double noise, int64_t N) { return N == nB || noise * (0.2 + 0.8 * m / N) <= most; };
+    const double bit = lg <= 10 ? 2.5 : lg == 11 ? 2.8 : lg == 13 ? 2.9 : lg <= 14 ? 3.0 : 4.1;
+    const double most = 1.04 * lg * bit * (0.2 + 0.8 * m / nB);
+    auto quiet = [&](double noise, int64_t N) { return noise * (0.2 + 0.8 * m / N) <= most; };
     double best = 0;
     if (m <= 8192) {
         for (const BlueLength &l : lens) {
