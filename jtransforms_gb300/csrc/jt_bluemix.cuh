@@ -3,8 +3,8 @@
 //
 // y_k = conj(b_k) sum_j (x_j conj(b_j)) b_{k-j}, b_j = e^{i pi j^2 / n}, is a
 // cyclic convolution of any length N >= 2n - 1.  N is a product of the
-// radices below, at most a few percent above 2n - 1 (a power of two is up to
-// twice that).  One kernel up to N = 8192 (blue_mid_kernel<true>); beyond that
+// radices below, no noisier than the power of two that would serve (up to twice
+// as long as it need be; blue_split).  One kernel up to N = 8192 (blue_mid_kernel<true>); beyond that
 // N = n1 n2 in three:
 //   in    n1-point columns of the n1 x n2 view, chirped and zero beyond n as
 //         they are read, four-step twiddle on the store
@@ -17,10 +17,10 @@
 // forward pass holds the inputs of the inverse transform's first pass when
 // that has the same radix, so the inverse takes the radices in reverse.
 //
-// Measured (GB300, FloatFFT_1D(10007) x 1024, both directions): 612 us, 1300
-// with seven kernels around a power-of-two convolution of 32768 (here 20160 =
-// 16 x 1260 points): columns in 44 and out 34 us per 84 MB of convolutions,
-// waiting for their loads, rows 72 us, issuing in 64 % of the cycles.
+// Measured (GB300, FloatFFT_1D(10007) x 1024, both directions): 608 us, 1300
+// with seven kernels around a power-of-two convolution of 32768 (here 20736 =
+// 16 x 1296 points): the columns wait for their loads, the rows (half of the
+// time) issue in 64 % of the cycles.
 //
 // Reference: bluestein_complex, fft/DoubleFFT_1D.java:1864-2107.
 #pragma once

@@ -415,8 +415,8 @@ __device__ C2 *tile_passes_fp(C2 *src, C2 *dst, int lines, int L, int Lp, int np
 // ---------------------------------------------------------------------------
 // The same passes of doubles in 64-bit block fixed point (jt_fixmath.cuh): the
 // FP64 pipe, at two instructions a clock and SM, was what they waited for.
-// Measured (GB300, 2 M points): n = 122 757 us where FP64 took 2602, 1331 475 /
-// 929; DCT of n = 1000 85 / 139.
+// Measured (GB300, 2 M points): n = 122 767 us where FP64 took 2602, 1331 471 /
+// 929; DCT of n = 1000 90 / 139.
 // ---------------------------------------------------------------------------
 // Words per line after the two buffers: three rounds of bits, the exponent,
 // the scaling of lines at the ends of the double range.

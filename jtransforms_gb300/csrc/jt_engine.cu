@@ -959,8 +959,8 @@ template <typename T> struct Fft1 {
     // Tables of the float Bluestein kernels.
     // Convolutions up to 300,000 points, and up to 2^20 where the power of two
     // (nB) is longer by two fifths, measured faster than the power-of-two
-    // passes between separate chirp kernels (8 M points of n = 10007: 259
-    // against 539 us, 65521: 333 / 339, 300007: 410 / 605; but 524287: 505 /
+    // passes between separate chirp kernels (8 M points of n = 10007: 248
+    // against 539 us, 65521: 303 / 339, 300007: 331 / 605; but 524287: 505 /
     // 369, 1000003: 675 / 395, whose columns take three passes).
     int init_blue() {
         const bool found = blue_split(2 * n - 1, nB, &bn1, &bn2);

@@ -14,13 +14,14 @@
 // right to 2^-62 (fx_root).  The result is rounded to double once.
 //
 // Measured (GB300, DoubleFFT_3D(256^3).complexForward and inverse, 268 MB):
-// 888 us where the FP64 passes took 4617; DoubleFFT_1D(4096) x 256, both
-// directions: 43 against 183 us; DoubleFFT_1D(1024), one line: 14 against
+// 873 us where the FP64 passes took 4617; DoubleFFT_1D(4096) x 256, both
+// directions: 40 against 183 us; DoubleFFT_1D(1024), one line: 11 against
 // 37 us a call (the FP64 pipe's latency).  Relative L2 error against quad
-// precision over normal, uniform, tone, smooth, real and log-distributed
-// inputs: 0.5-1.0e-16 at n = 16..8192, 1.1-2.3e-16 before.  What bounds a
-// pass over 256-point lines now is latency: the ALU is 59 % busy, the FP64
-// pipe 41 % (the conversions back to double), memory 51 % of its copy rate,
+// precision over normal, uniform, tone, smooth, real, constant and
+// log-distributed inputs and a spike: at most 1.3e-16 at n = 16..8192, 2.5e-16
+// before; 1.0e-16 at 2^14..2^18, 3.5e-16 before.  What bounds a
+// pass over 256-point lines now is latency: the ALU is 62 % busy, the FP64
+// pipe 43 % (the conversions back to double), memory 52 % of its copy rate,
 // with four CTAs of 128 registers a thread per SM.
 //
 // Range: lines whose largest exponent leaves no room (below 2^-900 or above

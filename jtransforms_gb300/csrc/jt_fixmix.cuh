@@ -9,9 +9,9 @@
 // jt_device.cuh.
 //
 // Measured (GB300, one direction, FP64 tile passes before): 2 M points of n =
-// 1000 55 us (185), of 96 39 (105), of 3000 73 (228); one transform of n = 1000
-// 15.5 us (39.4), of 10^6 75 (375).  Relative L2 error against quad precision,
-// n = 24..1000: 0.9-1.8e-16 (1.8-2.7e-16).
+// 1000 49 us (185), of 96 31 (105), of 3000 65 (228); one transform of n = 1000
+// 10.8 us (39.4), of 10^6 67 (375).  Relative L2 error against quad precision:
+// at most 1.4e-16 for n = 24..3600, 3.3e-16 before.
 //
 // Reference: the FFTPACK passes, fft/DoubleFFT_1D.java:6630-7842.
 #pragma once

@@ -24,13 +24,13 @@
 //
 // What bounded the FP64 form (jt_r2r.cuh) was the FP64 pipe; see jt_fix64.cuh.
 // Lines with an infinity or a NaN still run it.  Measured (GB300, both
-// directions): DoubleDCT_2D(1024^2) 74 us where the FP64 form took 254,
-// DoubleDHT_3D(128^3) 148 where it took 508; a quarter to a half of the error
-// against quad precision on 32^2..256^2 images and noise (where one
-// coefficient dominates an image's norm its last rounding decides either).
+// directions): DoubleDCT_2D(1024^2) 72 us where the FP64 form took 254,
+// DoubleDHT_3D(128^3) 116 where it took 508.  Relative L2 error
+// of DCTs of noise and images, 32^2 to 1024^2, against quad precision: 6.4-8.0e-17,
+// 2.0-3.7e-16 before.
 // At these sizes a kernel is one wave of few warps and bound by their
-// latency: 3 of the 10 cycles between two of a warp's instructions wait for
-// the instruction cache.
+// latency: of the 10 cycles between two of a warp's instructions 3 to 4 wait
+// for its loads and 1.4 for shared memory.
 #pragma once
 
 #include "jt_fix64.cuh"

@@ -23,8 +23,9 @@ __device__ __forceinline__ void pdl_begin() {
 
 // Elementwise kernels, one number a thread: a block lives about as long as those
 // two instructions take, so grids above four waves (of 152 SMs, eight blocks of
-// 256 each) launch in plain stream order and skip them (FloatFFT_1D(188779) x 64, pre/mul/post around a power of two,
-// both directions: 1541 us with them in every block, 1411 without).
+// 256 each) launch in plain stream order and skip them (FloatFFT_1D(188779) x 64,
+// pre/mul/post around a power of two, both directions: 1541 us with them in every
+// block, 1411 without).
 #define JT_PDL_BLOCKS (4 * 8 * 152)
 __device__ __forceinline__ void pdl_begin_few() {
     if (gridDim.x <= JT_PDL_BLOCKS) pdl_begin();

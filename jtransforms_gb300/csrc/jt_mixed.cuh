@@ -10,10 +10,11 @@
 // butterflies read neighbouring entries; indexes are divided by multiplying
 // with reciprocals.
 //
-// Measured (GB300, FloatFFT_1D(1000) x 32768, 262 MB, both directions): 256 us,
-// 765 with the tile passes of jt_device.cuh, which crossed shared memory ten
+// Measured (GB300, FloatFFT_1D(1000) x 32768, 262 MB, both directions): 251 us,
+// 755 with the tile passes of jt_device.cuh, which crossed shared memory ten
 // times, divided by run-time lengths and gathered their twiddles; a
-// FloatFFT_2D(1080, 1920).realForwardFull 58 against 129 us.  Rows move at
+// FloatFFT_2D(1080, 1920).realForwardFull 39 against 128 us (rows of half the
+// length and half the columns, since).  Rows move at
 // 3.9-5.4 TB/s of 6.8 (one line of 1000 per CTA: 32 warps per SM, waiting for
 // their loads a third of the time); lines of 3000 and more, of which one or
 // two fit an SM, at 1.9-3.0.
